@@ -14,11 +14,13 @@
 // (exact division by the odd m), so q_j is the Montgomery multiplier of the
 // step and no division is ever executed. The chain ends at r_0 = 2^(10e) mod m.
 //
-// Six residue kinds:
+// Seven residue kinds:
 //   width 1 (m < 2^28): R = 2^32, residues kept lazily in [0, 4m).
 //   middle width 1 (2^28 <= m < 2^31): R = 2^32, residues in [0, m).
 //   strict width 1 (2^28 <= m < 2^32): R = 2^32, residues in [0, m), carries kept.
-//   short width 2 (2^32 <= m < 2^44): R = 2^48, residues in [0, 4m).
+//   float-quotient width 2 (2^32 <= m < 94 * 2^32): R = 2^24, residues below 8m,
+//     the top of each square taken off by a float quotient.
+//   short width 2 (94 * 2^32 <= m < 2^44): R = 2^48, residues in [0, 4m).
 //   width 2 (2^28 <= m < 2^60): R = 2^64 by two word steps, residues in [0, 4m).
 //   wide width 2 (2^60 <= m < 2^62): the same steps with residues in [0, 2m).
 // The ladder step is y <- REDC(y^2) << b with b the next exponent bit; in the
@@ -44,6 +46,13 @@ __device__ __forceinline__ float rcp_approx(float x)
 {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float rsqrt_approx(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
@@ -463,6 +472,146 @@ __device__ __forceinline__ uint64_t w2s_pow2(uint64_t E, uint64_t m, uint32_t mp
     r = min(r, r - 2 * m);
     r = min(r, r - m);
     return r;
+}
+
+// ------------------------------------------------ width 2, m < 94 * 2^32 --
+// 2^32 <= m < 94 * 2^32 (positions up to 1e11): the square is reduced from both
+// ends at once. Its top comes off by a float quotient, its bottom by a 24-bit
+// Montgomery step, with one multiplier v = u + (q - o) 2^24 for both:
+//   u = y^2 m^-1 mod 2^24          (exact, from the low word of y^2)
+//   q ~ floor(y^2 / (2^24 m))      (float, from the top 23 bits of y)
+//   X = y^2 - v m = 2^24 z, z = y^2 2^-24 mod m up to a multiple of m.
+// The float work is done before the high words of y^2 would be needed, so y^2
+// and v m are formed mod 2^64 only: 8 multiply halves a step (y0^2, u, y0 y1,
+// v0 n0, v0 n1, v1 n0 with n = 2^64 - m) against 14 in w2s_sqr, which pays
+// for the full square and two exact word steps.
+// Floats: the 23 bits y >> 18 are used as they are, as a denormal (2^-149 each);
+// s carries 2^119 of that, so t = s (y >> 18) is y / sqrt(2^24 m) times 2^-30,
+// and t^2 + 2^-60 (2^23 - o) has q - o in its low mantissa bits.
+// Bounds: s <= 2^125 / sqrt(m) and t are rounded down, so q never exceeds
+// y^2 / (2^24 m). It falls short by the floor (1), the truncation of y (2^-5 y/m)
+// and the roundings (12 2^-24 q), so with y < B m
+//   X / (2^24 m) lies in (o - 1, o + 1 + B / 32 + 12 2^-48 B^2 m), B twice that.
+// o = 2 (m < 15 * 2^34): z in (m, 3.95m), q >= 2 always. o = 1 (CK): z in (0, 2.65m),
+// X < 2^64 up to m = 94 * 2^32; there q - 1 may be -1, so it is offset by 2^22 and
+// ck takes the offset's 2^46 m out of X again (a register more). In both y < 2^41.
+template <bool CK>
+struct W2FState {
+    uint32_t y0, y1, n0, n1, ip;                        // y, 2^64 - m, m^-1 mod 2^32
+    uint32_t top;                                       // y >> 18
+    float s;
+    // X = y^2 - v m
+    __device__ __forceinline__ void square(uint32_t &x0, uint32_t &x1) const
+    {
+        const float t = __fmul_rd(__uint_as_float(top), s);
+        const uint32_t q = __float_as_uint(__fmaf_rd(t, t, (CK ? 12582911.0f : 8388606.0f) * 8.67361737988403547e-19f));
+        const uint64_t a = (uint64_t)y0 * y0;
+        const uint32_t u = (uint32_t)a * ip;
+        const uint32_t v0 = __byte_perm(u, q, 0x4210), v1 = __byte_perm(q, 0u, 0x4421);
+        const uint32_t p = y0 * y1 + (CK ? (0u - n0) << 13 : 0u);
+        uint32_t h;
+        asm("{\n\t.reg .u32 g;\n\t"
+            "mad.lo.cc.u32 %0, %2, %3, %4;\n\t"         // y0^2 + v0 n0
+            "madc.hi.u32 g, %2, %3, %5;\n\t"
+            "mad.lo.u32 g, %2, %6, g;\n\t"              // + v0 n1 2^32
+            "mad.lo.u32 %1, %7, %3, g;\n\t}"            // + v1 n0 2^32
+            : "=&r"(x0), "=r"(h)
+            : "r"(v0), "r"(n0), "r"((uint32_t)a), "r"((uint32_t)(a >> 32)), "r"(n1), "r"(v1));
+        x1 = h + (p << 1);                              // + y0 (2 y1) 2^32
+    }
+    // y = X >> (24 - b)
+    __device__ __forceinline__ void step(uint32_t b)
+    {
+        uint32_t x0, x1;
+        square(x0, x1);
+        const uint32_t sh = 8u | b;
+        y0 = __funnelshift_l(x0, x1, sh);
+        y1 = __funnelshift_l(x1, 0u, sh);
+        top = __funnelshift_r(y0, y1, 18);
+    }
+    // Constants of the ladder and its start y = 2^(24 + p) up to a multiple of m,
+    // 1 <= p <= 31: the float quotient (below 2^23) is within 2.5 of 2^(24+p) / m,
+    // so y lies in (m/2, 4.5m) with two m added back. s: m rounded up, one Newton
+    // step on the approximate root with the residual formed exactly, less one ulp.
+    __device__ __forceinline__ void start(uint64_t m, uint32_t mp, uint32_t p)
+    {
+        const uint64_t n = 0ull - m;
+        n0 = (uint32_t)n;
+        n1 = (uint32_t)(n >> 32);
+        ip = 0u - mp;
+        const float fm = __fmaf_ru(__uint2float_rn((uint32_t)(m >> 32)), 4294967296.0f, __uint2float_ru((uint32_t)m));
+        const float r0 = rsqrt_approx(fm);
+        const float h = fm * r0;
+        const float e = __fmaf_rn(-__fmaf_rn(fm, r0, -h), r0, __fmaf_rn(-h, r0, 1.0f));
+        const float r = __fmaf_rn(0.5f * e, r0, r0);
+        s = __uint_as_float(__float_as_uint(4.25352958651173080e37f * r) - 1u);     // 2^125 r
+        const float i0 = r * r;
+        const float inv = __fmaf_rn(i0, __fmaf_rn(-fm, i0, 1.0f), i0);
+        const float scale = __int_as_float((int)((127u + 24u + p) << 23));          // 2^(24+p)
+        const uint32_t q = __float2uint_rz(scale * inv);
+        const uint64_t y = (1ull << (24 + p)) + 2 * m - (uint64_t)q * m;
+        y0 = (uint32_t)y;
+        y1 = (uint32_t)(y >> 32);
+        top = __funnelshift_r(y0, y1, 18);
+    }
+    // y -> [0, m): a float quotient that is low by at most one.
+    __device__ __forceinline__ uint64_t finish(uint64_t m) const
+    {
+        const float t = __fmul_rd(__uint_as_float(top), s);
+        const uint32_t k = __float2uint_rz(__fmaf_rn(t * s, 1.03397576569128459e-25f, -0.001f));    // 2^-83
+        const uint64_t y = (((uint64_t)y1 << 32) | y0) - (uint64_t)k * m;
+        return min(y, y - m);
+    }
+};
+
+// The ladder runs in Montgomery form with R = 2^24 on Ep = E - 24, Ep >= 2^5:
+// the five leading bits at once, then one step a bit.
+template <bool CK>
+__device__ __forceinline__ uint64_t w2f_pow2(uint64_t E, uint64_t m, uint32_t mp)
+{
+    const uint64_t Ep = E - 24;
+    W2FState<CK> st;
+    int i = 64 - __clzll((long long)Ep) - 5;
+    st.start(m, mp, (uint32_t)(Ep >> i));
+    for (--i; i >= 0; --i) st.step((uint32_t)(Ep >> i) & 1u);
+    return st.finish(m);
+}
+
+// Two ladders in turn, of terms whose exponents agree above bit S in the whole
+// warp (e_max the largest, 630 above the smallest): those bits are taken from one
+// value P, so that both ladders share the shift counts; the low S bits come from
+// each exponent. A group across a multiple of 2^S (1 % at S = 16) runs its ladders
+// one after the other. S = 13 measured 566.1 ms at 1e10, S = 16 561.6 ms. Exponents
+// below 2^48 (kW2FExp) keep P in one word.
+template <bool CK>
+__device__ __forceinline__ void w2f_pow2_pair(uint64_t EA, uint64_t ma, uint32_t mpa, uint64_t EB, uint64_t mb,
+                                              uint32_t mpb, uint64_t e_max, uint64_t &ra, uint64_t &rb)
+{
+    constexpr int S = 16;
+    const uint32_t P = (uint32_t)((e_max - 24) >> S);
+    if (e_max >= (1ull << (S + 6)) && (uint32_t)((e_max - 630 - 24) >> S) == P) {
+        W2FState<CK> A, B;
+        int j = 27 - __clz(P);
+        A.start(ma, mpa, P >> j);
+        B.start(mb, mpb, P >> j);
+#pragma unroll 8
+        for (--j; j >= 0; --j) {
+            const uint32_t bit = (P >> j) & 1u;
+            A.step(bit);
+            B.step(bit);
+        }
+        const uint32_t la = (uint32_t)(EA - 24), lb = (uint32_t)(EB - 24);
+#pragma unroll
+        for (int l = S - 1; l >= 0; --l) {
+            A.step(la >> l & 1u);
+            B.step(lb >> l & 1u);
+        }
+        ra = A.finish(ma);
+        rb = B.finish(mb);
+        return;
+    }
+    ra = w2f_pow2<CK>(EA, ma, mpa);
+    rb = w2f_pow2<CK>(EB, mb, mpb);
 }
 
 // ------------------------------------------------------- width 2, m >= 2^60 --

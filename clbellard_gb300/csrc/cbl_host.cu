@@ -58,6 +58,7 @@ struct cbl_ctx {
     // prepared multi-position run (cbl_prepare / cbl_run_prepared)
     int prep_npos = 0;
     int prep_nseg = 0;
+    int prep_level = 0;                              // term-kernel level of the prepared table
     uint64_t prep_ntiles = 0;
     uint64_t prep_terms = 0;
     bool prep_carry = false;                         // a prepared slot may take >= 2^31 flushes
@@ -222,10 +223,18 @@ uint64_t order_and_number(std::vector<Seg> &v, uint32_t tile_k)
     return t;
 }
 
-int grid_192(cbl_ctx *c)
+int grid_192(const cbl_ctx *c, int level)
 {
-    int per = c->ctas_per_sm > 0 ? c->ctas_per_sm : terms192_max_ctas_per_sm(256);
+    int per = c->ctas_per_sm > 0 ? c->ctas_per_sm : terms192_max_ctas_per_sm(level);
     return std::max(1, c->sm_count * per);
+}
+
+// Term-kernel level of a set of segments, from their largest modulus.
+int segs_level(const std::vector<Seg> &v)
+{
+    int level = 0;
+    for (const Seg &s : v) level = std::max(level, term_level((uint64_t)s.den0 * (s.k1 - 1) + s.den1));
+    return level;
 }
 
 // Upload segments and run the persistent term kernel (accumulates into slots).
@@ -243,8 +252,9 @@ int run_segments(cbl_ctx *c, std::vector<Seg> &v)
     // slot 0 collects every launch since cbl_Set0mem: carry once it may have
     // taken 2^31 flushes (at most one per tile)
     c->slot0_tiles = std::min<uint64_t>(c->slot0_tiles + ntiles, kCarryTiles);
-    CK(launch_terms192(c->d_segs, (int)v.size(), ntiles, (uint32_t)c->tile_k, c->d_counter, c->d_slots,
-                       grid_192(c), 256, c->st, 0, slot_needs_carry(c->slot0_tiles)));
+    const int level = segs_level(v);
+    CK(launch_terms192(level, c->d_segs, (int)v.size(), ntiles, (uint32_t)c->tile_k, c->d_counter, c->d_slots,
+                       grid_192(c, level), c->st, 0, slot_needs_carry(c->slot0_tiles)));
     c->launches++;
     return CBL_OK;
 }
@@ -777,6 +787,7 @@ static int upload_prepared(cbl_ctx *c)
     CK(cudaStreamSynchronize(c->st));
     drop_graph(c);
     c->prep_nseg = (int)v.size();
+    c->prep_level = segs_level(v);
     c->prep_ntiles = ntiles;
     c->partial = 0;
     c->seg_hash = fnv1a(c->prep_shift.data(), sizeof(int) * n, fnv1a(v.data(), sizeof(Seg) * v.size()));
@@ -832,8 +843,8 @@ static int enqueue_prepared(cbl_ctx *c, bool capturing)
     CK(clear_slots(c, 7 * n));
     CK(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), c->st));
     CK(cudaEventRecordWithFlags(c->ev_k0, c->st, evf));
-    CK(launch_terms192(c->d_segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k, c->d_counter, c->d_slots,
-                       grid_192(c), 256, c->st, 0, prepared_carry(c)));
+    CK(launch_terms192(c->prep_level, c->d_segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k, c->d_counter,
+                       c->d_slots, grid_192(c, c->prep_level), c->st, 0, prepared_carry(c)));
     CK(cudaEventRecordWithFlags(c->ev_k1, c->st, evf));
     CK(launch_combine(c->d_slots, n, c->d_shift, c->d_out3, nullptr, c->st));
     return CBL_OK;
@@ -1270,7 +1281,7 @@ int cbl_prepared_info(const cbl_ctx *c, uint64_t *terms, uint64_t *tiles, int *s
     if (terms) *terms = c->prep_terms;
     if (tiles) *tiles = c->prep_ntiles;
     if (segments) *segments = c->prep_nseg;
-    if (grid) *grid = grid_192(const_cast<cbl_ctx *>(c));
+    if (grid) *grid = grid_192(c, c->prep_level);
     return CBL_OK;
     CBL_GUARD_END
 }
@@ -1331,7 +1342,14 @@ int cbl_autotune(cbl_ctx *c, const uint64_t *pos, int n, int force, int *best_ti
         int rc = cbl_set_tuning(c, tile, ctas);
         if (rc) return rc;
     } else {
-        const int occ = terms192_max_ctas_per_sm(256);
+        uint64_t d_max = 0;
+        for (int i = 0; i < n; ++i) {
+            uint64_t d = 0;
+            const int rc = cbl_pos_to_d(pos[i], &d, nullptr);
+            if (rc) return rc;
+            d_max = std::max(d_max, d);
+        }
+        const int occ = terms192_max_ctas_per_sm(term_level(10 * (d_max + kTail192) + 9));
         const int tiles[] = {512, 1024, 2048, 4096, 8192};
         ms_best = 1e300;
         for (int t : tiles) {
@@ -1373,8 +1391,8 @@ int cbl_run_prepared_budget(cbl_ctx *c, double budget_ms, uint64_t *tiles_done, 
         c->partial = 1;
     }
     const uint64_t budget_ns = (uint64_t)(budget_ms * 1e6) + 1;
-    CK(launch_terms192(c->d_segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k, c->d_counter, c->d_slots,
-                       grid_192(c), 256, c->st, budget_ns, prepared_carry(c)));
+    CK(launch_terms192(c->prep_level, c->d_segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k, c->d_counter,
+                       c->d_slots, grid_192(c, c->prep_level), c->st, budget_ns, prepared_carry(c)));
     c->launches++;
     CK(cudaMemcpyAsync(c->h_small, c->d_counter, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->st));
     int rc = sync(c);

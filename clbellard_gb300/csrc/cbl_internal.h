@@ -27,6 +27,9 @@ constexpr uint32_t kDen1[7] = {1, 3, 1, 3, 5, 7, 9};
 constexpr uint64_t kW1Max = 1ull << 28;   // width 1 (one 32-bit word) for m < 2^28
 constexpr uint64_t kW1MMax = 1ull << 31;  // middle width 1 for 2^28 <= m < 2^31
 constexpr uint64_t kW1SMax = 1ull << 32;  // strict width 1 for 2^31 <= m < 2^32
+constexpr uint64_t kW2FLow = 15ull << 34; // float-quotient steps without an offset for 2^32 <= m < 15 * 2^34
+constexpr uint64_t kW2FMax = 94ull << 32; // float-quotient steps for 2^32 <= m < 94 * 2^32, inside short width 2
+constexpr uint64_t kW2FExp = 1ull << 48;  // ... in tiles whose exponents are below 2^48 (the short kind's steps above)
 constexpr uint64_t kW2SMax = 1ull << 44;  // short width 2 for 2^32 <= m < 2^44
 constexpr uint64_t kW2Max = 1ull << 60;   // width 2 (two words, residues < 4m) for m < 2^60
 constexpr uint64_t kW2XMax = 1ull << 62;  // wide width 2 (residues < 2m) for 2^60 <= m < 2^62
@@ -51,6 +54,12 @@ static_assert(sizeof(Seg) == 48, "Seg layout");
 constexpr uint32_t kFlagSign = 1u;
 inline uint32_t seg_flags(int sign, int width) { return (uint32_t)(sign & 1) | ((uint32_t)width << 4); }
 
+// Widest residues of a table's segments, which picks the term kernel's
+// instantiation: 0 one-word kinds only (m < 2^32), 1 up to the short two-word
+// kind (m < 2^44), 2 any. A wider level than needed is slower, never wrong.
+constexpr int kTermLevels = 3;
+__host__ __device__ inline int term_level(uint64_t max_m) { return max_m < kW1SMax ? 0 : max_m < kW2SMax ? 1 : 2; }
+
 // Launch wrappers (cbl_kernels.cu).
 // budget_ns = 0: run to the end; else warps stop taking tiles after budget_ns
 // and the finished tiles are [0, *counter).
@@ -59,9 +68,9 @@ inline uint32_t seg_flags(int sign, int width) { return (uint32_t)(sign & 1) | (
 // then carry each wrap into the digit sum two places up (exact mod 2^192).
 // A slot receives at most one flush per tile, so slot_needs_carry() decides it
 // from the tile counts.
-cudaError_t launch_terms192(const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
-                            unsigned long long *counter, unsigned long long *slots, int grid, int block,
-                            cudaStream_t st, uint64_t budget_ns, bool carry);
+cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
+                            unsigned long long *counter, unsigned long long *slots, int grid, cudaStream_t st,
+                            uint64_t budget_ns, bool carry);
 constexpr uint64_t kCarryTiles = 1ull << 31;
 inline bool slot_needs_carry(uint64_t max_tiles_per_slot) { return max_tiles_per_slot >= kCarryTiles; }
 // slots (nslot x 6 digit sums) of position i, series f = slots[(slot_base[i] + f) * 6 ..]:
@@ -95,6 +104,6 @@ cudaError_t launch_probe_imad(uint32_t *sink, int grid, int block, int iters, ui
 int probe_imad_grid(int sm_count);   // one full wave of probe CTAs
 
 int device_sm_count(int device);
-int terms192_max_ctas_per_sm(int block);
+int terms192_max_ctas_per_sm(int level);
 
 }  // namespace cbl

@@ -49,7 +49,8 @@ __device__ __forceinline__ void shr192(uint32_t q[6], int s)
 // One term's six quotient digits: k < d gives frac(2^(10(d-k))/m), k >= d the
 // tail value 2^(-10(k-d))/m (digits of 1/m shifted right by 10(k-d)).
 // KIND: 1 = width 1 (m < 2^28), 5 = middle width 1 (2^28 <= m < 2^31),
-// 3 = strict width 1 (2^28 <= m < 2^32), 4 = short width 2 (2^32 <= m < 2^44),
+// 3 = strict width 1 (2^28 <= m < 2^32), 7 and 8 = float-quotient width 2 (2^32 <= m
+// < 15 * 2^34 and < 94 * 2^32), 4 = short width 2 (2^32 <= m < 2^44),
 // 2 = width 2 (2^28 <= m < 2^60), 6 = wide width 2 (2^60 <= m < 2^62).
 template <int KIND, bool TAIL>
 __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, uint32_t q[6])
@@ -65,6 +66,9 @@ __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, 
     } else if (KIND == 3) {
         const uint32_t r6 = w1s_pow2(E, (uint32_t)m, mp);
         w1_digits(r6, (uint32_t)m, mp, q);
+    } else if (KIND == 7 || KIND == 8) {
+        const uint64_t r6 = w2f_pow2<KIND == 8>(E, m, mp);
+        w2_digits(r6, m, mp, q);
     } else if (KIND == 4) {
         const uint64_t r6 = w2s_pow2(E, m, mp);
         w2_digits(r6, m, mp, q);
@@ -78,19 +82,26 @@ __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, 
     if (TAIL) shr192(q, (int)(10 * (k - d)));
 }
 
-// Two terms (k and k+32) of a lane per iteration, their ladders interleaved
-// (kinds 1, 3, 4, 5; the width-2 kinds above 2^44 run one term at a time).
+// Two terms (ka and ka+32) of a lane per iteration, their ladders interleaved
+// (kinds 1, 3, 4, 5, 7, 8; the width-2 kinds above 2^44 run one term at a time).
+// The warp's 64 terms are k .. k+63.
 // Same-box timings against one term per iteration, identical bits: 1e9
 // 40.65 -> 38.55 ms, 1e10 841.0 -> 838.9 ms, batch 10.61 -> 10.08 s. Pairing
 // only some kinds traded these against each other (the kernel's code layout
 // and registers change with every instantiation), so all four are paired.
 template <int KIND>
-__device__ __forceinline__ void term_pair(uint64_t d, uint64_t ka, uint64_t ma, uint64_t mb, uint32_t qa[6],
-                                          uint32_t qb[6])
+__device__ __forceinline__ void term_pair(uint64_t d, uint64_t k, uint64_t ka, uint64_t ma, uint64_t mb,
+                                          uint32_t qa[6], uint32_t qb[6])
 {
     const uint32_t mpa = neg_inv32((uint32_t)ma), mpb = neg_inv32((uint32_t)mb);
     const uint64_t Ea = 10ull * (d - ka) + 192ull, Eb = Ea - 320ull;
-    if (KIND == 4) {
+    if (KIND == 7 || KIND == 8) {
+        uint64_t ra, rb;
+        const uint64_t e_max = 10ull * (d - k) + 192ull;
+        w2f_pow2_pair<KIND == 8>(Ea, ma, mpa, Eb, mb, mpb, e_max, ra, rb);
+        w2_digits(ra, ma, mpa, qa);
+        w2_digits(rb, mb, mpb, qb);
+    } else if (KIND == 4) {
         W2SState A{0, 0, (uint32_t)ma, (uint32_t)(ma >> 32), mpa}, B{0, 0, (uint32_t)mb, (uint32_t)(mb >> 32), mpb};
         walk_bits_start_pair<4>(Ea - 48, Eb - 48, A, B, W2SStart{});   // R = 2^48
         uint64_t ra = ((uint64_t)A.y1 << 32) | A.y0, rb = ((uint64_t)B.y1 << 32) | B.y0;
@@ -128,11 +139,12 @@ __device__ __forceinline__ void run_tile(const Seg &s, uint64_t kb, uint64_t ke,
                                          uint32_t &cnt)
 {
     uint64_t k = kb + lane;
-    if (!TAIL && (KIND == 1 || KIND == 3 || KIND == 4 || KIND == 5)) {
-        for (; k + 32 < ke; k += 64) {                  // terms k and k+32 together
+    if (!TAIL && (KIND == 1 || KIND == 3 || KIND == 4 || KIND == 5 || KIND == 7 || KIND == 8)) {
+        uint64_t k0 = kb;
+        for (; k0 + 64 <= ke; k += 64, k0 += 64) {                  // terms k and k+32 together
             const uint64_t ma = (uint64_t)s.den0 * k + s.den1, mb = ma + 32ull * s.den0;
             uint32_t qa[6], qb[6];
-            term_pair<KIND>(s.d, k, ma, mb, qa, qb);
+            term_pair<KIND>(s.d, k0, k, ma, mb, qa, qb);
             acc_add(acc, qa);
             acc_add(acc, qb);
             cnt += 2;
@@ -212,6 +224,28 @@ __device__ __forceinline__ void flush_segment(const Seg &s, int lane, Acc192 &ac
     warp_flush(acc, lane, slots + (size_t)s.slot * 6, carry);
 }
 
+// One tile's terms, by residue kind and main body / tail. LEVEL limits the kinds
+// that a launch can meet (term_level): the kernel's registers and code follow its
+// widest kind, and the one-word kinds ran 5 % slower beside the two-word ones
+// (1e9: 36.8 ms alone in the kernel, 38.8 ms with the float-quotient steps there).
+template <int LEVEL, bool TAIL>
+__device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_t ke, int lane, Acc192 &acc,
+                                              uint32_t &cnt)
+{
+    const int width = (int)((s.flags >> 4) & 15u);
+    if (LEVEL >= 1 && width == 4) {
+        const uint64_t m_last = (uint64_t)s.den0 * (ke - 1) + s.den1;
+        const bool fq = TAIL || 10 * (s.d - kb) + 192 < kW2FExp;
+        if (fq && m_last < kW2FLow) run_tile<7, TAIL>(s, kb, ke, lane, acc, cnt);
+        else if (fq && m_last < kW2FMax) run_tile<8, TAIL>(s, kb, ke, lane, acc, cnt);
+        else run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
+    } else if (LEVEL >= 2 && width == 2) run_tile<2, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (LEVEL >= 2 && width == 6) run_tile<6, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (width == 3) run_tile<3, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (width == 5) run_tile<5, TAIL>(s, kb, ke, lane, acc, cnt);
+    else run_tile<1, TAIL>(s, kb, ke, lane, acc, cnt);
+}
+
 // With budget_ns != 0 a warp takes no new tile once budget_ns have passed
 // since it started. The deadline is checked before the tile counter is
 // incremented, so every tile taken is finished and the finished tiles are
@@ -220,7 +254,13 @@ __device__ __forceinline__ void flush_segment(const Seg &s, int lane, Acc192 &ac
 // flushes them when it moves to another segment, when a lane's term count
 // reaches 2^30, and before it exits: one slot update per run of tiles
 // instead of one per tile.
-__global__ void __launch_bounds__(kBlock192) terms192_kernel(const Seg *__restrict__ segs, int nseg,
+// Registers: the one-word kinds run best at 5 CTAs an SM with 46 registers (1e9:
+// 35.9 ms; 37.4 ms with the 40 that ptxas takes unbounded, 36.2 ms at 4 CTAs),
+// the float-quotient kind at 64 registers and 4 CTAs (1e10: 561.7 ms; 591 ms when held
+// to 48 registers for 5 CTAs, with spills), the single ladders of the general
+// two-word kinds at 5 CTAs (2^27 terms at 1e13: 5.81 ms against 5.96 ms at 4).
+template <int LEVEL>
+__global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel(const Seg *__restrict__ segs, int nseg,
                                                              uint64_t ntiles, uint32_t tile_k,
                                                              unsigned long long *counter,
                                                              unsigned long long *slots, uint64_t budget_ns,
@@ -254,42 +294,33 @@ __global__ void __launch_bounds__(kBlock192) terms192_kernel(const Seg *__restri
         const Seg s = segs[lo];
         const uint64_t kb = s.k0 + (t - s.tile0) * tile_k;
         const uint64_t ke = min(s.k1, kb + tile_k);
-        const int width = (int)((s.flags >> 4) & 15u);
-        const bool tail = kb >= s.d;
-        if (tail) {
-            if (width == 1) run_tile<1, true>(s, kb, ke, lane, acc, cnt);
-            else if (width == 5) run_tile<5, true>(s, kb, ke, lane, acc, cnt);
-            else if (width == 3) run_tile<3, true>(s, kb, ke, lane, acc, cnt);
-            else if (width == 4) run_tile<4, true>(s, kb, ke, lane, acc, cnt);
-            else if (width == 6) run_tile<6, true>(s, kb, ke, lane, acc, cnt);
-            else run_tile<2, true>(s, kb, ke, lane, acc, cnt);
-        } else {
-            if (width == 1) run_tile<1, false>(s, kb, ke, lane, acc, cnt);
-            else if (width == 5) run_tile<5, false>(s, kb, ke, lane, acc, cnt);
-            else if (width == 3) run_tile<3, false>(s, kb, ke, lane, acc, cnt);
-            else if (width == 4) run_tile<4, false>(s, kb, ke, lane, acc, cnt);
-            else if (width == 6) run_tile<6, false>(s, kb, ke, lane, acc, cnt);
-            else run_tile<2, false>(s, kb, ke, lane, acc, cnt);
-        }
+        if (kb >= s.d) run_tile_kind<LEVEL, true>(s, kb, ke, lane, acc, cnt);
+        else run_tile_kind<LEVEL, false>(s, kb, ke, lane, acc, cnt);
     }
     if (cur >= 0) flush_segment(segs[cur], lane, acc, cnt, slots, carry);
 }
 
-cudaError_t launch_terms192(const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
-                            unsigned long long *counter, unsigned long long *slots, int grid, int block,
-                            cudaStream_t st, uint64_t budget_ns, bool carry)
+typedef void (*Terms192Fn)(const Seg *, int, uint64_t, uint32_t, unsigned long long *, unsigned long long *, uint64_t,
+                           int);
+
+static Terms192Fn terms192_fn(int level)
 {
-    (void)block;
-    terms192_kernel<<<grid, kBlock192, 0, st>>>(segs, nseg, ntiles, tile_k, counter, slots, budget_ns,
-                                                carry ? 1 : 0);
+    return level == 0 ? terms192_kernel<0> : level == 1 ? terms192_kernel<1> : terms192_kernel<2>;
+}
+
+cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
+                            unsigned long long *counter, unsigned long long *slots, int grid, cudaStream_t st,
+                            uint64_t budget_ns, bool carry)
+{
+    terms192_fn(level)<<<grid, kBlock192, 0, st>>>(segs, nseg, ntiles, tile_k, counter, slots, budget_ns,
+                                                   carry ? 1 : 0);
     return cudaGetLastError();
 }
 
-int terms192_max_ctas_per_sm(int block)
+int terms192_max_ctas_per_sm(int level)
 {
     int n = 0;
-    (void)block;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, terms192_kernel, kBlock192, 0) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, terms192_fn(level), kBlock192, 0) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }
 
@@ -426,6 +457,8 @@ __global__ void terms_each_kernel(uint64_t d, uint32_t den0, uint32_t den1, int 
             if (m < kW1Max) term_digits<1, false>(d, k, m, q);
             else if (m < kW1MMax) term_digits<5, false>(d, k, m, q);
             else if (m < kW1SMax) term_digits<3, false>(d, k, m, q);
+            else if (m < kW2FLow) term_digits<7, false>(d, k, m, q);
+            else if (m < kW2FMax) term_digits<8, false>(d, k, m, q);
             else if (m < kW2SMax) term_digits<4, false>(d, k, m, q);
             else if (m < kW2Max) term_digits<2, false>(d, k, m, q);
             else term_digits<6, false>(d, k, m, q);
@@ -555,7 +588,9 @@ __global__ void __launch_bounds__(kBlockDD) dd_terms_kernel(double2 *bigsum, uin
             r = redc_word(y * mp, (uint32_t)m, y, 0u);
         } else {
             uint64_t y;
-            if (m < kW2SMax) y = w2s_pow2(e + 64, m, mp);
+            if (m < kW2FLow) y = w2f_pow2<false>(e + 64, m, mp);
+            else if (m < kW2FMax) y = w2f_pow2<true>(e + 64, m, mp);
+            else if (m < kW2SMax) y = w2s_pow2(e + 64, m, mp);
             else if (m < kW2Max) y = w2_pow2(e + 64, m, mp);
             else y = w2x_pow2(e + 64, m, mp);
             uint32_t q[2];

@@ -173,7 +173,7 @@ namespace {
 struct DeviceSetup {
     bool ready = false;
     unsigned char *scratch = nullptr;   // device address of g_noalloc_scratch on this device
-    int grid = 0;
+    int grid[kTermLevels] = {0, 0, 0};
 };
 
 constexpr int kMaxDevices = 64;
@@ -196,7 +196,7 @@ int setup_device(int dev, DeviceSetup **out)
         cudaFuncAttributes attr;
         if (cudaFuncGetAttributes(&attr, noalloc_table_kernel) != cudaSuccess) return CBL_E_CUDA;
         s.scratch = static_cast<unsigned char *>(p);
-        s.grid = sms * terms192_max_ctas_per_sm(256);
+        for (int l = 0; l < kTermLevels; ++l) s.grid[l] = sms * terms192_max_ctas_per_sm(l);
         s.ready = true;
     }
     *out = &s;
@@ -216,13 +216,15 @@ extern "C" int cbl_batch_noalloc(const uint64_t *pos, int n, uint64_t *d_out3n, 
     PositionArgs args;
     args.n = n;
     int nseg = 0;
-    uint64_t ntiles = 0, max_series_tiles = 0;
+    uint64_t ntiles = 0, max_series_tiles = 0, max_m = 0;
     for (int i = 0; i < n; ++i) {
         uint64_t d = 0;
         const int rc = cbl_pos_to_d(pos[i], &d, nullptr);
         if (rc) return rc;
         if ((u128)10 * (d + kTail192 - 1) + 9 >= (u128)kW2XMax) return CBL_E_POSITION;
         args.d[i] = d;
+        const uint64_t m_last = 10 * (d + kTail192 - 1) + 9;
+        max_m = max_m > m_last ? max_m : m_last;
         Piece p[kMaxPieces];
         for (int f = 0; f < 7; ++f) {
             const int np = series_pieces(d, f, p);
@@ -250,7 +252,8 @@ extern "C" int cbl_batch_noalloc(const uint64_t *pos, int n, uint64_t *d_out3n, 
     if (cudaMemsetAsync(base, 0, kOffSegs, st) != cudaSuccess) return CBL_E_CUDA;
     noalloc_table_kernel<<<1, kMaxPos, 0, st>>>(args, dsegs);
     if (cudaGetLastError() != cudaSuccess) return CBL_E_CUDA;
-    if (launch_terms192(dsegs, nseg, ntiles, (uint32_t)kTileTerms, counter, slots, ds->grid, 256, st, 0,
+    const int level = term_level(max_m);
+    if (launch_terms192(level, dsegs, nseg, ntiles, (uint32_t)kTileTerms, counter, slots, ds->grid[level], st, 0,
                         slot_needs_carry(max_series_tiles)) != cudaSuccess)
         return CBL_E_CUDA;
     if (launch_combine(slots, n, shift, d_out3n, nullptr, st) != cudaSuccess) return CBL_E_CUDA;
