@@ -15,9 +15,9 @@
 // step and no division is ever executed. The chain ends at r_0 = 2^(10e) mod m.
 //
 // Seven residue kinds:
-//   width 1 (m < 2^28): R = 2^32, residues kept lazily in [0, 4m).
-//   middle width 1 (2^28 <= m < 2^31): R = 2^32, residues in [0, m).
-//   strict width 1 (2^28 <= m < 2^32): R = 2^32, residues in [0, m), carries kept.
+//   width 1 (m < 2^25; the formulas hold below 2^28): R = 2^32, residues kept lazily in [0, 4m).
+//   middle width 1 (2^25 <= m < 2^31): R = 2^32, residues in [0, m).
+//   strict width 1 (2^31 <= m < 2^32): R = 2^32, signed residues.
 //   float-quotient width 2 (2^32 <= m < 94 * 2^32): R = 2^24, residues below 8m,
 //     the top of each square taken off by a float quotient.
 //   short width 2 (94 * 2^32 <= m < 2^44): R = 2^48, residues in [0, 4m).
@@ -214,38 +214,38 @@ __device__ __forceinline__ uint32_t w1_digits(uint32_t r, uint32_t m, uint32_t m
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
         q[j] = r * mp;
-        r = redc_word(q[j], m, r, 0u);                  // (r + q m) / 2^32 < m
+        r = __umulhi(q[j], m) + 1u;                     // (r + q m) / 2^32 < m: r > 0, so its low word carries
     }
     return r;
 }
 
 // --------------------------------------------------------- strict width 1 --
-// 2^31 <= m < 2^32: R = 2^32, residues in [0, m). The doubling comes first,
-// into the second multiplicand only: y2 = 2^b y, less m when the shift carries
-// out of bit 31, is below 2^32 (not necessarily below m), so t = y y2 < m 2^32.
-// u m + t can pass 2^64 once: the carry chain returns the carry c out of the
-// high word, REDC = x + c 2^32 < 2m, and one conditional subtraction brings it
-// below m. (Valid for 2^28 <= m < 2^32.)
-__device__ __forceinline__ uint32_t w1s_sqr(uint32_t y, uint32_t m, uint32_t mp, uint32_t b)
+// 2^31 <= m < 2^32: R = 2^32, signed residues -2^31 < y < 2^31 (every class mod m has
+// one). t = |y| (2^b |y|) < 2^63, and REDC by subtraction: with u = t0 m^-1 the low
+// words of t and u m are equal, so z = t1 - hi(u m) in (-m, 2^31) needs no carry.
+// z <= -2^31 takes one m more; with 2^31 added to hi(u m) inside the multiply
+// that is one signed compare. (The additive form in [0, m) paid for the carries
+// of both the doubling and the sum: about 9 more ALU cycles a step.)
+__device__ __forceinline__ int32_t w1s_sqr(int32_t y, uint32_t m, uint32_t ip, uint32_t b)
 {
-    const uint32_t x2 = y << b;
-    const uint32_t c2 = __funnelshift_l(y, 0u, b);                 // bit shifted out of y
-    const uint32_t y2 = c2 ? x2 - m : x2;                          // 2^b y mod m, < 2^32
-    const uint64_t t = (uint64_t)y * y2;
-    const uint32_t u = (uint32_t)t * mp;
-    uint32_t c;
-    const uint32_t x = redc_word_c(u, m, (uint32_t)t, (uint32_t)(t >> 32), c);
-    return c ? x - m : min(x, x - m);                              // REDC mod m, in [0, m)
+    const uint64_t t = (uint64_t)((int64_t)y * y) << b;             // < 2^63
+    const uint32_t u = (uint32_t)t * ip, t1 = (uint32_t)(t >> 32);
+    uint32_t h;                                                     // hi(u m) - 2^31, signed
+    asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(h) : "r"(u), "r"(m), "r"(0x80000000u));
+    const uint32_t c = (int32_t)h >= (int32_t)t1 ? m + 0x80000000u : 0x80000000u;
+    return (int32_t)(t1 - h + c);
 }
 
 struct W1SState {
-    uint32_t y, m, mp;
-    __device__ __forceinline__ void step(uint32_t b) { y = w1s_sqr(y, m, mp, b); }
+    int32_t y;
+    uint32_t m, ip;                                     // ip = m^-1 mod 2^32
+    __device__ __forceinline__ void step(uint32_t b) { y = w1s_sqr(y, m, ip, b); }
+    __device__ __forceinline__ uint32_t residue() const { return y < 0 ? (uint32_t)y + m : (uint32_t)y; }
 };
 
 
 // ------------------------------------------------------ middle width 1 --
-// 2^28 <= m < 2^31: R = 2^32, residues in [0, m). The doubling comes first:
+// 2^25 <= m < 2^31: R = 2^32, residues in [0, m). The doubling comes first:
 // t = y (2^b y) < 2m^2 < 2^63 and u m < 2^63, so the word step has no carry
 // out and REDC(t) = REDC(y^2) 2^b mod m is below 2m; one min(z, z - m)
 // brings it below m. (Two ALU operations fewer than reducing, then doubling
@@ -265,7 +265,7 @@ struct W1MState {
 
 // 2^(32 + p) mod m in [0, m), 1 <= p <= 15, 2^28 <= m < 2^32: q1 <= 2^19 is
 // off by at most one, so one correction either way suffices.
-__device__ __forceinline__ uint32_t w1m_start(uint32_t m, uint32_t p)
+__device__ __forceinline__ uint32_t w1s_start(uint32_t m, uint32_t p)
 {
     const float inv = rcp_approx(__uint2float_rn(m));
     const float scale = __int_as_float((int)((127u + 32u + p) << 23));
@@ -276,11 +276,24 @@ __device__ __forceinline__ uint32_t w1m_start(uint32_t m, uint32_t p)
     return (uint32_t)r;
 }
 
+// A value congruent to 2^(32 + p), 1 <= p <= 15, for 2^25 <= m < 2^31, below m from
+// 2^28 on and below 1.8m under it (w1m_sqr then still gives a sum below 2m). The float
+// quotient (< 2^22, three roundings of 2^-24: within 0.75, and 0.1 from 2^28 on) less
+// 0.8 is rounded down, so -q m mod 2^32 is the positive rest, below 2m from 2^28 on
+// and below 2.8m under it.
+__device__ __forceinline__ uint32_t w1m_start(uint32_t m, uint32_t p)
+{
+    const float inv = rcp_approx(__uint2float_rn(m));
+    const float scale = __int_as_float((int)((127u + 32u + p) << 23));
+    const uint32_t r = 0u - __float2uint_rz(__fmaf_rn(scale, inv, -0.8f)) * m;
+    return min(r, r - m);
+}
+
 struct W1MStart {
     __device__ __forceinline__ void operator()(W1MState &st, uint32_t p) const { st.y = w1m_start(st.m, p); }
 };
 
-// r6 = 2^E mod m in [0, m) for E >= 33, 2^28 <= m < 2^31. The start value
+// r6 = 2^E mod m in [0, m) for E >= 42, 2^25 <= m < 2^31. The start value
 // takes the leading up-to-four bits of E - 32 at once.
 __device__ __forceinline__ uint32_t w1m_pow2(uint64_t E, uint32_t m, uint32_t mp)
 {
@@ -290,16 +303,20 @@ __device__ __forceinline__ uint32_t w1m_pow2(uint64_t E, uint32_t m, uint32_t mp
 }
 
 struct W1SStart {
-    __device__ __forceinline__ void operator()(W1SState &st, uint32_t p) const { st.y = w1m_start(st.m, p); }
+    __device__ __forceinline__ void operator()(W1SState &st, uint32_t p) const
+    {
+        const uint32_t r = w1s_start(st.m, p);
+        st.y = (int32_t)(r >> 31 ? r - st.m : r);
+    }
 };
 
 // r6 = 2^E mod m in [0, m) for E >= 33 (2^31 <= m < 2^32), from the same
 // 4-bit start value.
 __device__ __forceinline__ uint32_t w1s_pow2(uint64_t E, uint32_t m, uint32_t mp)
 {
-    W1SState st{0, m, mp};
+    W1SState st{0, m, 0u - mp};
     walk_bits_start<4>(E - 32, st, W1SStart{});
-    return st.y;
+    return st.residue();
 }
 
 // ---------------------------------------------------------------- width 2 --
@@ -604,7 +621,7 @@ __device__ __forceinline__ void w2f_pow2_pair(uint64_t EA, uint64_t ma, uint32_t
 #pragma unroll
         for (int l = S - 1; l >= 0; --l) {
             A.step(la >> l & 1u);
-            B.step(lb >> l & 1u);
+            B.step((l < 6 ? la : lb) >> l & 1u);        // EA - EB = 320 = 5 * 2^6
         }
         ra = A.finish(ma);
         rb = B.finish(mb);
@@ -700,6 +717,40 @@ __device__ __forceinline__ void walk_bits_start_pair(uint64_t EpA, uint64_t EpB,
             B.step((lb >> i) & 1u);
         }
     }
+}
+
+// Two ladders of a warp's group of 64 terms (k and k+32 of every lane; ep_max the
+// group's largest exponent, 630 above its smallest). When the group's exponents
+// agree above bit S, those bits come from one word P and both ladders share the
+// shift counts, and so they do in the last six bits (EpA - EpB = 320 = 5 * 2^6).
+// Other groups, and exponents outside [2^(S+4) + 630, 2^(S+32)), walk their own bits.
+// S: 12 / 13 / 14 / 15 measured 127.0 / 125.9 / 125.1 / 125.2 ms on 512 positions below 1e8.
+constexpr int kGroupBits = 14;
+template <int NB, typename State, typename Start>
+__device__ __forceinline__ void walk_bits_group(uint64_t EpA, uint64_t EpB, uint64_t ep_max, State &A, State &B,
+                                                Start start)
+{
+    constexpr int S = kGroupBits;
+    const uint32_t P = (uint32_t)(ep_max >> S);
+    if (ep_max >= (1ull << (S + 4)) + 630 && ep_max >> (S + 32) == 0 && (uint32_t)((ep_max - 630) >> S) == P) {
+        int j = 32 - NB - __clz(P);
+        start(A, P >> j);
+        start(B, P >> j);
+#pragma unroll 4
+        for (--j; j >= 0; --j) {
+            const uint32_t b = (P >> j) & 1u;
+            A.step(b);
+            B.step(b);
+        }
+        const uint32_t la = (uint32_t)EpA, lb = (uint32_t)EpB;
+#pragma unroll
+        for (int l = S - 1; l >= 0; --l) {
+            A.step((la >> l) & 1u);
+            B.step(((l < 6 ? la : lb) >> l) & 1u);
+        }
+        return;
+    }
+    walk_bits_start_pair<NB>(EpA, EpB, A, B, start);
 }
 
 struct W1Start1 {                                        // the single-bit start of the width-1 kind

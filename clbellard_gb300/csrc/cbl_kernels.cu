@@ -48,7 +48,7 @@ __device__ __forceinline__ void shr192(uint32_t q[6], int s)
 
 // One term's six quotient digits: k < d gives frac(2^(10(d-k))/m), k >= d the
 // tail value 2^(-10(k-d))/m (digits of 1/m shifted right by 10(k-d)).
-// KIND: 1 = width 1 (m < 2^28), 5 = middle width 1 (2^28 <= m < 2^31),
+// KIND: 1 = width 1 (m < 2^28), 5 = middle width 1 (2^25 <= m < 2^31),
 // 3 = strict width 1 (2^28 <= m < 2^32), 7 and 8 = float-quotient width 2 (2^32 <= m
 // < 15 * 2^34 and < 94 * 2^32), 4 = short width 2 (2^32 <= m < 2^44),
 // 2 = width 2 (2^28 <= m < 2^60), 6 = wide width 2 (2^60 <= m < 2^62).
@@ -82,22 +82,21 @@ __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, 
     if (TAIL) shr192(q, (int)(10 * (k - d)));
 }
 
-// Two terms (ka and ka+32) of a lane per iteration, their ladders interleaved
+// Two terms (exponents Ea and Ea - 320) of a lane per iteration, their ladders interleaved
 // (kinds 1, 3, 4, 5, 7, 8; the width-2 kinds above 2^44 run one term at a time).
-// The warp's 64 terms are k .. k+63.
+// e_max is the largest exponent of the warp's 64.
 // Same-box timings against one term per iteration, identical bits: 1e9
 // 40.65 -> 38.55 ms, 1e10 841.0 -> 838.9 ms, batch 10.61 -> 10.08 s. Pairing
 // only some kinds traded these against each other (the kernel's code layout
 // and registers change with every instantiation), so all four are paired.
 template <int KIND>
-__device__ __forceinline__ void term_pair(uint64_t d, uint64_t k, uint64_t ka, uint64_t ma, uint64_t mb,
-                                          uint32_t qa[6], uint32_t qb[6])
+__device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t ma, uint64_t mb, uint32_t qa[6],
+                                          uint32_t qb[6])
 {
     const uint32_t mpa = neg_inv32((uint32_t)ma), mpb = neg_inv32((uint32_t)mb);
-    const uint64_t Ea = 10ull * (d - ka) + 192ull, Eb = Ea - 320ull;
+    const uint64_t Eb = Ea - 320ull;
     if (KIND == 7 || KIND == 8) {
         uint64_t ra, rb;
-        const uint64_t e_max = 10ull * (d - k) + 192ull;
         w2f_pow2_pair<KIND == 8>(Ea, ma, mpa, Eb, mb, mpb, e_max, ra, rb);
         w2_digits(ra, ma, mpa, qa);
         w2_digits(rb, mb, mpb, qb);
@@ -113,7 +112,7 @@ __device__ __forceinline__ void term_pair(uint64_t d, uint64_t k, uint64_t ka, u
         w2_digits(rb, mb, mpb, qb);
     } else if (KIND == 1) {
         W1State A{0, (uint32_t)ma, mpa}, B{0, (uint32_t)mb, mpb};
-        walk_bits_start_pair<1>(Ea - 32, Eb - 32, A, B, W1Start1{});
+        walk_bits_group<1>(Ea - 32, Eb - 32, e_max - 32, A, B, W1Start1{});
         uint32_t ya = A.y, yb = B.y;
         ya = min(ya, ya - 2u * (uint32_t)ma);
         ya = min(ya, ya - (uint32_t)ma);
@@ -123,14 +122,14 @@ __device__ __forceinline__ void term_pair(uint64_t d, uint64_t k, uint64_t ka, u
         w1_digits(yb, (uint32_t)mb, mpb, qb);
     } else if (KIND == 5) {
         W1MState A{0, (uint32_t)ma, mpa}, B{0, (uint32_t)mb, mpb};
-        walk_bits_start_pair<4>(Ea - 32, Eb - 32, A, B, W1MStart{});
+        walk_bits_group<4>(Ea - 32, Eb - 32, e_max - 32, A, B, W1MStart{});
         w1_digits(A.y, (uint32_t)ma, mpa, qa);
         w1_digits(B.y, (uint32_t)mb, mpb, qb);
     } else {
-        W1SState A{0, (uint32_t)ma, mpa}, B{0, (uint32_t)mb, mpb};
-        walk_bits_start_pair<4>(Ea - 32, Eb - 32, A, B, W1SStart{});
-        w1_digits(A.y, (uint32_t)ma, mpa, qa);
-        w1_digits(B.y, (uint32_t)mb, mpb, qb);
+        W1SState A{0, (uint32_t)ma, 0u - mpa}, B{0, (uint32_t)mb, 0u - mpb};
+        walk_bits_group<4>(Ea - 32, Eb - 32, e_max - 32, A, B, W1SStart{});
+        w1_digits(A.residue(), (uint32_t)ma, mpa, qa);
+        w1_digits(B.residue(), (uint32_t)mb, mpb, qb);
     }
 }
 
@@ -140,11 +139,19 @@ __device__ __forceinline__ void run_tile(const Seg &s, uint64_t kb, uint64_t ke,
 {
     uint64_t k = kb + lane;
     if (!TAIL && (KIND == 1 || KIND == 3 || KIND == 4 || KIND == 5 || KIND == 7 || KIND == 8)) {
-        uint64_t k0 = kb;
-        for (; k0 + 64 <= ke; k += 64, k0 += 64) {                  // terms k and k+32 together
-            const uint64_t ma = (uint64_t)s.den0 * k + s.den1, mb = ma + 32ull * s.den0;
+        constexpr bool wide = KIND == 4 || KIND == 7 || KIND == 8;
+        uint64_t ea = 10ull * (s.d - k) + 192ull, ma = (uint64_t)s.den0 * k + s.den1;
+        uint64_t e_max = ea + 10u * lane;
+        const uint64_t m32 = 32ull * s.den0;
+        for (uint32_t n = (uint32_t)(ke - kb) >> 6; n > 0; --n) {   // terms k and k+32 together
             uint32_t qa[6], qb[6];
-            term_pair<KIND>(s.d, k0, k, ma, mb, qa, qb);
+            // e_max kept in registers cost the two-word kinds more than its two adds
+            // (1e10: 550.1 against 542.6 ms) and gained on the one-word kinds (1e9: 32.7 to 32.2 ms)
+            term_pair<KIND>(ea, wide ? ea + 10u * lane : e_max, ma, ma + m32, qa, qb);
+            e_max -= 640;
+            ma += 2 * m32;
+            ea -= 640;
+            k += 64;
             acc_add(acc, qa);
             acc_add(acc, qb);
             cnt += 2;
@@ -233,7 +240,9 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
                                               uint32_t &cnt)
 {
     const int width = (int)((s.flags >> 4) & 15u);
-    if (LEVEL >= 1 && width == 4) {
+    if (LEVEL == 2 && width == 4) {
+        run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
+    } else if (LEVEL == 1 && width == 4) {
         const uint64_t m_last = (uint64_t)s.den0 * (ke - 1) + s.den1;
         const bool fq = TAIL || 10 * (s.d - kb) + 192 < kW2FExp;
         if (fq && m_last < kW2FLow) run_tile<7, TAIL>(s, kb, ke, lane, acc, cnt);
@@ -242,7 +251,7 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
     } else if (LEVEL >= 2 && width == 2) run_tile<2, TAIL>(s, kb, ke, lane, acc, cnt);
     else if (LEVEL >= 2 && width == 6) run_tile<6, TAIL>(s, kb, ke, lane, acc, cnt);
     else if (width == 3) run_tile<3, TAIL>(s, kb, ke, lane, acc, cnt);
-    else if (width == 5) run_tile<5, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (width == 5 || (uint64_t)s.den0 * kb + s.den1 >= kW1MMin) run_tile<5, TAIL>(s, kb, ke, lane, acc, cnt);
     else run_tile<1, TAIL>(s, kb, ke, lane, acc, cnt);
 }
 
@@ -454,7 +463,7 @@ __global__ void terms_each_kernel(uint64_t d, uint32_t den0, uint32_t den1, int 
     uint32_t q[6] = {0, 0, 0, 0, 0, 0};
     if (m != 1) {
         if (k < d) {
-            if (m < kW1Max) term_digits<1, false>(d, k, m, q);
+            if (m < kW1MMin) term_digits<1, false>(d, k, m, q);
             else if (m < kW1MMax) term_digits<5, false>(d, k, m, q);
             else if (m < kW1SMax) term_digits<3, false>(d, k, m, q);
             else if (m < kW2FLow) term_digits<7, false>(d, k, m, q);
@@ -463,7 +472,7 @@ __global__ void terms_each_kernel(uint64_t d, uint32_t den0, uint32_t den1, int 
             else if (m < kW2Max) term_digits<2, false>(d, k, m, q);
             else term_digits<6, false>(d, k, m, q);
         } else {
-            if (m < kW1Max) term_digits<1, true>(d, k, m, q);
+            if (m < kW1MMin) term_digits<1, true>(d, k, m, q);
             else if (m < kW1MMax) term_digits<5, true>(d, k, m, q);
             else if (m < kW1SMax) term_digits<3, true>(d, k, m, q);
             else if (m < kW2SMax) term_digits<4, true>(d, k, m, q);
@@ -582,7 +591,7 @@ __global__ void __launch_bounds__(kBlockDD) dd_terms_kernel(double2 *bigsum, uin
         uint64_t r;
         if (m < kW1SMax) {
             uint32_t y;
-            if (m < kW1Max) y = w1_pow2(e + 32, (uint32_t)m, mp);
+            if (m < kW1MMin) y = w1_pow2(e + 32, (uint32_t)m, mp);
             else if (m < kW1MMax) y = w1m_pow2(e + 32, (uint32_t)m, mp);
             else y = w1s_pow2(e + 32, (uint32_t)m, mp);
             r = redc_word(y * mp, (uint32_t)m, y, 0u);
