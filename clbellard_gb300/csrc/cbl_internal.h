@@ -61,6 +61,12 @@ inline uint32_t seg_flags(int sign, int width) { return (uint32_t)(sign & 1) | (
 constexpr int kTermLevels = 3;
 __host__ __device__ inline int term_level(uint64_t max_m) { return max_m < kW1SMax ? 0 : max_m < kW2SMax ? 1 : 2; }
 
+// How a pass without a time budget deals its tiles out: from the tile counter, or
+// (fixed) as 2^log2_parts parts of part_k terms each, one contiguous share a block.
+struct TileSplit {
+    uint32_t log2_parts, fixed, part_k;
+};
+
 // Launch wrappers (cbl_kernels.cu).
 // budget_ns = 0: run to the end; else warps stop taking tiles after budget_ns
 // and the finished tiles are [0, *counter).

@@ -11,6 +11,7 @@
 //                    1118-1144, 1274-1353), the only FP64 on the GPU.
 #include "cbl_arith.cuh"
 #include "cbl_internal.h"
+#include <algorithm>
 
 namespace cbl {
 
@@ -183,34 +184,36 @@ __device__ __forceinline__ void slot_add(unsigned long long *slot6, int j, unsig
     }
 }
 
-// Warp sum of the lanes' 192-bit values, normalised, added into a slot's six
-// 64-bit digit sums. Each add is < 2^32, so a slot that receives fewer than
+// Digit sums S (each below 2^56), normalised, added into a slot's six 64-bit
+// digit sums. Each add is < 2^32, so a slot that receives fewer than
 // 2^32 flushes from zero cannot wrap and takes plain fire-and-forget adds;
 // with carry set (a slot that may receive 2^31 or more flushes, or a preset
 // start value) slot_add carries the wraps, and the number of flushes per slot
 // is unbounded.
-__device__ __forceinline__ void warp_flush(const Acc192 &acc, int lane, unsigned long long *slot6, int carry)
+__device__ __forceinline__ void add_digits(const uint64_t S[6], unsigned long long *slot6, int carry)
 {
-    uint64_t S[6];
+    uint64_t c = 0;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
-        const uint32_t lo = __reduce_add_sync(0xffffffffu, acc.w[j] & 0xffffu);
-        const uint32_t hi = __reduce_add_sync(0xffffffffu, acc.w[j] >> 16);
-        S[j] = (uint64_t)lo + ((uint64_t)hi << 16);
-    }
-    if (lane == 0) {
-        uint64_t c = 0;
-#pragma unroll
-        for (int j = 0; j < 6; ++j) {
-            const uint64_t t = S[j] + c;
-            const uint32_t dj = (uint32_t)t;
-            c = t >> 32;
-            if (dj) {
-                if (carry) slot_add(slot6, j, (unsigned long long)dj);
-                else atomicAdd(slot6 + j, (unsigned long long)dj);
-            }
+        const uint64_t t = S[j] + c;
+        const uint32_t dj = (uint32_t)t;
+        c = t >> 32;
+        if (dj) {
+            if (carry) slot_add(slot6, j, (unsigned long long)dj);
+            else atomicAdd(slot6 + j, (unsigned long long)dj);
         }
     }
+}
+
+// Sums over a warp's lanes of the low and high halves of digit j.
+__device__ __forceinline__ uint32_t warp_low(const Acc192 &acc, int j)
+{
+    return __reduce_add_sync(0xffffffffu, acc.w[j] & 0xffffu);
+}
+
+__device__ __forceinline__ uint32_t warp_high(const Acc192 &acc, int j)
+{
+    return __reduce_add_sync(0xffffffffu, acc.w[j] >> 16);
 }
 
 __device__ __forceinline__ uint64_t global_ns()
@@ -224,11 +227,50 @@ __device__ __forceinline__ uint64_t global_ns()
 // Fold a warp's accumulated terms of one segment and add them into its slot.
 // Every k of a lane has the parity of seg.k0 + lane (tiles hold an even number
 // of terms), so the lane's sign (-1)^(k + sign) is fixed for the segment.
+__device__ __forceinline__ void fold_sign(const Seg &s, int lane, Acc192 &acc, uint32_t cnt)
+{
+    if (((s.k0 + (uint64_t)lane + (s.flags & kFlagSign)) & 1ull) != 0) acc_negate_minus(acc, cnt);
+}
+
 __device__ __forceinline__ void flush_segment(const Seg &s, int lane, Acc192 &acc, uint32_t cnt,
                                               unsigned long long *slots, int carry)
 {
-    if (((s.k0 + (uint64_t)lane + (s.flags & kFlagSign)) & 1ull) != 0) acc_negate_minus(acc, cnt);
-    warp_flush(acc, lane, slots + (size_t)s.slot * 6, carry);
+    fold_sign(s, lane, acc, cnt);
+    uint64_t S[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) S[j] = (uint64_t)warp_low(acc, j) + ((uint64_t)warp_high(acc, j) << 16);
+    if (lane == 0) add_digits(S, slots + (size_t)s.slot * 6, carry);
+}
+
+// The last flush of a block whose warps shared one run of tiles: warps still
+// in warp 0's segment add up in shared memory first, so the block updates the slot once.
+__device__ __forceinline__ void flush_block(const Seg *segs, int cur, int lane, Acc192 &acc, uint32_t cnt,
+                                            unsigned long long *slots, int carry)
+{
+    __shared__ uint32_t half[12];
+    __shared__ int seg0;
+    if (threadIdx.x < 12) half[threadIdx.x] = 0;
+    if (threadIdx.x == 0) seg0 = cur;
+    __syncthreads();
+    if (cur >= 0 && cur != seg0) flush_segment(segs[cur], lane, acc, cnt, slots, carry);
+    else if (cur >= 0) {
+        fold_sign(segs[cur], lane, acc, cnt);
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            const uint32_t lo = warp_low(acc, j), hi = warp_high(acc, j);
+            if (lane == 0) {
+                atomicAdd(&half[2 * j], lo);
+                atomicAdd(&half[2 * j + 1], hi);
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && seg0 >= 0) {
+        uint64_t S[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) S[j] = (uint64_t)half[2 * j] + ((uint64_t)half[2 * j + 1] << 16);
+        add_digits(S, slots + (size_t)segs[seg0].slot * 6, carry);
+    }
 }
 
 // One tile's terms, by residue kind and main body / tail. LEVEL limits the kinds
@@ -262,7 +304,7 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
 // A warp keeps its lanes' sums across consecutive tiles of one segment and
 // flushes them when it moves to another segment, when a lane's term count
 // reaches 2^30, and before it exits: one slot update per run of tiles
-// instead of one per tile.
+// instead of one per tile. (split: see tile_split.)
 // Registers: the one-word kinds run best at 5 CTAs an SM with 46 registers (1e9:
 // 35.9 ms; 37.4 ms with the 40 that ptxas takes unbounded, 36.2 ms at 4 CTAs),
 // the float-quotient kind at 64 registers and 4 CTAs (1e10: 561.7 ms; 591 ms when held
@@ -270,25 +312,33 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
 // two-word kinds at 5 CTAs (2^27 terms at 1e13: 5.81 ms against 5.96 ms at 4).
 template <int LEVEL>
 __global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel(const Seg *__restrict__ segs, int nseg,
-                                                             uint64_t ntiles, uint32_t tile_k,
+                                                             uint64_t ntiles, uint32_t tile_k, TileSplit split,
                                                              unsigned long long *counter,
                                                              unsigned long long *slots, uint64_t budget_ns,
                                                              int carry)
 {
     const int lane = threadIdx.x & 31;
     const uint64_t t_start = budget_ns ? global_ns() : 0;
+    uint64_t nitems = ntiles << split.log2_parts, item = 0;
+    if (split.fixed) {                              // this block's share, dealt to its warps in turn
+        item = nitems * blockIdx.x / gridDim.x + (threadIdx.x >> 5);
+        nitems = nitems * (blockIdx.x + 1) / gridDim.x;
+    }
     int cur = -1;                                   // segment of the sums held in acc
     Acc192 acc;
     acc_zero(acc);
     uint32_t cnt = 0;
-    for (;;) {
-        unsigned long long t = 0;
-        if (lane == 0) {
-            if (budget_ns && global_ns() - t_start > budget_ns) t = ~0ull;
-            else t = atomicAdd(counter, 1ull);
+    for (;; item += kBlock192 / 32) {
+        if (!split.fixed) {
+            unsigned long long t = 0;
+            if (lane == 0) {
+                if (budget_ns && global_ns() - t_start > budget_ns) t = ~0ull;
+                else t = atomicAdd(counter, 1ull);
+            }
+            item = __shfl_sync(0xffffffffu, t, 0);
         }
-        t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= ntiles) break;
+        if (item >= nitems) break;
+        const uint64_t t = item >> split.log2_parts;
         int lo = 0, hi = nseg - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -301,27 +351,54 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel
             cur = lo;
         }
         const Seg s = segs[lo];
-        const uint64_t kb = s.k0 + (t - s.tile0) * tile_k;
-        const uint64_t ke = min(s.k1, kb + tile_k);
+        const uint64_t k0 = s.k0 + (t - s.tile0) * tile_k;
+        const uint64_t kb = k0 + ((uint32_t)item & ((1u << split.log2_parts) - 1u)) * split.part_k;
+        const uint64_t ke = min(min(s.k1, k0 + tile_k), kb + split.part_k);
+        if (kb >= ke) continue;
         if (kb >= s.d) run_tile_kind<LEVEL, true>(s, kb, ke, lane, acc, cnt);
         else run_tile_kind<LEVEL, false>(s, kb, ke, lane, acc, cnt);
     }
-    if (cur >= 0) flush_segment(segs[cur], lane, acc, cnt, slots, carry);
+    if (split.fixed) flush_block(segs, cur, lane, acc, cnt, slots, carry);
+    else if (cur >= 0) flush_segment(segs[cur], lane, acc, cnt, slots, carry);
 }
 
-typedef void (*Terms192Fn)(const Seg *, int, uint64_t, uint32_t, unsigned long long *, unsigned long long *, uint64_t,
-                           int);
+typedef void (*Terms192Fn)(const Seg *, int, uint64_t, uint32_t, TileSplit, unsigned long long *, unsigned long long *,
+                           uint64_t, int);
 
 static Terms192Fn terms192_fn(int level)
 {
     return level == 0 ? terms192_kernel<0> : level == 1 ? terms192_kernel<1> : terms192_kernel<2>;
 }
 
+// A pass with fewer tiles than resident warps leaves most of the GPU idle and its
+// lanes a long serial run (position 1e6: 1367 tiles for 6080 warps, 64 terms a
+// lane). Its tiles are cut into parts of down to 64 terms, about four a warp, and
+// every block takes one contiguous share: no counter to wait for, and one slot
+// update a block instead of one a part (those queue at three cache lines: 141 us
+// at 1e6). Measured, term kernel: 1e4 24.5 -> 8 us, 1e5 39 -> 10.4 us, 1e6 52 -> 39 us,
+// 2^20 terms at 1e11 187 -> 64 us. From one tile a warp on, contiguous shares lose to
+// the counter (1e7 268 -> 274 us, 1e8 2.61 -> 2.82 ms): costs differ along the table.
+TileSplit tile_split(uint64_t ntiles, uint32_t tile_k, int grid)
+{
+    const uint64_t warps = (uint64_t)grid * (kBlock192 / 32);
+    TileSplit sp{0, 0, tile_k};
+    if (ntiles >= warps) return sp;
+    sp.fixed = 1;
+    while (sp.part_k > 64 && (ntiles << sp.log2_parts) < 4 * warps) {
+        ++sp.log2_parts;
+        sp.part_k = ((tile_k >> sp.log2_parts) + 63) / 64 * 64;
+    }
+    return sp;
+}
+
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
                             unsigned long long *counter, unsigned long long *slots, int grid, cudaStream_t st,
                             uint64_t budget_ns, bool carry)
 {
-    terms192_fn(level)<<<grid, kBlock192, 0, st>>>(segs, nseg, ntiles, tile_k, counter, slots, budget_ns,
+    // a budgeted pass stops and resumes at whole tiles
+    const TileSplit sp = budget_ns ? TileSplit{0, 0, tile_k} : tile_split(ntiles, tile_k, grid);
+    if (sp.fixed) grid = (int)std::min<uint64_t>(grid, ntiles << sp.log2_parts);
+    terms192_fn(level)<<<grid, kBlock192, 0, st>>>(segs, nseg, ntiles, tile_k, sp, counter, slots, budget_ns,
                                                    carry ? 1 : 0);
     return cudaGetLastError();
 }
