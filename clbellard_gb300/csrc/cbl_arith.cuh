@@ -207,12 +207,13 @@ __device__ __forceinline__ uint32_t w1_pow2(uint64_t E, uint32_t m, uint32_t mp)
     return y;
 }
 
-// Six quotient digits of r_0 / m from r6 (digit 0 least significant), and r_0.
-// Valid for any odd m < 2^32.
-__device__ __forceinline__ uint32_t w1_digits(uint32_t r, uint32_t m, uint32_t mp, uint32_t q[6])
+// N quotient digits of r_0 / m from r_N (digit 0 least significant), and r_0.
+// Valid for any odd m < 2^32, m > 1.
+template <int N>
+__device__ __forceinline__ uint32_t w1_digits(uint32_t r, uint32_t m, uint32_t mp, uint32_t q[N])
 {
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
+    for (int j = 0; j < N; ++j) {
         q[j] = r * mp;
         r = __umulhi(q[j], m) + 1u;                     // (r + q m) / 2^32 < m: r > 0, so its low word carries
     }
@@ -682,11 +683,6 @@ __device__ __forceinline__ uint64_t w2_redc_down(uint64_t r, uint64_t m, uint32_
     return ((uint64_t)r1 << 32) | r0;
 }
 
-__device__ __forceinline__ uint64_t w2_digits(uint64_t r, uint64_t m, uint32_t mp, uint32_t q[6])
-{
-    return w2_redc_down<6>(r, m, mp, q);
-}
-
 // Two ladders at once (terms k and k+32 of one lane): when both exponents have
 // the same bit length (in the same word) the steps interleave, giving the
 // scheduler two independent chains; otherwise they run one after the other.
@@ -767,18 +763,22 @@ struct W2SStart {
 };
 
 // ------------------------------------------------------------ fixed point --
-// 192-bit accumulator as six 32-bit digits, digit 0 least significant.
-struct Acc192 {
-    uint32_t w[6];
+// Accumulator of N 32-bit digits, digit 0 least significant: 192 bits for the
+// integer mode, 128 for the double-double mode's terms.
+template <int N>
+struct Acc {
+    uint32_t w[N];
 };
+typedef Acc<6> Acc192;
 
-__device__ __forceinline__ void acc_zero(Acc192 &a)
+template <int N>
+__device__ __forceinline__ void acc_zero(Acc<N> &a)
 {
 #pragma unroll
-    for (int j = 0; j < 6; ++j) a.w[j] = 0;
+    for (int j = 0; j < N; ++j) a.w[j] = 0;
 }
 
-__device__ __forceinline__ void acc_add(Acc192 &a, const uint32_t q[6])
+__device__ __forceinline__ void acc_add(Acc<6> &a, const uint32_t q[6])
 {
     asm("add.cc.u32  %0, %0, %6;\n\t"
         "addc.cc.u32 %1, %1, %7;\n\t"
@@ -788,6 +788,26 @@ __device__ __forceinline__ void acc_add(Acc192 &a, const uint32_t q[6])
         "addc.u32    %5, %5, %11;"
         : "+r"(a.w[0]), "+r"(a.w[1]), "+r"(a.w[2]), "+r"(a.w[3]), "+r"(a.w[4]), "+r"(a.w[5])
         : "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3]), "r"(q[4]), "r"(q[5]));
+}
+
+__device__ __forceinline__ void acc_add(Acc<4> &a, const uint32_t q[4])
+{
+    asm("add.cc.u32  %0, %0, %4;\n\t"
+        "addc.cc.u32 %1, %1, %5;\n\t"
+        "addc.cc.u32 %2, %2, %6;\n\t"
+        "addc.u32    %3, %3, %7;"
+        : "+r"(a.w[0]), "+r"(a.w[1]), "+r"(a.w[2]), "+r"(a.w[3])
+        : "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3]));
+}
+
+// a <- -a (mod 2^128).
+__device__ __forceinline__ void acc_negate(Acc<4> &a)
+{
+    asm("sub.cc.u32  %0, 0, %0;\n\t"
+        "subc.cc.u32 %1, 0, %1;\n\t"
+        "subc.cc.u32 %2, 0, %2;\n\t"
+        "subc.u32    %3, 0, %3;"
+        : "+r"(a.w[0]), "+r"(a.w[1]), "+r"(a.w[2]), "+r"(a.w[3]));
 }
 
 // a <- -a - c (mod 2^192): the sum of c negative terms NOT(q_i) = -q_i - 1.

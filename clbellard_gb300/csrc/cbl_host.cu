@@ -73,6 +73,7 @@ struct cbl_ctx {
     std::vector<int> prep_shift;
     // double-double buffers
     double2 *d_bigsum = nullptr;
+    int dd_blocks = 1;                               // leading bigSum entries in use since cbl_Set0mem (the tail's at least)
     double2 *d_ddpartial = nullptr;
     double2 *d_ddans = nullptr;
     // scratch host
@@ -229,12 +230,15 @@ int grid_192(const cbl_ctx *c, int level)
     return std::max(1, c->sm_count * per);
 }
 
-// Term-kernel level of a set of segments, from their largest modulus.
+// Term-kernel level of a set of segments.
 int segs_level(const std::vector<Seg> &v)
 {
-    int level = 0;
-    for (const Seg &s : v) level = std::max(level, term_level((uint64_t)s.den0 * (s.k1 - 1) + s.den1));
-    return level;
+    uint64_t lo = UINT64_MAX, hi = 0;
+    for (const Seg &s : v) {
+        lo = std::min(lo, (uint64_t)s.den0 * s.k0 + s.den1);
+        hi = std::max(hi, (uint64_t)s.den0 * (s.k1 - 1) + s.den1);
+    }
+    return term_level(lo, hi);
 }
 
 // Upload segments and run the persistent term kernel (accumulates into slots).
@@ -262,11 +266,16 @@ int run_segments(cbl_ctx *c, std::vector<Seg> &v)
 int dd_range(cbl_ctx *c, uint64_t k0, uint64_t k1, uint64_t d, int sign, uint32_t den0, uint32_t den1)
 {
     if (k1 > k0 && (u128)den0 * (k1 - 1) + den1 >= (u128)kW2XMax) return CBL_E_POSITION;
+    if (k0 == 0 && den1 == 1) k0 = 1;                    // m = 1 contributes exactly 0
     // chunks of 2^30 terms keep each launch to a bounded time
     const uint64_t chunk = 1ull << 30;
     for (uint64_t a = k0; a < k1; a += chunk) {
         const uint64_t b = std::min(k1, a + chunk);
-        CK(launch_dd_terms(c->d_bigsum, kDDBlocks, 256, a, b, d, sign, den0, den1, c->st));
+        const int level = term_level((uint64_t)den0 * a + den1, (uint64_t)den0 * (b - 1) + den1);
+        const int grid = std::min(kDDBlocks, c->sm_count * dd_terms_max_ctas_per_sm(level));
+        int blocks = 0;
+        CK(launch_dd_terms(level, c->d_bigsum, grid, &blocks, a, b, d, sign, den0, den1, c->st));
+        c->dd_blocks = std::max(c->dd_blocks, blocks);
         c->launches++;
     }
     return CBL_OK;
@@ -563,6 +572,7 @@ int cbl_Set0mem(cbl_ctx *c)
         c->slot0_tiles = 0;
     } else {
         CK(cudaMemsetAsync(c->d_bigsum, 0, sizeof(double2) * kDDBlocks, c->st));
+        c->dd_blocks = 1;
     }
     return CBL_OK;
     CBL_GUARD_END
@@ -635,7 +645,7 @@ int cbl_Ssum(cbl_ctx *c)
     if (!c) return CBL_E_ARG;
     cudaSetDevice(c->device);
     if (is192(c)) CK(launch_ssum192(c->d_slots, c->d_partial, c->st));
-    else CK(launch_dd_ssum(c->d_bigsum, kDDBlocks, c->d_ddpartial, c->st));
+    else CK(launch_dd_ssum(c->d_bigsum, c->dd_blocks, c->d_ddpartial, c->st));
     c->launches++;
     return CBL_OK;
     CBL_GUARD_END
@@ -1349,7 +1359,7 @@ int cbl_autotune(cbl_ctx *c, const uint64_t *pos, int n, int force, int *best_ti
             if (rc) return rc;
             d_max = std::max(d_max, d);
         }
-        const int occ = terms192_max_ctas_per_sm(term_level(10 * (d_max + kTail192) + 9));
+        const int occ = terms192_max_ctas_per_sm(term_level(0, 10 * (d_max + kTail192) + 9));
         const int tiles[] = {512, 1024, 2048, 4096, 8192};
         ms_best = 1e300;
         for (int t : tiles) {

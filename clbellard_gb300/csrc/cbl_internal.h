@@ -55,11 +55,17 @@ static_assert(sizeof(Seg) == 48, "Seg layout");
 constexpr uint32_t kFlagSign = 1u;
 inline uint32_t seg_flags(int sign, int width) { return (uint32_t)(sign & 1) | ((uint32_t)width << 4); }
 
-// Widest residues of a table's segments, which picks the term kernel's
-// instantiation: 0 one-word kinds only (m < 2^32), 1 up to the short two-word
-// kind (m < 2^44), 2 any. A wider level than needed is slower, never wrong.
+// Instantiation of the term kernel for a table whose moduli lie in [min_m, max_m]:
+// 0 one-word kinds only (m < 2^32), 1 also the float-quotient and short two-word
+// kinds (m < 2^44), 2 any kind but without the float-quotient steps (moduli below
+// 94 * 2^32 take the short kind's there). Short two-word terms run 2 % faster at
+// level 2 (48 registers, 5 CTAs an SM) than beside the float-quotient steps at level 1,
+// so a table without moduli for those takes level 2.
 constexpr int kTermLevels = 3;
-__host__ __device__ inline int term_level(uint64_t max_m) { return max_m < kW1SMax ? 0 : max_m < kW2SMax ? 1 : 2; }
+__host__ __device__ inline int term_level(uint64_t min_m, uint64_t max_m)
+{
+    return max_m < kW1SMax ? 0 : max_m < kW2SMax && min_m < kW2FMax ? 1 : 2;
+}
 
 // How a pass without a time budget deals its tiles out: from the tile counter, or
 // (fixed) as 2^log2_parts parts of part_k terms each, one contiguous share a block.
@@ -97,9 +103,11 @@ cudaError_t launch_sum7_192(uint64_t *partial, uint64_t *ans, int numer_log2, cu
 cudaError_t launch_terms_each(uint64_t d, uint32_t den0, uint32_t den1, int sign, const uint64_t *k,
                               int n, uint64_t *out3n, cudaStream_t st);
 
-// Double-double (mode 0) kernels.
-cudaError_t launch_dd_terms(double2 *bigsum, int nblk, int block, uint64_t k0, uint64_t k1,
-                            uint64_t d, int sign, uint32_t den0, uint32_t den1, cudaStream_t st);
+// Double-double (mode 0) kernels. launch_dd_terms runs at most `grid` blocks (one
+// wave), block i adding into bigsum[i]; *blocks = the number launched.
+cudaError_t launch_dd_terms(int level, double2 *bigsum, int grid, int *blocks, uint64_t k0, uint64_t k1, uint64_t d,
+                            int sign, uint32_t den0, uint32_t den1, cudaStream_t st);
+int dd_terms_max_ctas_per_sm(int level);
 cudaError_t launch_dd_tail(double2 *bigsum, uint64_t d, int sign, uint32_t den0, uint32_t den1,
                            cudaStream_t st);
 cudaError_t launch_dd_ssum(const double2 *bigsum, int nblk, double2 *partial, cudaStream_t st);

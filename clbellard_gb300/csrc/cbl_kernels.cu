@@ -53,34 +53,34 @@ __device__ __forceinline__ void shr192(uint32_t q[6], int s)
 // 3 = strict width 1 (2^28 <= m < 2^32), 7 and 8 = float-quotient width 2 (2^32 <= m
 // < 15 * 2^34 and < 94 * 2^32), 4 = short width 2 (2^32 <= m < 2^44),
 // 2 = width 2 (2^28 <= m < 2^60), 6 = wide width 2 (2^60 <= m < 2^62).
-template <int KIND, bool TAIL>
-__device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, uint32_t q[6])
+template <int KIND, bool TAIL, int N>
+__device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, uint32_t q[N])
 {
     const uint32_t mp = neg_inv32((uint32_t)m);
-    const uint64_t E = TAIL ? 192ull : 10ull * (d - k) + 192ull;
+    const uint64_t E = TAIL ? 32ull * N : 10ull * (d - k) + 32ull * N;
     if (KIND == 1) {
-        const uint32_t r6 = w1_pow2(E, (uint32_t)m, mp);
-        w1_digits(r6, (uint32_t)m, mp, q);
+        const uint32_t r = w1_pow2(E, (uint32_t)m, mp);
+        w1_digits<N>(r, (uint32_t)m, mp, q);
     } else if (KIND == 5) {
-        const uint32_t r6 = w1m_pow2(E, (uint32_t)m, mp);
-        w1_digits(r6, (uint32_t)m, mp, q);
+        const uint32_t r = w1m_pow2(E, (uint32_t)m, mp);
+        w1_digits<N>(r, (uint32_t)m, mp, q);
     } else if (KIND == 3) {
-        const uint32_t r6 = w1s_pow2(E, (uint32_t)m, mp);
-        w1_digits(r6, (uint32_t)m, mp, q);
+        const uint32_t r = w1s_pow2(E, (uint32_t)m, mp);
+        w1_digits<N>(r, (uint32_t)m, mp, q);
     } else if (KIND == 7 || KIND == 8) {
-        const uint64_t r6 = w2f_pow2<KIND == 8>(E, m, mp);
-        w2_digits(r6, m, mp, q);
+        const uint64_t r = w2f_pow2<KIND == 8>(E, m, mp);
+        w2_redc_down<N>(r, m, mp, q);
     } else if (KIND == 4) {
-        const uint64_t r6 = w2s_pow2(E, m, mp);
-        w2_digits(r6, m, mp, q);
+        const uint64_t r = w2s_pow2(E, m, mp);
+        w2_redc_down<N>(r, m, mp, q);
     } else if (KIND == 6) {
-        const uint64_t r6 = w2x_pow2(E, m, mp);
-        w2_digits(r6, m, mp, q);
+        const uint64_t r = w2x_pow2(E, m, mp);
+        w2_redc_down<N>(r, m, mp, q);
     } else {
-        const uint64_t r6 = w2_pow2(E, m, mp);
-        w2_digits(r6, m, mp, q);
+        const uint64_t r = w2_pow2(E, m, mp);
+        w2_redc_down<N>(r, m, mp, q);
     }
-    if (TAIL) shr192(q, (int)(10 * (k - d)));
+    if constexpr (TAIL) shr192(q, (int)(10 * (k - d)));
 }
 
 // Two terms (exponents Ea and Ea - 320) of a lane per iteration, their ladders interleaved
@@ -90,17 +90,17 @@ __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, 
 // 40.65 -> 38.55 ms, 1e10 841.0 -> 838.9 ms, batch 10.61 -> 10.08 s. Pairing
 // only some kinds traded these against each other (the kernel's code layout
 // and registers change with every instantiation), so all four are paired.
-template <int KIND>
-__device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t ma, uint64_t mb, uint32_t qa[6],
-                                          uint32_t qb[6])
+template <int KIND, int N>
+__device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t ma, uint64_t mb, uint32_t qa[N],
+                                          uint32_t qb[N])
 {
     const uint32_t mpa = neg_inv32((uint32_t)ma), mpb = neg_inv32((uint32_t)mb);
     const uint64_t Eb = Ea - 320ull;
     if (KIND == 7 || KIND == 8) {
         uint64_t ra, rb;
         w2f_pow2_pair<KIND == 8>(Ea, ma, mpa, Eb, mb, mpb, e_max, ra, rb);
-        w2_digits(ra, ma, mpa, qa);
-        w2_digits(rb, mb, mpb, qb);
+        w2_redc_down<N>(ra, ma, mpa, qa);
+        w2_redc_down<N>(rb, mb, mpb, qb);
     } else if (KIND == 4) {
         W2SState A{0, 0, (uint32_t)ma, (uint32_t)(ma >> 32), mpa}, B{0, 0, (uint32_t)mb, (uint32_t)(mb >> 32), mpb};
         walk_bits_start_pair<4>(Ea - 48, Eb - 48, A, B, W2SStart{});   // R = 2^48
@@ -109,8 +109,8 @@ __device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t 
         ra = min(ra, ra - ma);
         rb = min(rb, rb - 2 * mb);
         rb = min(rb, rb - mb);
-        w2_digits(ra, ma, mpa, qa);
-        w2_digits(rb, mb, mpb, qb);
+        w2_redc_down<N>(ra, ma, mpa, qa);
+        w2_redc_down<N>(rb, mb, mpb, qb);
     } else if (KIND == 1) {
         W1State A{0, (uint32_t)ma, mpa}, B{0, (uint32_t)mb, mpb};
         walk_bits_group<1>(Ea - 32, Eb - 32, e_max - 32, A, B, W1Start1{});
@@ -119,36 +119,36 @@ __device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t 
         ya = min(ya, ya - (uint32_t)ma);
         yb = min(yb, yb - 2u * (uint32_t)mb);
         yb = min(yb, yb - (uint32_t)mb);
-        w1_digits(ya, (uint32_t)ma, mpa, qa);
-        w1_digits(yb, (uint32_t)mb, mpb, qb);
+        w1_digits<N>(ya, (uint32_t)ma, mpa, qa);
+        w1_digits<N>(yb, (uint32_t)mb, mpb, qb);
     } else if (KIND == 5) {
         W1MState A{0, (uint32_t)ma, mpa}, B{0, (uint32_t)mb, mpb};
         walk_bits_group<4>(Ea - 32, Eb - 32, e_max - 32, A, B, W1MStart{});
-        w1_digits(A.y, (uint32_t)ma, mpa, qa);
-        w1_digits(B.y, (uint32_t)mb, mpb, qb);
+        w1_digits<N>(A.y, (uint32_t)ma, mpa, qa);
+        w1_digits<N>(B.y, (uint32_t)mb, mpb, qb);
     } else {
         W1SState A{0, (uint32_t)ma, 0u - mpa}, B{0, (uint32_t)mb, 0u - mpb};
         walk_bits_group<4>(Ea - 32, Eb - 32, e_max - 32, A, B, W1SStart{});
-        w1_digits(A.residue(), (uint32_t)ma, mpa, qa);
-        w1_digits(B.residue(), (uint32_t)mb, mpb, qb);
+        w1_digits<N>(A.residue(), (uint32_t)ma, mpa, qa);
+        w1_digits<N>(B.residue(), (uint32_t)mb, mpb, qb);
     }
 }
 
-template <int KIND, bool TAIL>
-__device__ __forceinline__ void run_tile(const Seg &s, uint64_t kb, uint64_t ke, int lane, Acc192 &acc,
+template <int KIND, bool TAIL, int N>
+__device__ __forceinline__ void run_tile(const Seg &s, uint64_t kb, uint64_t ke, int lane, Acc<N> &acc,
                                          uint32_t &cnt)
 {
     uint64_t k = kb + lane;
     if (!TAIL && (KIND == 1 || KIND == 3 || KIND == 4 || KIND == 5 || KIND == 7 || KIND == 8)) {
         constexpr bool wide = KIND == 4 || KIND == 7 || KIND == 8;
-        uint64_t ea = 10ull * (s.d - k) + 192ull, ma = (uint64_t)s.den0 * k + s.den1;
+        uint64_t ea = 10ull * (s.d - k) + 32ull * N, ma = (uint64_t)s.den0 * k + s.den1;
         uint64_t e_max = ea + 10u * lane;
         const uint64_t m32 = 32ull * s.den0;
         for (uint32_t n = (uint32_t)(ke - kb) >> 6; n > 0; --n) {   // terms k and k+32 together
-            uint32_t qa[6], qb[6];
+            uint32_t qa[N], qb[N];
             // e_max kept in registers cost the two-word kinds more than its two adds
             // (1e10: 550.1 against 542.6 ms) and gained on the one-word kinds (1e9: 32.7 to 32.2 ms)
-            term_pair<KIND>(ea, wide ? ea + 10u * lane : e_max, ma, ma + m32, qa, qb);
+            term_pair<KIND, N>(ea, wide ? ea + 10u * lane : e_max, ma, ma + m32, qa, qb);
             e_max -= 640;
             ma += 2 * m32;
             ea -= 640;
@@ -160,8 +160,8 @@ __device__ __forceinline__ void run_tile(const Seg &s, uint64_t kb, uint64_t ke,
     }
     for (; k < ke; k += 32) {
         const uint64_t m = (uint64_t)s.den0 * k + s.den1;
-        uint32_t q[6];
-        term_digits<KIND, TAIL>(s.d, k, m, q);
+        uint32_t q[N];
+        term_digits<KIND, TAIL, N>(s.d, k, m, q);
         acc_add(acc, q);
         ++cnt;
     }
@@ -277,8 +277,8 @@ __device__ __forceinline__ void flush_block(const Seg *segs, int cur, int lane, 
 // that a launch can meet (term_level): the kernel's registers and code follow its
 // widest kind, and the one-word kinds ran 5 % slower beside the two-word ones
 // (1e9: 36.8 ms alone in the kernel, 38.8 ms with the float-quotient steps there).
-template <int LEVEL, bool TAIL>
-__device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_t ke, int lane, Acc192 &acc,
+template <int LEVEL, bool TAIL, int N>
+__device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_t ke, int lane, Acc<N> &acc,
                                               uint32_t &cnt)
 {
     const int width = (int)((s.flags >> 4) & 15u);
@@ -286,7 +286,7 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
         run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
     } else if (LEVEL == 1 && width == 4) {
         const uint64_t m_last = (uint64_t)s.den0 * (ke - 1) + s.den1;
-        const bool fq = TAIL || 10 * (s.d - kb) + 192 < kW2FExp;
+        const bool fq = TAIL || 10 * (s.d - kb) + 32 * N < kW2FExp;
         if (fq && m_last < kW2FLow) run_tile<7, TAIL>(s, kb, ke, lane, acc, cnt);
         else if (fq && m_last < kW2FMax) run_tile<8, TAIL>(s, kb, ke, lane, acc, cnt);
         else run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
@@ -310,7 +310,7 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
 // the float-quotient kind at 64 registers and 4 CTAs (1e10: 561.7 ms; 591 ms when held
 // to 48 registers for 5 CTAs, with spills), the single ladders of the general
 // two-word kinds at 5 CTAs (2^27 terms at 1e13: 5.81 ms against 5.96 ms at 4).
-template <int LEVEL>
+template <int LEVEL, bool FIXED>
 __global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel(const Seg *__restrict__ segs, int nseg,
                                                              uint64_t ntiles, uint32_t tile_k, TileSplit split,
                                                              unsigned long long *counter,
@@ -319,8 +319,9 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel
 {
     const int lane = threadIdx.x & 31;
     const uint64_t t_start = budget_ns ? global_ns() : 0;
-    uint64_t nitems = ntiles << split.log2_parts, item = 0;
-    if (split.fixed) {                              // this block's share, dealt to its warps in turn
+    uint64_t nitems = ntiles, item = 0;
+    if (FIXED) {                                    // this block's share, dealt to its warps in turn
+        nitems <<= split.log2_parts;
         item = nitems * blockIdx.x / gridDim.x + (threadIdx.x >> 5);
         nitems = nitems * (blockIdx.x + 1) / gridDim.x;
     }
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel
     acc_zero(acc);
     uint32_t cnt = 0;
     for (;; item += kBlock192 / 32) {
-        if (!split.fixed) {
+        if (!FIXED) {
             unsigned long long t = 0;
             if (lane == 0) {
                 if (budget_ns && global_ns() - t_start > budget_ns) t = ~0ull;
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel
             item = __shfl_sync(0xffffffffu, t, 0);
         }
         if (item >= nitems) break;
-        const uint64_t t = item >> split.log2_parts;
+        const uint64_t t = FIXED ? item >> split.log2_parts : item;
         int lo = 0, hi = nseg - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -352,22 +353,26 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel
         }
         const Seg s = segs[lo];
         const uint64_t k0 = s.k0 + (t - s.tile0) * tile_k;
-        const uint64_t kb = k0 + ((uint32_t)item & ((1u << split.log2_parts) - 1u)) * split.part_k;
-        const uint64_t ke = min(min(s.k1, k0 + tile_k), kb + split.part_k);
-        if (kb >= ke) continue;
+        uint64_t kb = k0, ke = min(s.k1, k0 + tile_k);
+        if (FIXED) {
+            kb += ((uint32_t)item & ((1u << split.log2_parts) - 1u)) * split.part_k;
+            ke = min(ke, kb + split.part_k);
+            if (kb >= ke) continue;
+        }
         if (kb >= s.d) run_tile_kind<LEVEL, true>(s, kb, ke, lane, acc, cnt);
         else run_tile_kind<LEVEL, false>(s, kb, ke, lane, acc, cnt);
     }
-    if (split.fixed) flush_block(segs, cur, lane, acc, cnt, slots, carry);
+    if (FIXED) flush_block(segs, cur, lane, acc, cnt, slots, carry);
     else if (cur >= 0) flush_segment(segs[cur], lane, acc, cnt, slots, carry);
 }
 
 typedef void (*Terms192Fn)(const Seg *, int, uint64_t, uint32_t, TileSplit, unsigned long long *, unsigned long long *,
                            uint64_t, int);
 
+template <bool FIXED>
 static Terms192Fn terms192_fn(int level)
 {
-    return level == 0 ? terms192_kernel<0> : level == 1 ? terms192_kernel<1> : terms192_kernel<2>;
+    return level == 0 ? terms192_kernel<0, FIXED> : level == 1 ? terms192_kernel<1, FIXED> : terms192_kernel<2, FIXED>;
 }
 
 // A pass with fewer tiles than resident warps leaves most of the GPU idle and its
@@ -398,15 +403,15 @@ cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntile
     // a budgeted pass stops and resumes at whole tiles
     const TileSplit sp = budget_ns ? TileSplit{0, 0, tile_k} : tile_split(ntiles, tile_k, grid);
     if (sp.fixed) grid = (int)std::min<uint64_t>(grid, ntiles << sp.log2_parts);
-    terms192_fn(level)<<<grid, kBlock192, 0, st>>>(segs, nseg, ntiles, tile_k, sp, counter, slots, budget_ns,
-                                                   carry ? 1 : 0);
+    const Terms192Fn fn = sp.fixed ? terms192_fn<true>(level) : terms192_fn<false>(level);
+    fn<<<grid, kBlock192, 0, st>>>(segs, nseg, ntiles, tile_k, sp, counter, slots, budget_ns, carry ? 1 : 0);
     return cudaGetLastError();
 }
 
 int terms192_max_ctas_per_sm(int level)
 {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, terms192_fn(level), kBlock192, 0) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, terms192_fn<false>(level), kBlock192, 0) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }
 
@@ -540,21 +545,21 @@ __global__ void terms_each_kernel(uint64_t d, uint32_t den0, uint32_t den1, int 
     uint32_t q[6] = {0, 0, 0, 0, 0, 0};
     if (m != 1) {
         if (k < d) {
-            if (m < kW1MMin) term_digits<1, false>(d, k, m, q);
-            else if (m < kW1MMax) term_digits<5, false>(d, k, m, q);
-            else if (m < kW1SMax) term_digits<3, false>(d, k, m, q);
-            else if (m < kW2FLow) term_digits<7, false>(d, k, m, q);
-            else if (m < kW2FMax) term_digits<8, false>(d, k, m, q);
-            else if (m < kW2SMax) term_digits<4, false>(d, k, m, q);
-            else if (m < kW2Max) term_digits<2, false>(d, k, m, q);
-            else term_digits<6, false>(d, k, m, q);
+            if (m < kW1MMin) term_digits<1, false, 6>(d, k, m, q);
+            else if (m < kW1MMax) term_digits<5, false, 6>(d, k, m, q);
+            else if (m < kW1SMax) term_digits<3, false, 6>(d, k, m, q);
+            else if (m < kW2FLow) term_digits<7, false, 6>(d, k, m, q);
+            else if (m < kW2FMax) term_digits<8, false, 6>(d, k, m, q);
+            else if (m < kW2SMax) term_digits<4, false, 6>(d, k, m, q);
+            else if (m < kW2Max) term_digits<2, false, 6>(d, k, m, q);
+            else term_digits<6, false, 6>(d, k, m, q);
         } else {
-            if (m < kW1MMin) term_digits<1, true>(d, k, m, q);
-            else if (m < kW1MMax) term_digits<5, true>(d, k, m, q);
-            else if (m < kW1SMax) term_digits<3, true>(d, k, m, q);
-            else if (m < kW2SMax) term_digits<4, true>(d, k, m, q);
-            else if (m < kW2Max) term_digits<2, true>(d, k, m, q);
-            else term_digits<6, true>(d, k, m, q);
+            if (m < kW1MMin) term_digits<1, true, 6>(d, k, m, q);
+            else if (m < kW1MMax) term_digits<5, true, 6>(d, k, m, q);
+            else if (m < kW1SMax) term_digits<3, true, 6>(d, k, m, q);
+            else if (m < kW2SMax) term_digits<4, true, 6>(d, k, m, q);
+            else if (m < kW2Max) term_digits<2, true, 6>(d, k, m, q);
+            else term_digits<6, true, 6>(d, k, m, q);
         }
         if ((k + (uint64_t)sign) & 1ull)
             for (int j = 0; j < 6; ++j) q[j] = ~q[j];
@@ -653,78 +658,139 @@ __device__ __forceinline__ DD block_reduce_dd(DD v)
     return DD{sh_hi[0], sh_lo[0]};
 }
 
-__global__ void __launch_bounds__(kBlockDD) dd_terms_kernel(double2 *bigsum, uint64_t k0, uint64_t k1, uint64_t d,
-                                                            int sign, uint32_t den0, uint32_t den1)
+// 128-bit fraction, mod 1 and taken in [-1/2, 1/2), as a double-double.
+__device__ __forceinline__ DD dd_from_fraction(const uint32_t w[4])
 {
-    const uint64_t gsize = (uint64_t)gridDim.x * blockDim.x;
-    DD sum{0.0, 0.0};
-    for (uint64_t k = k0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < k1; k += gsize) {
-        const uint64_t m = (uint64_t)den0 * k + den1;
-        if (m == 1) continue;
-        const uint32_t mp = neg_inv32((uint32_t)m);
-        // r = 2^(10(d-k)) mod m: the ladder to 2^(10(d-k) + 32 j) and j REDC
-        // steps down (j = 1 one word, 2 two words); no quotient digits.
-        const uint64_t e = 10ull * (d - k);
-        uint64_t r;
-        if (m < kW1SMax) {
-            uint32_t y;
-            if (m < kW1MMin) y = w1_pow2(e + 32, (uint32_t)m, mp);
-            else if (m < kW1MMax) y = w1m_pow2(e + 32, (uint32_t)m, mp);
-            else y = w1s_pow2(e + 32, (uint32_t)m, mp);
-            r = redc_word(y * mp, (uint32_t)m, y, 0u);
-        } else {
-            uint64_t y;
-            if (m < kW2FLow) y = w2f_pow2<false>(e + 64, m, mp);
-            else if (m < kW2FMax) y = w2f_pow2<true>(e + 64, m, mp);
-            else if (m < kW2SMax) y = w2s_pow2(e + 64, m, mp);
-            else if (m < kW2Max) y = w2_pow2(e + 64, m, mp);
-            else y = w2x_pow2(e + 64, m, mp);
-            uint32_t q[2];
-            r = w2_redc_down<2>(y, m, mp, q);
+    const DD top = two_sum((double)(int32_t)w[3] * 0x1p-32, (double)w[2] * 0x1p-64);
+    const DD low = two_sum((double)w[1] * 0x1p-96, (double)w[0] * 0x1p-128);
+    return dd_add(top, low);
+}
+
+// Residue kind of a modulus (Seg::flags), and the first k of the next kind.
+__device__ __forceinline__ uint32_t modulus_kind(uint64_t m, uint64_t &limit)
+{
+    if (m < kW1Max) { limit = kW1Max; return 1; }
+    if (m < kW1MMax) { limit = kW1MMax; return 5; }
+    if (m < kW1SMax) { limit = kW1SMax; return 3; }
+    if (m < kW2SMax) { limit = kW2SMax; return 4; }
+    if (m < kW2Max) { limit = kW2Max; return 2; }
+    limit = kW2XMax;
+    return 6;
+}
+
+// Terms k in [k0, k1) of one series, k1 <= d. A term r/m enters the sum as its first
+// 128 bits: the ladder runs to 2^(10(d-k) + 128) and four REDC steps give them as
+// quotient digits, as in the 192-bit mode. Lanes add 128-bit integers mod 1, a block
+// turns its sum into one double-double and adds that into its bigSum entry, so
+// FP64 (1.6 operations a clock and SM here) runs once a block and not 25
+// operations and two divisions a term: 2^25 terms at 1e10 in 3.25 ms before. The truncations
+// (below 2^-128 a term, of either sign) stay under the rounding of one double-double add.
+// Warps take tiles of tile_k terms (a multiple of 64) in turn.
+template <int LEVEL>
+__global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 3 : 5) dd_terms_kernel(double2 *bigsum, uint64_t k0, uint64_t k1,
+                                                                             uint64_t d, int sign, uint32_t den0,
+                                                                             uint32_t den1, uint64_t tile_k)
+{
+    __shared__ uint32_t half[8];
+    const int lane = threadIdx.x & 31;
+    const uint64_t step = (uint64_t)gridDim.x * (kBlockDD / 32) * tile_k;
+    if (threadIdx.x < 8) half[threadIdx.x] = 0;
+    __syncthreads();
+    Acc<4> acc;
+    acc_zero(acc);
+    uint64_t odd = k0 & 1;                              // acc holds terms of lanes whose k has parity odd + lane
+    for (uint64_t kb = k0 + ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * tile_k; kb < k1; kb += step) {
+        const uint64_t ke = min(k1, kb + tile_k);
+        uint32_t cnt = 0;
+        for (uint64_t a = kb, b; a < ke; a = b) {       // one run per residue kind
+            uint64_t limit;
+            Seg s{d, a, ke, 0, den0, den1, 0, modulus_kind((uint64_t)den0 * a + den1, limit) << 4};
+            b = min(ke, (limit - den1 + den0 - 1) / den0);
+            if ((a & 1) != odd) {
+                acc_negate(acc);
+                odd ^= 1;
+            }
+            run_tile_kind<LEVEL, false>(s, a, b, lane, acc, cnt);
         }
-        // r and m are exact doubles below 2^53; above, exact double-doubles
-        DD t = (m < kDDMax) ? dd_div_nn((double)r, (double)m) : dd_div_dd(dd_from_u64(r), dd_from_u64(m));
-        if ((k + (uint64_t)sign) & 1ull) { t.hi = -t.hi; t.lo = -t.lo; }
-        sum = dd_frac(dd_add(sum, t));
     }
-    const DD b = block_reduce_dd(sum);
+    if ((odd + lane + sign) & 1) acc_negate(acc);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t lo = __reduce_add_sync(0xffffffffu, acc.w[j] & 0xffffu);
+        const uint32_t hi = __reduce_add_sync(0xffffffffu, acc.w[j] >> 16);
+        if (lane == 0) {
+            atomicAdd(&half[2 * j], lo);
+            atomicAdd(&half[2 * j + 1], hi);
+        }
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
+        uint32_t w[4];
+        uint64_t c = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            c += (uint64_t)half[2 * j] + ((uint64_t)half[2 * j + 1] << 16);
+            w[j] = (uint32_t)c;
+            c >>= 32;
+        }
         const double2 o = bigsum[blockIdx.x];
-        const DD s = dd_frac(dd_add(DD{o.x, o.y}, b));
-        bigsum[blockIdx.x] = make_double2(s.hi, s.lo);
+        const DD v = dd_frac(dd_add(DD{o.x, o.y}, dd_from_fraction(w)));
+        bigsum[blockIdx.x] = make_double2(v.hi, v.lo);
     }
 }
 
-cudaError_t launch_dd_terms(double2 *bigsum, int nblk, int block, uint64_t k0, uint64_t k1, uint64_t d, int sign,
-                            uint32_t den0, uint32_t den1, cudaStream_t st)
+typedef void (*DDTermsFn)(double2 *, uint64_t, uint64_t, uint64_t, int, uint32_t, uint32_t, uint64_t);
+
+static DDTermsFn dd_terms_fn(int level)
 {
-    (void)block;
-    dd_terms_kernel<<<nblk, kBlockDD, 0, st>>>(bigsum, k0, k1, d, sign, den0, den1);
+    return level == 0 ? dd_terms_kernel<0> : level == 1 ? dd_terms_kernel<1> : dd_terms_kernel<2>;
+}
+
+int dd_terms_max_ctas_per_sm(int level)
+{
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dd_terms_fn(level), kBlockDD, 0) != cudaSuccess) return 1;
+    return n > 0 ? n : 1;
+}
+
+cudaError_t launch_dd_terms(int level, double2 *bigsum, int grid, int *blocks, uint64_t k0, uint64_t k1, uint64_t d,
+                            int sign, uint32_t den0, uint32_t den1, cudaStream_t st)
+{
+    // eight tiles a resident warp: their costs fall along k, and each warp takes every eighth part
+    const uint64_t warps = (uint64_t)grid * (kBlockDD / 32), n = k1 - k0;
+    const uint64_t tile_k = std::max<uint64_t>(1, (n + 8 * 64 * warps - 1) / (8 * 64 * warps)) * 64;
+    *blocks = (int)std::min<uint64_t>(grid, (n + tile_k - 1) / tile_k);
+    dd_terms_fn(level)<<<*blocks, kBlockDD, 0, st>>>(bigsum, k0, k1, d, sign, den0, den1, tile_k);
     return cudaGetLastError();
 }
 
+// One warp: lane i < 10 divides the tail term k = d + i, lane 0 adds them in order.
 __global__ void dd_tail_kernel(double2 *bigsum, uint64_t d, int sign, uint32_t den0, uint32_t den1)
 {
-    DD sum{0.0, 0.0};
-    double p = 1.0;
-    for (int i = 0; i < kTailDD; ++i) {
-        const uint64_t k = d + (uint64_t)i;
+    const int lane = threadIdx.x;
+    DD t{0.0, 0.0};
+    if (lane < kTailDD) {
+        const uint64_t k = d + (uint64_t)lane;
         const uint64_t m = (uint64_t)den0 * k + den1;
+        const double p = __longlong_as_double((1023ll - 10 * lane) << 52);      // 2^(-10 lane)
         if (m != 1) {
-            DD t = (m < kDDMax) ? dd_div_nn(p, (double)m) : dd_div_dd(DD{p, 0.0}, dd_from_u64(m));
+            t = (m < kDDMax) ? dd_div_nn(p, (double)m) : dd_div_dd(DD{p, 0.0}, dd_from_u64(m));
             if ((k + (uint64_t)sign) & 1ull) { t.hi = -t.hi; t.lo = -t.lo; }
-            sum = dd_add(sum, t);
         }
-        p *= 0.0009765625;   // 2^-10
     }
-    const double2 o = bigsum[0];
-    const DD s = dd_frac(dd_add(DD{o.x, o.y}, sum));
-    bigsum[0] = make_double2(s.hi, s.lo);
+    DD sum{0.0, 0.0};
+    for (int i = 0; i < kTailDD; ++i)
+        sum = dd_add(sum, DD{__shfl_sync(0xffffffffu, t.hi, i), __shfl_sync(0xffffffffu, t.lo, i)});
+    if (lane == 0) {
+        const double2 o = bigsum[0];
+        const DD s = dd_frac(dd_add(DD{o.x, o.y}, sum));
+        bigsum[0] = make_double2(s.hi, s.lo);
+    }
 }
 
 cudaError_t launch_dd_tail(double2 *bigsum, uint64_t d, int sign, uint32_t den0, uint32_t den1, cudaStream_t st)
 {
-    dd_tail_kernel<<<1, 1, 0, st>>>(bigsum, d, sign, den0, den1);
+    dd_tail_kernel<<<1, 32, 0, st>>>(bigsum, d, sign, den0, den1);
     return cudaGetLastError();
 }
 

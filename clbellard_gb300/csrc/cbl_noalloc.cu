@@ -252,7 +252,7 @@ extern "C" int cbl_batch_noalloc(const uint64_t *pos, int n, uint64_t *d_out3n, 
     if (cudaMemsetAsync(base, 0, kOffSegs, st) != cudaSuccess) return CBL_E_CUDA;
     noalloc_table_kernel<<<1, kMaxPos, 0, st>>>(args, dsegs);
     if (cudaGetLastError() != cudaSuccess) return CBL_E_CUDA;
-    const int level = term_level(max_m);
+    const int level = term_level(0, max_m);
     if (launch_terms192(level, dsegs, nseg, ntiles, (uint32_t)kTileTerms, counter, slots, ds->grid[level], st, 0,
                         slot_needs_carry(max_series_tiles)) != cudaSuccess)
         return CBL_E_CUDA;
