@@ -24,7 +24,7 @@ using namespace cbl;
 namespace {
 
 constexpr uint64_t kMaxNeedD = 999999999999999999ull;   // Bellard_192.hsp:450
-constexpr int kDDBlocks = 4096;                         // dd per-block partials (bigSum)
+constexpr int kDDBlocks = 4096;                         // mode 0's per-block partials (bigSum)
 constexpr int kDefaultTile = 32 * 64;                   // terms per warp tile
 
 typedef unsigned __int128 u128;
@@ -72,8 +72,8 @@ struct cbl_ctx {
     std::vector<Seg> prep_segs;                      // host copy of the prepared segments
     std::vector<int> prep_shift;
     // double-double buffers
-    double2 *d_bigsum = nullptr;
-    int dd_blocks = 1;                               // leading bigSum entries in use since cbl_Set0mem (the tail's at least)
+    uint4 *d_bigsum = nullptr;                       // 128-bit fractions, one per block of the term kernel
+    int dd_blocks = 1;                               // leading bigSum entries in use since cbl_Set0mem
     double2 *d_ddpartial = nullptr;
     double2 *d_ddans = nullptr;
     // scratch host
@@ -263,20 +263,23 @@ int run_segments(cbl_ctx *c, std::vector<Seg> &v)
     return CBL_OK;
 }
 
-int dd_range(cbl_ctx *c, uint64_t k0, uint64_t k1, uint64_t d, int sign, uint32_t den0, uint32_t den1)
+// Terms k in [k0, k1) of one series (k1 <= d) into bigSum, and with tail k = d .. d+9.
+int dd_range(cbl_ctx *c, uint64_t k0, uint64_t k1, uint64_t d, int sign, uint32_t den0, uint32_t den1, bool tail)
 {
     if (k1 > k0 && (u128)den0 * (k1 - 1) + den1 >= (u128)kW2XMax) return CBL_E_POSITION;
     if (k0 == 0 && den1 == 1) k0 = 1;                    // m = 1 contributes exactly 0
-    // chunks of 2^30 terms keep each launch to a bounded time
+    // chunks of 2^30 terms keep each launch to a bounded time; the last takes the tail
     const uint64_t chunk = 1ull << 30;
-    for (uint64_t a = k0; a < k1; a += chunk) {
-        const uint64_t b = std::min(k1, a + chunk);
-        const int level = term_level((uint64_t)den0 * a + den1, (uint64_t)den0 * (b - 1) + den1);
+    for (uint64_t a = k0; a < k1 || tail; a += chunk) {
+        const uint64_t b = std::max(a, std::min(k1, a + chunk));
+        const bool last = b >= k1;
+        const int level = b > a ? term_level((uint64_t)den0 * a + den1, (uint64_t)den0 * (b - 1) + den1) : 0;
         const int grid = std::min(kDDBlocks, c->sm_count * dd_terms_max_ctas_per_sm(level));
         int blocks = 0;
-        CK(launch_dd_terms(level, c->d_bigsum, grid, &blocks, a, b, d, sign, den0, den1, c->st));
+        CK(launch_dd_terms(level, c->d_bigsum, grid, &blocks, a, b, d, sign, den0, den1, tail && last, c->st));
         c->dd_blocks = std::max(c->dd_blocks, blocks);
         c->launches++;
+        if (last) break;
     }
     return CBL_OK;
 }
@@ -444,7 +447,7 @@ int cbl_create(int device, int precision, cbl_ctx **out)
     if (!rc && cudaMalloc(&c->d_counter, sizeof(unsigned long long)) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_partial, sizeof(uint64_t) * 3) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ans, sizeof(uint64_t) * 3) != cudaSuccess) rc = CBL_E_NOMEM;
-    if (!rc && cudaMalloc(&c->d_bigsum, sizeof(double2) * kDDBlocks) != cudaSuccess) rc = CBL_E_NOMEM;
+    if (!rc && cudaMalloc(&c->d_bigsum, sizeof(uint4) * kDDBlocks) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ddpartial, sizeof(double2)) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ddans, sizeof(double2)) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMallocHost(&c->h_small, sizeof(uint64_t) * 8) != cudaSuccess) rc = CBL_E_NOMEM;
@@ -457,7 +460,7 @@ int cbl_create(int device, int precision, cbl_ctx **out)
         cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6 * c->slot_cap, c->st);
         cudaMemsetAsync(c->d_partial, 0, sizeof(uint64_t) * 3, c->st);
         cudaMemsetAsync(c->d_ans, 0, sizeof(uint64_t) * 3, c->st);
-        cudaMemsetAsync(c->d_bigsum, 0, sizeof(double2) * kDDBlocks, c->st);
+        cudaMemsetAsync(c->d_bigsum, 0, sizeof(uint4) * kDDBlocks, c->st);
         cudaMemsetAsync(c->d_ddpartial, 0, sizeof(double2), c->st);
         cudaMemsetAsync(c->d_ddans, 0, sizeof(double2), c->st);
         if (cudaStreamSynchronize(c->st) != cudaSuccess) rc = CBL_E_CUDA;
@@ -571,7 +574,7 @@ int cbl_Set0mem(cbl_ctx *c)
         CK(cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6, c->st));
         c->slot0_tiles = 0;
     } else {
-        CK(cudaMemsetAsync(c->d_bigsum, 0, sizeof(double2) * kDDBlocks, c->st));
+        CK(cudaMemsetAsync(c->d_bigsum, 0, sizeof(uint4) * kDDBlocks, c->st));
         c->dd_blocks = 1;
     }
     return CBL_OK;
@@ -603,7 +606,7 @@ static int sglobal(cbl_ctx *c, uint64_t offset, uint64_t d, uint64_t k_max, int6
         if (rc) return rc == CBL_E_POSITION ? CBL_E_RANGE : rc;
         return run_segments(c, v);
     }
-    return dd_range(c, offset, k_max, d, (int)numesign, (uint32_t)den0, (uint32_t)den1);
+    return dd_range(c, offset, k_max, d, (int)numesign, (uint32_t)den0, (uint32_t)den1, false);
 }
 
 int cbl_Sglobal32mtg(cbl_ctx *c, uint64_t offset, uint64_t d, uint64_t k_max, int64_t numesign, uint64_t den0,
@@ -633,9 +636,7 @@ int cbl_Sglobal_after(cbl_ctx *c, uint64_t d, int64_t numesign, uint64_t den0, u
         if (rc) return rc;
         return run_segments(c, v);
     }
-    CK(launch_dd_tail(c->d_bigsum, d, (int)numesign, (uint32_t)den0, (uint32_t)den1, c->st));
-    c->launches++;
-    return CBL_OK;
+    return dd_range(c, d, d, d, (int)numesign, (uint32_t)den0, (uint32_t)den1, true);
     CBL_GUARD_END
 }
 
@@ -684,15 +685,9 @@ int cbl_BatchCalc(cbl_ctx *c, uint64_t k_start, uint64_t k_end, int f, uint64_t 
         rc = run_segments(c, v);
         if (rc) return rc;
     } else {
-        if (k_start < kend) {
-            int rc = dd_range(c, k_start, kend, d, kSign[f], kDen0[f], kDen1[f]);
-            if (rc) return rc;
-        }
-        if (tail) {
-            if ((u128)kDen0[f] * (d + kTailDD) + kDen1[f] >= (u128)kW2XMax) return CBL_E_POSITION;
-            CK(launch_dd_tail(c->d_bigsum, d, kSign[f], kDen0[f], kDen1[f], c->st));
-            c->launches++;
-        }
+        if (tail && (u128)kDen0[f] * (d + kTailDD) + kDen1[f] >= (u128)kW2XMax) return CBL_E_POSITION;
+        const int rc = dd_range(c, std::min(k_start, kend), kend, d, kSign[f], kDen0[f], kDen1[f], tail);
+        if (rc) return rc;
     }
     return cbl_Ssum(c);
     CBL_GUARD_END

@@ -34,7 +34,6 @@ constexpr uint64_t kW2FExp = 1ull << 48;  // ... in tiles whose exponents are be
 constexpr uint64_t kW2SMax = 1ull << 44;  // short width 2 for 2^32 <= m < 2^44
 constexpr uint64_t kW2Max = 1ull << 60;   // width 2 (two words, residues < 4m) for m < 2^60
 constexpr uint64_t kW2XMax = 1ull << 62;  // wide width 2 (residues < 2m) for 2^60 <= m < 2^62
-constexpr uint64_t kDDMax = 1ull << 53;   // double-double mode: m and r exact as doubles below, double-doubles above
 
 constexpr int kTail192 = 20;   // tail terms k = d..d+19 (Bellard.cl:1164-1239)
 constexpr int kTailDD = 10;    // tail terms k = d..d+9  (Bellard.cl:1125)
@@ -103,14 +102,13 @@ cudaError_t launch_sum7_192(uint64_t *partial, uint64_t *ans, int numer_log2, cu
 cudaError_t launch_terms_each(uint64_t d, uint32_t den0, uint32_t den1, int sign, const uint64_t *k,
                               int n, uint64_t *out3n, cudaStream_t st);
 
-// Double-double (mode 0) kernels. launch_dd_terms runs at most `grid` blocks (one
-// wave), block i adding into bigsum[i]; *blocks = the number launched.
-cudaError_t launch_dd_terms(int level, double2 *bigsum, int grid, int *blocks, uint64_t k0, uint64_t k1, uint64_t d,
-                            int sign, uint32_t den0, uint32_t den1, cudaStream_t st);
+// Double-double (mode 0) kernels. bigSum is kDDBlocks 128-bit fractions mod 1
+// (little-endian words). launch_dd_terms runs at most `grid` blocks (one wave), block i
+// adding into bigsum[i]; *blocks = the number launched; tail adds the terms k = d .. d+9.
+cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *blocks, uint64_t k0, uint64_t k1, uint64_t d,
+                            int sign, uint32_t den0, uint32_t den1, bool tail, cudaStream_t st);
 int dd_terms_max_ctas_per_sm(int level);
-cudaError_t launch_dd_tail(double2 *bigsum, uint64_t d, int sign, uint32_t den0, uint32_t den1,
-                           cudaStream_t st);
-cudaError_t launch_dd_ssum(const double2 *bigsum, int nblk, double2 *partial, cudaStream_t st);
+cudaError_t launch_dd_ssum(const uint4 *bigsum, int nblk, double2 *partial, cudaStream_t st);
 cudaError_t launch_dd_sum7(double2 *partial, double2 *ans, int numer, cudaStream_t st);
 
 // Throughput probe: grid x block threads each run `iters` rounds of 16

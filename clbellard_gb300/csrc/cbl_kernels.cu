@@ -24,30 +24,31 @@ __device__ __forceinline__ int numer_log2(int f)
 }
 
 // ---------------------------------------------------------------- helpers --
-// q >>= s for s in [0, 192), on six 32-bit digits (digit 0 least significant),
-// with static register indexing only.
-__device__ __forceinline__ void shr192(uint32_t q[6], int s)
+// q >>= s on N 32-bit digits (digit 0 least significant), with static register
+// indexing only.
+template <int N>
+__device__ __forceinline__ void shr_digits(uint32_t q[N], int s)
 {
-    if (s >= 192) {
+    if (s >= 32 * N) {
 #pragma unroll
-        for (int j = 0; j < 6; ++j) q[j] = 0;
+        for (int j = 0; j < N; ++j) q[j] = 0;
         return;
     }
     const int ws = s >> 5, bs = s & 31;
 #pragma unroll
-    for (int t = 0; t < 5; ++t) {
+    for (int t = 0; t < N - 1; ++t) {
         if (t < ws) {
 #pragma unroll
-            for (int j = 0; j < 5; ++j) q[j] = q[j + 1];
-            q[5] = 0;
+            for (int j = 0; j < N - 1; ++j) q[j] = q[j + 1];
+            q[N - 1] = 0;
         }
     }
 #pragma unroll
-    for (int j = 0; j < 5; ++j) q[j] = __funnelshift_r(q[j], q[j + 1], bs);
-    q[5] >>= bs;
+    for (int j = 0; j < N - 1; ++j) q[j] = __funnelshift_r(q[j], q[j + 1], bs);
+    q[N - 1] >>= bs;
 }
 
-// One term's six quotient digits: k < d gives frac(2^(10(d-k))/m), k >= d the
+// One term's N quotient digits: k < d gives frac(2^(10(d-k))/m), k >= d the
 // tail value 2^(-10(k-d))/m (digits of 1/m shifted right by 10(k-d)).
 // KIND: 1 = width 1 (m < 2^28), 5 = middle width 1 (2^25 <= m < 2^31),
 // 3 = strict width 1 (2^28 <= m < 2^32), 7 and 8 = float-quotient width 2 (2^32 <= m
@@ -80,7 +81,7 @@ __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, 
         const uint64_t r = w2_pow2(E, m, mp);
         w2_redc_down<N>(r, m, mp, q);
     }
-    if constexpr (TAIL) shr192(q, (int)(10 * (k - d)));
+    if (TAIL) shr_digits<N>(q, (int)(10 * (k - d)));
 }
 
 // Two terms (exponents Ea and Ea - 320) of a lane per iteration, their ladders interleaved
@@ -482,6 +483,7 @@ __global__ void combine_kernel(const unsigned long long *slots, int npos, const 
     if (i >= npos) return;
     uint64_t ans[3] = {0, 0, 0};
     const int sh = shift ? shift[i] : 0;
+#pragma unroll                                          // all 42 loads in flight at once
     for (int f = 0; f < 7; ++f) {
         uint64_t w[3];
         normalise6(slots + ((size_t)i * 7 + f) * 6, w);
@@ -603,60 +605,7 @@ __device__ __forceinline__ DD dd_frac(DD a)
     return (t != 0.0) ? two_sum(a.hi - t, a.lo) : a;
 }
 
-// x / y to ~106 bits (nn_div, Bellard.cl:99-106), with an exact fma residual.
-__device__ __forceinline__ DD dd_div_nn(double x, double y)
-{
-    const double q1 = x / y;
-    const double rem = fma(-q1, y, x);
-    const double q2 = rem / y;
-    return two_sum(q1, q2);
-}
-
-// An integer 0 <= x < 2^63 as an exact double-double: hi = x rounded to 53
-// bits, lo = the (small, signed) rest.
-__device__ __forceinline__ DD dd_from_u64(uint64_t x)
-{
-    const double hi = __ull2double_rn(x);
-    const int64_t rest = (int64_t)(x - __double2ull_rn(hi));
-    return DD{hi, (double)rest};
-}
-
-// a / b for exact double-doubles a >= 0, b > 0 of integers (the OVERDOUBLE case
-// m >= 2^53 of Bellard.cl:937-945, 1040-1047): q1 = a.hi / b.hi, the remainder
-// a - q1 b formed with an exact product (fma) and a single rounding of the
-// q1 b.lo term, then one correction quotient. For b ~ 2^e the remainder is
-// ~2^(e-53) and carries errors ~2^(e-106), so the quotient keeps ~104 bits.
-__device__ __forceinline__ DD dd_div_dd(DD a, DD b)
-{
-    const double q1 = a.hi / b.hi;
-    const double p_hi = q1 * b.hi;
-    const double p_lo = fma(q1, b.hi, -p_hi);            // q1 b.hi = p_hi + p_lo exactly
-    double e = a.hi - p_hi;                               // exact: p_hi is within a factor 2 of a.hi
-    e += a.lo - p_lo;
-    e = fma(-q1, b.lo, e);
-    const double q2 = e / b.hi;
-    return two_sum(q1, q2);
-}
-
 constexpr int kBlockDD = 256;
-
-__device__ __forceinline__ DD block_reduce_dd(DD v)
-{
-    __shared__ double sh_hi[kBlockDD], sh_lo[kBlockDD];
-    const int t = threadIdx.x;
-    sh_hi[t] = v.hi;
-    sh_lo[t] = v.lo;
-    for (int i = kBlockDD / 2; i > 0; i >>= 1) {
-        __syncthreads();
-        if (t < i) {
-            const DD a = dd_frac(dd_add(DD{sh_hi[t], sh_lo[t]}, DD{sh_hi[t + i], sh_lo[t + i]}));
-            sh_hi[t] = a.hi;
-            sh_lo[t] = a.lo;
-        }
-    }
-    __syncthreads();
-    return DD{sh_hi[0], sh_lo[0]};
-}
 
 // 128-bit fraction, mod 1 and taken in [-1/2, 1/2), as a double-double.
 __device__ __forceinline__ DD dd_from_fraction(const uint32_t w[4])
@@ -678,18 +627,42 @@ __device__ __forceinline__ uint32_t modulus_kind(uint64_t m, uint64_t &limit)
     return 6;
 }
 
-// Terms k in [k0, k1) of one series, k1 <= d. A term r/m enters the sum as its first
-// 128 bits: the ladder runs to 2^(10(d-k) + 128) and four REDC steps give them as
-// quotient digits, as in the 192-bit mode. Lanes add 128-bit integers mod 1, a block
-// turns its sum into one double-double and adds that into its bigSum entry, so
-// FP64 (1.6 operations a clock and SM here) runs once a block and not 25
-// operations and two divisions a term: 2^25 terms at 1e10 in 3.25 ms before. The truncations
-// (below 2^-128 a term, of either sign) stay under the rounding of one double-double add.
+// Sum over a block of its lanes' 128-bit accumulators, mod 1, in w of thread 0.
+// half: 8 words of shared memory, zero before the call.
+__device__ __forceinline__ void block_sum128(const Acc<4> &acc, uint32_t *half, uint32_t w[4])
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t lo = __reduce_add_sync(0xffffffffu, acc.w[j] & 0xffffu);
+        const uint32_t hi = __reduce_add_sync(0xffffffffu, acc.w[j] >> 16);
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&half[2 * j], lo);
+            atomicAdd(&half[2 * j + 1], hi);
+        }
+    }
+    __syncthreads();
+    uint64_t c = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        c += (uint64_t)half[2 * j] + ((uint64_t)half[2 * j + 1] << 16);
+        w[j] = (uint32_t)c;
+        c >>= 32;
+    }
+}
+
+// Terms k in [k0, k1) of one series, k1 <= d, and with tail the terms k = d .. d+9. A
+// term's fraction enters the sum as its first 128 bits: the ladder runs to
+// 2^(10(d-k) + 128) and four REDC steps give them as quotient digits, as in the
+// 192-bit mode. Lanes, blocks and bigSum add 128-bit integers mod 1, and Ssum makes one
+// double-double of the sum: FP64 (1.6 operations a clock and SM here) is left to
+// Ssum and Sum7, where the terms took two divisions and 25 operations each (2^25
+// terms at 1e10: 3.25 ms; 0.74 ms so). The truncations (below 2^-128 a term, of either
+// sign) stay under the rounding of one double-double addition.
 // Warps take tiles of tile_k terms (a multiple of 64) in turn.
 template <int LEVEL>
-__global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 3 : 5) dd_terms_kernel(double2 *bigsum, uint64_t k0, uint64_t k1,
+__global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 3 : 5) dd_terms_kernel(uint4 *bigsum, uint64_t k0, uint64_t k1,
                                                                              uint64_t d, int sign, uint32_t den0,
-                                                                             uint32_t den1, uint64_t tile_k)
+                                                                             uint32_t den1, uint64_t tile_k, int tail)
 {
     __shared__ uint32_t half[8];
     const int lane = threadIdx.x & 31;
@@ -699,12 +672,12 @@ __global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 3 : 5) dd_terms_kernel(
     Acc<4> acc;
     acc_zero(acc);
     uint64_t odd = k0 & 1;                              // acc holds terms of lanes whose k has parity odd + lane
+    uint32_t cnt = 0;
     for (uint64_t kb = k0 + ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * tile_k; kb < k1; kb += step) {
         const uint64_t ke = min(k1, kb + tile_k);
-        uint32_t cnt = 0;
         for (uint64_t a = kb, b; a < ke; a = b) {       // one run per residue kind
             uint64_t limit;
-            Seg s{d, a, ke, 0, den0, den1, 0, modulus_kind((uint64_t)den0 * a + den1, limit) << 4};
+            const Seg s{d, a, ke, 0, den0, den1, 0, modulus_kind((uint64_t)den0 * a + den1, limit) << 4};
             b = min(ke, (limit - den1 + den0 - 1) / den0);
             if ((a & 1) != odd) {
                 acc_negate(acc);
@@ -714,32 +687,27 @@ __global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 3 : 5) dd_terms_kernel(
         }
     }
     if ((odd + lane + sign) & 1) acc_negate(acc);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const uint32_t lo = __reduce_add_sync(0xffffffffu, acc.w[j] & 0xffffu);
-        const uint32_t hi = __reduce_add_sync(0xffffffffu, acc.w[j] >> 16);
-        if (lane == 0) {
-            atomicAdd(&half[2 * j], lo);
-            atomicAdd(&half[2 * j + 1], hi);
+    if (tail && blockIdx.x == 0 && threadIdx.x < kTailDD) {
+        const uint64_t k = d + lane, m = (uint64_t)den0 * k + den1;
+        if (m != 1) {
+            const unsigned __int128 x = ~(unsigned __int128)0 / m >> 10 * lane;     // 2^128 / m: m is odd
+            const uint32_t q[4] = {(uint32_t)x, (uint32_t)(x >> 32), (uint32_t)(x >> 64), (uint32_t)(x >> 96)};
+            if ((k + (uint64_t)sign) & 1) acc_negate(acc);
+            acc_add(acc, q);
+            if ((k + (uint64_t)sign) & 1) acc_negate(acc);
         }
     }
-    __syncthreads();
+    uint32_t w[4];
+    block_sum128(acc, half, w);
     if (threadIdx.x == 0) {
-        uint32_t w[4];
-        uint64_t c = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            c += (uint64_t)half[2 * j] + ((uint64_t)half[2 * j + 1] << 16);
-            w[j] = (uint32_t)c;
-            c >>= 32;
-        }
-        const double2 o = bigsum[blockIdx.x];
-        const DD v = dd_frac(dd_add(DD{o.x, o.y}, dd_from_fraction(w)));
-        bigsum[blockIdx.x] = make_double2(v.hi, v.lo);
+        uint4 o = bigsum[blockIdx.x];
+        Acc<4> v{{o.x, o.y, o.z, o.w}};
+        acc_add(v, w);
+        bigsum[blockIdx.x] = make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]);
     }
 }
 
-typedef void (*DDTermsFn)(double2 *, uint64_t, uint64_t, uint64_t, int, uint32_t, uint32_t, uint64_t);
+typedef void (*DDTermsFn)(uint4 *, uint64_t, uint64_t, uint64_t, int, uint32_t, uint32_t, uint64_t, int);
 
 static DDTermsFn dd_terms_fn(int level)
 {
@@ -753,56 +721,38 @@ int dd_terms_max_ctas_per_sm(int level)
     return n > 0 ? n : 1;
 }
 
-cudaError_t launch_dd_terms(int level, double2 *bigsum, int grid, int *blocks, uint64_t k0, uint64_t k1, uint64_t d,
-                            int sign, uint32_t den0, uint32_t den1, cudaStream_t st)
+cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *blocks, uint64_t k0, uint64_t k1, uint64_t d,
+                            int sign, uint32_t den0, uint32_t den1, bool tail, cudaStream_t st)
 {
     // eight tiles a resident warp: their costs fall along k, and each warp takes every eighth part
-    const uint64_t warps = (uint64_t)grid * (kBlockDD / 32), n = k1 - k0;
+    const uint64_t warps = (uint64_t)grid * (kBlockDD / 32), n = k1 > k0 ? k1 - k0 : 0;
     const uint64_t tile_k = std::max<uint64_t>(1, (n + 8 * 64 * warps - 1) / (8 * 64 * warps)) * 64;
-    *blocks = (int)std::min<uint64_t>(grid, (n + tile_k - 1) / tile_k);
-    dd_terms_fn(level)<<<*blocks, kBlockDD, 0, st>>>(bigsum, k0, k1, d, sign, den0, den1, tile_k);
+    *blocks = (int)std::min<uint64_t>(grid, std::max<uint64_t>(1, (n + tile_k - 1) / tile_k));
+    dd_terms_fn(level)<<<*blocks, kBlockDD, 0, st>>>(bigsum, k0, k0 + n, d, sign, den0, den1, tile_k, tail ? 1 : 0);
     return cudaGetLastError();
 }
 
-// One warp: lane i < 10 divides the tail term k = d + i, lane 0 adds them in order.
-__global__ void dd_tail_kernel(double2 *bigsum, uint64_t d, int sign, uint32_t den0, uint32_t den1)
+__global__ void __launch_bounds__(kBlockDD) dd_ssum_kernel(const uint4 *bigsum, int nblk, double2 *partial)
 {
-    const int lane = threadIdx.x;
-    DD t{0.0, 0.0};
-    if (lane < kTailDD) {
-        const uint64_t k = d + (uint64_t)lane;
-        const uint64_t m = (uint64_t)den0 * k + den1;
-        const double p = __longlong_as_double((1023ll - 10 * lane) << 52);      // 2^(-10 lane)
-        if (m != 1) {
-            t = (m < kDDMax) ? dd_div_nn(p, (double)m) : dd_div_dd(DD{p, 0.0}, dd_from_u64(m));
-            if ((k + (uint64_t)sign) & 1ull) { t.hi = -t.hi; t.lo = -t.lo; }
-        }
+    __shared__ uint32_t half[8];
+    if (threadIdx.x < 8) half[threadIdx.x] = 0;
+    __syncthreads();
+    Acc<4> acc;
+    acc_zero(acc);
+    for (int i = threadIdx.x; i < nblk; i += kBlockDD) {
+        const uint4 v = bigsum[i];
+        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+        acc_add(acc, q);
     }
-    DD sum{0.0, 0.0};
-    for (int i = 0; i < kTailDD; ++i)
-        sum = dd_add(sum, DD{__shfl_sync(0xffffffffu, t.hi, i), __shfl_sync(0xffffffffu, t.lo, i)});
-    if (lane == 0) {
-        const double2 o = bigsum[0];
-        const DD s = dd_frac(dd_add(DD{o.x, o.y}, sum));
-        bigsum[0] = make_double2(s.hi, s.lo);
+    uint32_t w[4];
+    block_sum128(acc, half, w);
+    if (threadIdx.x == 0) {
+        const DD v = dd_from_fraction(w);
+        *partial = make_double2(v.hi, v.lo);
     }
 }
 
-cudaError_t launch_dd_tail(double2 *bigsum, uint64_t d, int sign, uint32_t den0, uint32_t den1, cudaStream_t st)
-{
-    dd_tail_kernel<<<1, 32, 0, st>>>(bigsum, d, sign, den0, den1);
-    return cudaGetLastError();
-}
-
-__global__ void __launch_bounds__(kBlockDD) dd_ssum_kernel(const double2 *bigsum, int nblk, double2 *partial)
-{
-    DD s{0.0, 0.0};
-    for (int i = threadIdx.x; i < nblk; i += kBlockDD) s = dd_frac(dd_add(s, DD{bigsum[i].x, bigsum[i].y}));
-    const DD b = block_reduce_dd(s);
-    if (threadIdx.x == 0) *partial = make_double2(b.hi, b.lo);
-}
-
-cudaError_t launch_dd_ssum(const double2 *bigsum, int nblk, double2 *partial, cudaStream_t st)
+cudaError_t launch_dd_ssum(const uint4 *bigsum, int nblk, double2 *partial, cudaStream_t st)
 {
     dd_ssum_kernel<<<1, kBlockDD, 0, st>>>(bigsum, nblk, partial);
     return cudaGetLastError();

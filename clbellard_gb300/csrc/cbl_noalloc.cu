@@ -47,32 +47,50 @@ struct Piece {
     uint32_t kind;     // residue kind 1..6 (cbl_internal.h)
 };
 
+// First k with den0 k + den1 >= limit; with den0 and den1 known the division folds away.
+constexpr uint64_t first_k(uint64_t limit, uint64_t den0, uint64_t den1) { return (limit - den1 + den0 - 1) / den0; }
+
+struct KindCuts {
+    uint64_t k[7][5];
+};
+
+// Where each series passes the residue-kind boundaries 2^28, 2^31, 2^32, 2^44 and 2^60.
+constexpr KindCuts make_kind_cuts()
+{
+    KindCuts c{};
+    const uint64_t limit[5] = {kW1Max, kW1MMax, kW1SMax, kW2SMax, kW2Max};
+    for (int f = 0; f < 7; ++f)
+        for (int i = 0; i < 5; ++i) c.k[f][i] = first_k(limit[i], f < 2 ? 4 : 10, (0x9753131u >> (4 * f)) & 15u);
+    return c;
+}
+
+[[maybe_unused]] constexpr KindCuts kCuts = make_kind_cuts();
+__constant__ KindCuts d_cuts = make_kind_cuts();
+
 // The pieces of series f at position d, in increasing k. k = 0 of a series
 // with den1 = 1 has m = 1 and contributes exactly 0, so it is left out.
 __host__ __device__ inline int series_pieces(uint64_t d, int f, Piece out[kMaxPieces])
 {
-    const uint64_t den0 = series_den0(f), den1 = series_den1(f);
-    const uint64_t k0 = den1 == 1 ? 1 : 0, k1 = d + kTail192;
-    const uint64_t cut[6] = {d,
-                             (kW1Max - den1 + den0 - 1) / den0,     // first k with m >= 2^28
-                             (kW1MMax - den1 + den0 - 1) / den0,    // 2^31
-                             (kW1SMax - den1 + den0 - 1) / den0,    // 2^32
-                             (kW2SMax - den1 + den0 - 1) / den0,    // 2^44
-                             (kW2Max - den1 + den0 - 1) / den0};    // 2^60
-    uint64_t pts[8] = {k0, k1};
-    for (int i = 0; i < 6; ++i) pts[2 + i] = cut[i] < k0 ? k0 : (cut[i] > k1 ? k1 : cut[i]);
-    for (int i = 1; i < 8; ++i)                                      // insertion sort
-        for (int j = i; j > 0 && pts[j - 1] > pts[j]; --j) {
-            const uint64_t t = pts[j];
-            pts[j] = pts[j - 1];
-            pts[j - 1] = t;
-        }
+#ifdef __CUDA_ARCH__
+    const uint64_t *cut = d_cuts.k[f];
+#else
+    const uint64_t *cut = kCuts.k[f];
+#endif
+    constexpr uint32_t kind[6] = {1, 5, 3, 4, 2, 6};
+    uint64_t k = series_den1(f) == 1 ? 1 : 0;
+    const uint64_t k1 = d + kTail192;
     int n = 0;
-    for (int i = 0; i + 1 < 8; ++i) {
-        const uint64_t a = pts[i], b = pts[i + 1];
-        if (b <= a) continue;
-        const uint32_t kind = a >= cut[5] ? 6 : a >= cut[4] ? 2 : a >= cut[3] ? 4 : a >= cut[2] ? 3 : a >= cut[1] ? 5 : 1;
-        out[n++] = Piece{a, b, kind};
+    for (int i = 0; i < 6; ++i) {                                    // main body and tail of each kind's range
+        const uint64_t end = i < 5 && cut[i] < k1 ? cut[i] : k1;
+        const uint64_t body = end < d ? end : d;
+        if (k < body) {
+            out[n++] = Piece{k, body, kind[i]};
+            k = body;
+        }
+        if (k < end) {
+            out[n++] = Piece{k, end, kind[i]};
+            k = end;
+        }
     }
     return n;
 }
@@ -101,19 +119,24 @@ struct PositionArgs {
 // process exits; all calls on a device share it.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
-// One block of kMaxPos threads, thread i for position i. The table is ordered
+// One block, thread i for position i (of kMaxPos). The table is ordered
 // costliest tiles first: by bucket, then by d (larger first, ties by position
 // index), then by series; a series has at most one piece per bucket. Thread i
-// counts its pieces and tiles per bucket under its rank in that d order, one
-// thread turns the counts into offsets, then every thread writes its segments.
+// counts its pieces and tiles per bucket under its rank in that d order, the block
+// scans the counts (bucket-major, then rank) into offsets, 12 cells a thread, then
+// every thread writes its segments. One thread doing the scan, and 64-bit divisions
+// for the cuts, made this 34 us of a 1.46 ms call.
 __global__ void __launch_bounds__(kMaxPos) noalloc_table_kernel(PositionArgs a, Seg *segs)
 {
-    __shared__ uint32_t seg_off[kBuckets][kMaxPos];
-    __shared__ uint64_t tile_off[kBuckets][kMaxPos];
+    __shared__ uint32_t seg_off[kBuckets * kMaxPos];
+    __shared__ uint64_t tile_off[kBuckets * kMaxPos];
+    __shared__ uint32_t warp_segs;
+    __shared__ uint64_t warp_tiles;
+    static_assert(kMaxPos == 64, "two warps scan");
     const int i = threadIdx.x;
     for (int b = 0; b < kBuckets; ++b) {
-        seg_off[b][i] = 0;
-        tile_off[b][i] = 0;
+        seg_off[b * kMaxPos + i] = 0;
+        tile_off[b * kMaxPos + i] = 0;
     }
     __syncthreads();
     int rank = 0;
@@ -126,44 +149,62 @@ __global__ void __launch_bounds__(kMaxPos) noalloc_table_kernel(PositionArgs a, 
         for (int f = 0; f < 7; ++f) {
             const int np = series_pieces(d, f, p);
             for (int q = 0; q < np; ++q) {
-                const int b = piece_bucket(p[q], d);
-                seg_off[b][rank] += 1;
-                tile_off[b][rank] += piece_tiles(p[q]);
+                const int c = piece_bucket(p[q], d) * kMaxPos + rank;
+                seg_off[c] += 1;
+                tile_off[c] += piece_tiles(p[q]);
             }
         }
     }
     __syncthreads();
-    if (i == 0) {                                           // exclusive scan, bucket-major then rank
-        uint32_t s = 0;
-        uint64_t t = 0;
-        for (int b = 0; b < kBuckets; ++b)
-            for (int r = 0; r < a.n; ++r) {
-                const uint32_t cs = seg_off[b][r];
-                const uint64_t ct = tile_off[b][r];
-                seg_off[b][r] = s;
-                tile_off[b][r] = t;
-                s += cs;
-                t += ct;
-            }
+    uint32_t s = 0;                                         // exclusive scan over cells 12 i .. 12 i + 11
+    uint64_t t = 0;
+    for (int c = kBuckets * i; c < kBuckets * (i + 1); ++c) {
+        s += seg_off[c];
+        t += tile_off[c];
+    }
+    const uint32_t own_s = s;
+    const uint64_t own_t = t;
+    for (int w = 1; w < 32; w *= 2) {
+        const uint32_t us = __shfl_up_sync(0xffffffffu, s, w);
+        const uint64_t ut = __shfl_up_sync(0xffffffffu, t, w);
+        if ((i & 31) >= w) {
+            s += us;
+            t += ut;
+        }
+    }
+    if (i == 31) {
+        warp_segs = s;
+        warp_tiles = t;
+    }
+    __syncthreads();
+    s += (i >= 32 ? warp_segs : 0) - own_s;
+    t += (i >= 32 ? warp_tiles : 0) - own_t;
+    for (int c = kBuckets * i; c < kBuckets * (i + 1); ++c) {
+        const uint32_t cs = seg_off[c];
+        const uint64_t ct = tile_off[c];
+        seg_off[c] = s;
+        tile_off[c] = t;
+        s += cs;
+        t += ct;
     }
     __syncthreads();
     if (i >= a.n) return;
     for (int f = 0; f < 7; ++f) {
         const int np = series_pieces(d, f, p);
         for (int q = 0; q < np; ++q) {
-            const int b = piece_bucket(p[q], d);
+            const int c = piece_bucket(p[q], d) * kMaxPos + rank;
             Seg s;
             s.d = d;
             s.k0 = p[q].k0;
             s.k1 = p[q].k1;
-            s.tile0 = tile_off[b][rank];
+            s.tile0 = tile_off[c];
             s.den0 = series_den0(f);
             s.den1 = series_den1(f);
             s.slot = (uint32_t)(i * 7 + f);
             s.flags = (uint32_t)series_sign(f) | (p[q].kind << 4);
-            segs[seg_off[b][rank]] = s;
-            seg_off[b][rank] += 1;                          // this (bucket, rank) cell is this thread's alone
-            tile_off[b][rank] += piece_tiles(p[q]);
+            segs[seg_off[c]] = s;
+            seg_off[c] += 1;                                // this (bucket, rank) cell is this thread's alone
+            tile_off[c] += piece_tiles(p[q]);
         }
     }
 }
