@@ -41,15 +41,18 @@ struct cbl_ctx {
     int tile_k = kDefaultTile;
     int ctas_per_sm = 0;
     // 192-bit buffers
-    Seg *d_segs = nullptr;
-    Seg *h_segs = nullptr;
-    int seg_cap = 0;
+    // tile table: the segments, then (prepared passes) one shift per position
+    unsigned char *d_table = nullptr;
+    unsigned char *h_table = nullptr;         // its pinned staging
+    size_t table_cap = 0;
+    bool staging_busy = false;                // h_table may still feed a copy in flight
+    Seg *d_segs = nullptr;                    // = d_table
+    int *d_shift = nullptr;                   // inside d_table
     unsigned long long *d_counter = nullptr;
     unsigned long long *d_slots = nullptr;   // nslot x 6 digit sums; slot 0 is bigSum
     int slot_cap = 0;
     uint64_t *d_partial = nullptr;           // 3 words, most significant first
     uint64_t *d_ans = nullptr;               // 3 words
-    int *d_shift = nullptr;
     uint64_t *d_out3 = nullptr;
     uint64_t *h_out3 = nullptr;
     int pos_cap = 0;
@@ -68,7 +71,6 @@ struct cbl_ctx {
     cudaGraphExec_t graph = nullptr;                 // captured prepared pass
     bool use_graph = true;
     int partial = 0;                                 // a budgeted run is in progress
-    uint64_t seg_hash = 0;                           // identity of the prepared tile table
     std::vector<Seg> prep_segs;                      // host copy of the prepared segments
     std::vector<int> prep_shift;
     // double-double buffers
@@ -102,18 +104,41 @@ void drop_graph(cbl_ctx *c)
     c->graph = nullptr;
 }
 
-int ensure_segs(cbl_ctx *c, int n)
+int sync(cbl_ctx *c)
 {
-    if (n <= c->seg_cap) return CBL_OK;
-    int cap = std::max(n, 2 * c->seg_cap);
-    if (c->d_segs) cudaFree(c->d_segs);
-    if (c->h_segs) cudaFreeHost(c->h_segs);
-    c->d_segs = nullptr;
-    c->h_segs = nullptr;
-    c->seg_cap = 0;
-    if (cudaMalloc(&c->d_segs, sizeof(Seg) * cap) != cudaSuccess) return CBL_E_NOMEM;
-    if (cudaMallocHost(&c->h_segs, sizeof(Seg) * cap) != cudaSuccess) return CBL_E_NOMEM;
-    c->seg_cap = cap;
+    CK(cudaStreamSynchronize(c->st));
+    c->staging_busy = false;
+    return CBL_OK;
+}
+
+int ensure_table(cbl_ctx *c, size_t bytes)
+{
+    if (bytes <= c->table_cap) return CBL_OK;
+    const size_t cap = std::max(bytes, 2 * c->table_cap);
+    cudaFree(c->d_table);
+    cudaFreeHost(c->h_table);
+    c->d_table = c->h_table = nullptr;
+    c->table_cap = 0;
+    if (cudaMalloc(&c->d_table, cap) != cudaSuccess) return CBL_E_NOMEM;
+    if (cudaMallocHost(&c->h_table, cap) != cudaSuccess) return CBL_E_NOMEM;
+    c->table_cap = cap;
+    return CBL_OK;
+}
+
+// Upload a tile table (segments, then n shifts) through the pinned staging buffer,
+// waiting for the stream only where an earlier copy may still read that buffer.
+int upload_table(cbl_ctx *c, const std::vector<Seg> &v, const int *shift, int n)
+{
+    const size_t seg_bytes = sizeof(Seg) * v.size(), bytes = seg_bytes + sizeof(int) * (size_t)n;
+    int rc = c->staging_busy ? sync(c) : CBL_OK;
+    if (!rc) rc = ensure_table(c, bytes);
+    if (rc) return rc;
+    std::memcpy(c->h_table, v.data(), seg_bytes);
+    if (n > 0) std::memcpy(c->h_table + seg_bytes, shift, sizeof(int) * (size_t)n);
+    c->staging_busy = true;
+    CK(cudaMemcpyAsync(c->d_table, c->h_table, bytes, cudaMemcpyHostToDevice, c->st));
+    c->d_segs = reinterpret_cast<Seg *>(c->d_table);
+    c->d_shift = reinterpret_cast<int *>(c->d_table + seg_bytes);
     return CBL_OK;
 }
 
@@ -137,14 +162,11 @@ int ensure_pos(cbl_ctx *c, int n)
 {
     if (n <= c->pos_cap) return CBL_OK;
     int cap = std::max(n, 2 * c->pos_cap);
-    if (c->d_shift) cudaFree(c->d_shift);
     if (c->d_out3) cudaFree(c->d_out3);
     if (c->h_out3) cudaFreeHost(c->h_out3);
-    c->d_shift = nullptr;
     c->d_out3 = nullptr;
     c->h_out3 = nullptr;
     c->pos_cap = 0;
-    if (cudaMalloc(&c->d_shift, sizeof(int) * cap) != cudaSuccess) return CBL_E_NOMEM;
     if (cudaMalloc(&c->d_out3, sizeof(uint64_t) * 3 * cap) != cudaSuccess) return CBL_E_NOMEM;
     if (cudaMallocHost(&c->h_out3, sizeof(uint64_t) * 3 * cap) != cudaSuccess) return CBL_E_NOMEM;
     c->pos_cap = cap;
@@ -246,19 +268,14 @@ int run_segments(cbl_ctx *c, std::vector<Seg> &v)
 {
     if (v.empty()) return CBL_OK;
     const uint64_t ntiles = order_and_number(v, (uint32_t)c->tile_k);
-    int rc = ensure_segs(c, (int)v.size());
+    const int rc = upload_table(c, v, nullptr, 0);
     if (rc) return rc;
-    // the pinned staging buffer may still feed an earlier async copy
-    CK(cudaStreamSynchronize(c->st));
-    std::memcpy(c->h_segs, v.data(), sizeof(Seg) * v.size());
-    CK(cudaMemcpyAsync(c->d_segs, c->h_segs, sizeof(Seg) * v.size(), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), c->st));
     // slot 0 collects every launch since cbl_Set0mem: carry once it may have
     // taken 2^31 flushes (at most one per tile)
     c->slot0_tiles = std::min<uint64_t>(c->slot0_tiles + ntiles, kCarryTiles);
     const int level = segs_level(v);
     CK(launch_terms192(level, c->d_segs, (int)v.size(), ntiles, (uint32_t)c->tile_k, c->d_counter, c->d_slots,
-                       grid_192(c, level), c->st, 0, slot_needs_carry(c->slot0_tiles)));
+                       grid_192(c, level), c->st, 0, slot_needs_carry(c->slot0_tiles), true));
     c->launches++;
     return CBL_OK;
 }
@@ -281,12 +298,6 @@ int dd_range(cbl_ctx *c, uint64_t k0, uint64_t k1, uint64_t d, int sign, uint32_
         c->launches++;
         if (last) break;
     }
-    return CBL_OK;
-}
-
-int sync(cbl_ctx *c)
-{
-    CK(cudaStreamSynchronize(c->st));
     return CBL_OK;
 }
 
@@ -454,7 +465,7 @@ int cbl_create(int device, int precision, cbl_ctx **out)
     if (!rc && cudaEventCreate(&c->ev_k0) != cudaSuccess) rc = CBL_E_CUDA;
     if (!rc && cudaEventCreate(&c->ev_k1) != cudaSuccess) rc = CBL_E_CUDA;
     if (!rc) rc = ensure_slots(c, 8);
-    if (!rc) rc = ensure_segs(c, 64);
+    if (!rc) rc = ensure_table(c, 64 * sizeof(Seg));
     if (!rc) rc = ensure_pos(c, 1);
     if (!rc) {
         cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6 * c->slot_cap, c->st);
@@ -480,13 +491,12 @@ int cbl_destroy(cbl_ctx *c)
     if (!c) return CBL_E_ARG;
     cudaSetDevice(c->device);
     if (c->st) cudaStreamSynchronize(c->st);
-    cudaFree(c->d_segs);
-    cudaFreeHost(c->h_segs);
+    cudaFree(c->d_table);
+    cudaFreeHost(c->h_table);
     cudaFree(c->d_counter);
     cudaFree(c->d_slots);
     cudaFree(c->d_partial);
     cudaFree(c->d_ans);
-    cudaFree(c->d_shift);
     cudaFree(c->d_out3);
     cudaFreeHost(c->h_out3);
     cudaFree(c->d_kbuf);
@@ -734,7 +744,10 @@ int cbl_query(cbl_ctx *c)
     CBL_GUARD_BEGIN
     if (!c) return CBL_E_ARG;
     const cudaError_t e = cudaStreamQuery(c->st);
-    if (e == cudaSuccess) return 0;
+    if (e == cudaSuccess) {
+        c->staging_busy = false;
+        return 0;
+    }
     if (e == cudaErrorNotReady) {
         cudaGetLastError();
         return 1;
@@ -767,6 +780,13 @@ static uint64_t fnv1a(const void *p, size_t n, uint64_t h = 1469598103934665603u
     return h;
 }
 
+// Identity of the prepared tile table, for checkpoints.
+static uint64_t seg_hash(const cbl_ctx *c)
+{
+    return fnv1a(c->prep_shift.data(), sizeof(int) * c->prep_npos,
+                 fnv1a(c->prep_segs.data(), sizeof(Seg) * c->prep_segs.size()));
+}
+
 // Number the prepared segments' tiles for the current tile size and upload
 // them with the per-position shifts (again after a tile-size change).
 static int upload_prepared(cbl_ctx *c)
@@ -782,20 +802,13 @@ static int upload_prepared(cbl_ctx *c)
         max_slot_tiles = std::max(max_slot_tiles, t);
     }
     c->prep_carry = slot_needs_carry(max_slot_tiles);
-    int rc = ensure_segs(c, (int)v.size());
+    const int rc = upload_table(c, v, c->prep_shift.data(), n);
     if (rc) return rc;
-    CK(cudaStreamSynchronize(c->st));
-    std::memcpy(c->h_segs, v.data(), sizeof(Seg) * v.size());
-    CK(cudaMemcpyAsync(c->d_segs, c->h_segs, sizeof(Seg) * v.size(), cudaMemcpyHostToDevice, c->st));
-    std::memcpy(c->h_out3, c->prep_shift.data(), sizeof(int) * n);      // pinned staging for the shifts
-    CK(cudaMemcpyAsync(c->d_shift, c->h_out3, sizeof(int) * n, cudaMemcpyHostToDevice, c->st));
-    CK(cudaStreamSynchronize(c->st));
     drop_graph(c);
     c->prep_nseg = (int)v.size();
     c->prep_level = segs_level(v);
     c->prep_ntiles = ntiles;
     c->partial = 0;
-    c->seg_hash = fnv1a(c->prep_shift.data(), sizeof(int) * n, fnv1a(v.data(), sizeof(Seg) * v.size()));
     return CBL_OK;
 }
 
@@ -837,24 +850,25 @@ static cudaError_t clear_slots(cbl_ctx *c, int nslot)
 }
 
 // Enqueue the prepared pass: zero slots and tile counter, the persistent term
-// kernel between two events, the combine kernel. The first pass after a
-// prepare is captured into a CUDA graph and every later pass replays it.
-static int enqueue_prepared(cbl_ctx *c, bool capturing)
+// kernel between two events, the combine kernel. host3, ans: further places
+// (pinned host memory, dev_ans) that the combine kernel writes the results to.
+static int enqueue_prepared(cbl_ctx *c, bool capturing, uint64_t *host3, uint64_t *ans)
 {
     // inside a capture the events must be external records so that the graph
     // records them when it is replayed; outside a capture that flag is refused
     const unsigned int evf = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
     const int n = c->prep_npos;
     CK(clear_slots(c, 7 * n));
-    CK(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), c->st));
     CK(cudaEventRecordWithFlags(c->ev_k0, c->st, evf));
     CK(launch_terms192(c->prep_level, c->d_segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k, c->d_counter,
-                       c->d_slots, grid_192(c, c->prep_level), c->st, 0, prepared_carry(c)));
+                       c->d_slots, grid_192(c, c->prep_level), c->st, 0, prepared_carry(c), true));
     CK(cudaEventRecordWithFlags(c->ev_k1, c->st, evf));
-    CK(launch_combine(c->d_slots, n, c->d_shift, c->d_out3, nullptr, c->st));
+    CK(launch_combine(c->d_slots, n, c->d_shift, c->d_out3, host3, ans, c->st));
     return CBL_OK;
 }
 
+// The first pass after a prepare is captured into a CUDA graph and every later
+// pass replays it.
 static int launch_prepared(cbl_ctx *c)
 {
     if (c->prep_npos <= 0) return CBL_E_ARG;
@@ -863,7 +877,7 @@ static int launch_prepared(cbl_ctx *c)
         if (!c->graph) {
             cudaGraph_t g = nullptr;
             CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-            const int rc = enqueue_prepared(c, true);
+            const int rc = enqueue_prepared(c, true, nullptr, nullptr);
             const cudaError_t e = cudaStreamEndCapture(c->st, &g);
             if (rc || e != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
@@ -878,7 +892,7 @@ static int launch_prepared(cbl_ctx *c)
         }
         CK(cudaGraphLaunch(c->graph, c->st));
     } else {
-        const int rc = enqueue_prepared(c, false);
+        const int rc = enqueue_prepared(c, false, nullptr, nullptr);
         if (rc) return rc;
     }
     c->ev_valid = true;
@@ -886,20 +900,23 @@ static int launch_prepared(cbl_ctx *c)
     return CBL_OK;
 }
 
-static int run_positions(cbl_ctx *c, const uint64_t *d, const int *shift, int n)
+// Prepare n positions, run one pass and wait: the results are in h_out3 (and,
+// with to_ans, position 0's in dev_ans). A pass that is run once is launched
+// directly: capturing and instantiating a graph for it took 30 us of an 80 us call.
+static int run_positions(cbl_ctx *c, const uint64_t *d, const int *shift, int n, bool to_ans)
 {
     int rc = prepare_positions(c, d, shift, n);
-    return rc ? rc : launch_prepared(c);
+    if (!rc) rc = enqueue_prepared(c, false, c->h_out3, to_ans ? c->d_ans : nullptr);
+    if (rc) return rc;
+    c->ev_valid = true;
+    c->launches += 2;
+    return sync(c);
 }
 
 static int compute_d(cbl_ctx *c, uint64_t d, int shift, char hex[49])
 {
     if (is192(c)) {
-        int rc = run_positions(c, &d, &shift, 1);
-        if (rc) return rc;
-        CK(cudaMemcpyAsync(c->d_ans, c->d_out3, 24, cudaMemcpyDeviceToDevice, c->st));
-        CK(cudaMemcpyAsync(c->h_out3, c->d_out3, 24, cudaMemcpyDeviceToHost, c->st));
-        rc = sync(c);
+        const int rc = run_positions(c, &d, &shift, 1, true);
         if (rc) return rc;
         to_hex192(c->h_out3, hex);
         return CBL_OK;
@@ -1206,10 +1223,7 @@ int cbl_batch(cbl_ctx *c, const uint64_t *pos, int n, uint64_t *out3n)
         if (rc) return rc;
     }
     cudaSetDevice(c->device);
-    int rc = run_positions(c, d.data(), sh.data(), n);
-    if (rc) return rc;
-    CK(cudaMemcpyAsync(c->h_out3, c->d_out3, sizeof(uint64_t) * 3 * n, cudaMemcpyDeviceToHost, c->st));
-    rc = sync(c);
+    const int rc = run_positions(c, d.data(), sh.data(), n, false);
     if (rc) return rc;
     std::memcpy(out3n, c->h_out3, sizeof(uint64_t) * 3 * n);
     return CBL_OK;
@@ -1397,14 +1411,14 @@ int cbl_run_prepared_budget(cbl_ctx *c, double budget_ms, uint64_t *tiles_done, 
     }
     const uint64_t budget_ns = (uint64_t)(budget_ms * 1e6) + 1;
     CK(launch_terms192(c->prep_level, c->d_segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k, c->d_counter,
-                       c->d_slots, grid_192(c, c->prep_level), c->st, budget_ns, prepared_carry(c)));
+                       c->d_slots, grid_192(c, c->prep_level), c->st, budget_ns, prepared_carry(c), false));
     c->launches++;
     CK(cudaMemcpyAsync(c->h_small, c->d_counter, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->st));
     int rc = sync(c);
     if (rc) return rc;
     const uint64_t done = std::min<uint64_t>(c->h_small[0], c->prep_ntiles);
     if (done >= c->prep_ntiles) {
-        CK(launch_combine(c->d_slots, n, c->d_shift, c->d_out3, nullptr, c->st));
+        CK(launch_combine(c->d_slots, n, c->d_shift, c->d_out3, nullptr, nullptr, c->st));
         c->launches++;
         c->partial = 0;
     }
@@ -1433,7 +1447,7 @@ int cbl_checkpoint_save(cbl_ctx *c, void *buf, int64_t size)
     cudaSetDevice(c->device);
     int rc = sync(c);
     if (rc) return rc;
-    CkptHeader h{kCkptMagic, c->seg_hash, (uint64_t)c->prep_npos, c->prep_ntiles, 0};
+    CkptHeader h{kCkptMagic, seg_hash(c), (uint64_t)c->prep_npos, c->prep_ntiles, 0};
     if (c->partial) {
         CK(cudaMemcpy(&h.done, c->d_counter, sizeof(uint64_t), cudaMemcpyDeviceToHost));
         h.done = std::min<uint64_t>(h.done, c->prep_ntiles);
@@ -1455,7 +1469,7 @@ int cbl_checkpoint_load(cbl_ctx *c, const void *buf, int64_t size)
     CkptHeader h;
     std::memcpy(&h, buf, sizeof h);
     if (h.magic != kCkptMagic) return CBL_E_FORMAT;
-    if (h.hash != c->seg_hash || h.npos != (uint64_t)c->prep_npos || h.ntiles != c->prep_ntiles || h.done > h.ntiles)
+    if (h.hash != seg_hash(c) || h.npos != (uint64_t)c->prep_npos || h.ntiles != c->prep_ntiles || h.done > h.ntiles)
         return CBL_E_FORMAT;                               // not a checkpoint of this prepared run
     cudaSetDevice(c->device);
     CK(cudaMemcpy(c->d_slots, static_cast<const char *>(buf) + sizeof h,

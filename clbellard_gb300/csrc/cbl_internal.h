@@ -75,6 +75,7 @@ struct TileSplit {
 // Launch wrappers (cbl_kernels.cu).
 // budget_ns = 0: run to the end; else warps stop taking tiles after budget_ns
 // and the finished tiles are [0, *counter).
+// reset_counter: zero the tile counter first, where the launch uses it.
 // carry: the slots' digit sums may wrap past 2^64 (a slot can receive 2^31 or
 // more flushes since it was zeroed, or it started from a preset); the flushes
 // then carry each wrap into the digit sum two places up (exact mod 2^192).
@@ -82,14 +83,15 @@ struct TileSplit {
 // from the tile counts.
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
                             unsigned long long *counter, unsigned long long *slots, int grid, cudaStream_t st,
-                            uint64_t budget_ns, bool carry);
+                            uint64_t budget_ns, bool carry, bool reset_counter);
 constexpr uint64_t kCarryTiles = 1ull << 31;
 inline bool slot_needs_carry(uint64_t max_tiles_per_slot) { return max_tiles_per_slot >= kCarryTiles; }
-// slots (nslot x 6 digit sums) of position i, series f = slots[(slot_base[i] + f) * 6 ..]:
+// slots (nslot x 6 digit sums) of position i, series f = slots[(7 i + f) * 6 ..]:
 // out3[3i..3i+2] (word 0 most significant) = sum_f (S_f << (numer_log2[f] + shift[i])).
-// If partial7 != nullptr it also receives the 7 weighted partials per position.
+// The same words also go to copy3 (n positions, may be pinned host memory) and, for
+// position 0, to first3, where those are not null.
 cudaError_t launch_combine(const unsigned long long *slots, int npos, const int *shift,
-                           uint64_t *out3, uint64_t *partial7, cudaStream_t st);
+                           uint64_t *out3, uint64_t *copy3, uint64_t *first3, cudaStream_t st);
 // slots[0 .. 6*nslot) <- preset[j % 6] (device array of 6), instead of zero.
 cudaError_t launch_slot_fill(unsigned long long *slots, int nslot, const unsigned long long *preset,
                              cudaStream_t st);

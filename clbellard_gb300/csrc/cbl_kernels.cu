@@ -399,11 +399,15 @@ TileSplit tile_split(uint64_t ntiles, uint32_t tile_k, int grid)
 
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
                             unsigned long long *counter, unsigned long long *slots, int grid, cudaStream_t st,
-                            uint64_t budget_ns, bool carry)
+                            uint64_t budget_ns, bool carry, bool reset_counter)
 {
     // a budgeted pass stops and resumes at whole tiles
     const TileSplit sp = budget_ns ? TileSplit{0, 0, tile_k} : tile_split(ntiles, tile_k, grid);
     if (sp.fixed) grid = (int)std::min<uint64_t>(grid, ntiles << sp.log2_parts);
+    if (reset_counter && !sp.fixed) {
+        const cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
+        if (e != cudaSuccess) return e;
+    }
     const Terms192Fn fn = sp.fixed ? terms192_fn<true>(level) : terms192_fn<false>(level);
     fn<<<grid, kBlock192, 0, st>>>(segs, nseg, ntiles, tile_k, sp, counter, slots, budget_ns, carry ? 1 : 0);
     return cudaGetLastError();
@@ -477,7 +481,7 @@ cudaError_t launch_slot_fill(unsigned long long *slots, int nslot, const unsigne
 }
 
 __global__ void combine_kernel(const unsigned long long *slots, int npos, const int *shift, uint64_t *out3,
-                               uint64_t *partial7)
+                               uint64_t *copy3, uint64_t *first3)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npos) return;
@@ -488,22 +492,21 @@ __global__ void combine_kernel(const unsigned long long *slots, int npos, const 
         uint64_t w[3];
         normalise6(slots + ((size_t)i * 7 + f) * 6, w);
         shl192(w, numer_log2(f) + sh);
-        if (partial7) {
-            uint64_t *p = partial7 + ((size_t)i * 7 + f) * 3;
-            p[0] = w[2]; p[1] = w[1]; p[2] = w[0];
-        }
         add192(ans, w);
     }
-    out3[3 * (size_t)i + 0] = ans[2];
-    out3[3 * (size_t)i + 1] = ans[1];
-    out3[3 * (size_t)i + 2] = ans[0];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        out3[3 * (size_t)i + j] = ans[2 - j];
+        if (copy3) copy3[3 * (size_t)i + j] = ans[2 - j];
+        if (first3 && i == 0) first3[j] = ans[2 - j];
+    }
 }
 
 cudaError_t launch_combine(const unsigned long long *slots, int npos, const int *shift, uint64_t *out3,
-                           uint64_t *partial7, cudaStream_t st)
+                           uint64_t *copy3, uint64_t *first3, cudaStream_t st)
 {
     const int b = 128;
-    combine_kernel<<<(npos + b - 1) / b, b, 0, st>>>(slots, npos, shift, out3, partial7);
+    combine_kernel<<<(npos + b - 1) / b, b, 0, st>>>(slots, npos, shift, out3, copy3, first3);
     return cudaGetLastError();
 }
 

@@ -295,9 +295,9 @@ extern "C" int cbl_batch_noalloc(const uint64_t *pos, int n, uint64_t *d_out3n, 
     if (cudaGetLastError() != cudaSuccess) return CBL_E_CUDA;
     const int level = term_level(0, max_m);
     if (launch_terms192(level, dsegs, nseg, ntiles, (uint32_t)kTileTerms, counter, slots, ds->grid[level], st, 0,
-                        slot_needs_carry(max_series_tiles)) != cudaSuccess)
+                        slot_needs_carry(max_series_tiles), false) != cudaSuccess)
         return CBL_E_CUDA;
-    if (launch_combine(slots, n, shift, d_out3n, nullptr, st) != cudaSuccess) return CBL_E_CUDA;
+    if (launch_combine(slots, n, shift, d_out3n, nullptr, nullptr, st) != cudaSuccess) return CBL_E_CUDA;
     return CBL_OK;
     CBL_GUARD_END
 }
