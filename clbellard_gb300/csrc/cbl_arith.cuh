@@ -14,9 +14,10 @@
 // (exact division by the odd m), so q_j is the Montgomery multiplier of the
 // step and no division is ever executed. The chain ends at r_0 = 2^(10e) mod m.
 //
-// Seven residue kinds:
-//   width 1 (m < 2^25; the formulas hold below 2^28): R = 2^32, residues kept lazily in [0, 4m).
-//   middle width 1 (2^25 <= m < 2^31): R = 2^32, residues in [0, m).
+// Eight residue kinds:
+//   width 1 (m < 2^17; the formulas hold below 2^28): R = 2^32, residues kept lazily in [0, 4m).
+//   lazy width 1 (2^17 <= m < 2^29): R = 2^32, residues in [0, 2m).
+//   middle width 1 (2^29 <= m < 2^31; holds from 2^25): R = 2^32, residues in [0, m).
 //   strict width 1 (2^31 <= m < 2^32): R = 2^32, signed residues.
 //   float-quotient width 2 (2^32 <= m < 94 * 2^32): R = 2^24, residues below 8m,
 //     the top of each square taken off by a float quotient.
@@ -277,11 +278,10 @@ __device__ __forceinline__ uint32_t w1s_start(uint32_t m, uint32_t p)
     return (uint32_t)r;
 }
 
-// A value congruent to 2^(32 + p), 1 <= p <= 15, for 2^25 <= m < 2^31, below m from
-// 2^28 on and below 1.8m under it (w1m_sqr then still gives a sum below 2m). The float
-// quotient (< 2^22, three roundings of 2^-24: within 0.75, and 0.1 from 2^28 on) less
-// 0.8 is rounded down, so -q m mod 2^32 is the positive rest, below 2m from 2^28 on
-// and below 2.8m under it.
+// A value congruent to 2^(32 + p) for m < 2^31 with 2^(32 + p) / m < 2^22: below m from
+// m = 2^28 on (p <= 15), below 1.8m otherwise. The float quotient (three roundings of
+// 2^-24: within 0.75, and 0.1 from 2^28 on) less 0.8 is rounded down, so -q m mod 2^32
+// is the positive rest, below 2m from 2^28 on and below 2.8m otherwise.
 __device__ __forceinline__ uint32_t w1m_start(uint32_t m, uint32_t p)
 {
     const float inv = rcp_approx(__uint2float_rn(m));
@@ -293,6 +293,35 @@ __device__ __forceinline__ uint32_t w1m_start(uint32_t m, uint32_t p)
 struct W1MStart {
     __device__ __forceinline__ void operator()(W1MState &st, uint32_t p) const { st.y = w1m_start(st.m, p); }
 };
+
+// ------------------------------------------------------- lazy width 1 --
+// 2^17 <= m < 2^29: the middle kind's step without its correction. With y < 2m,
+// y (2^b y) < 8m^2 and REDC gives less than 8m^2 / 2^32 + m < 2m again. (Shifting
+// one multiplicand, not the result, keeps the bound to 2^29.)
+struct W1LState {
+    uint32_t y, m, mp;
+    __device__ __forceinline__ void step(uint32_t b)
+    {
+        const uint64_t t = (uint64_t)y * (y << b);
+        const uint32_t u = (uint32_t)t * mp;
+        y = redc_word(u, m, (uint32_t)t, (uint32_t)(t >> 32));
+    }
+    __device__ __forceinline__ uint32_t residue() const { return min(y, y - m); }
+};
+
+struct W1LStart {
+    __device__ __forceinline__ void operator()(W1LState &st, uint32_t p) const { st.y = w1m_start(st.m, p); }
+};
+
+// r6 = 2^E mod m in [0, m) from the leading NB bits of E - 32 at once: NB = 3 for
+// 2^17 <= m, 4 for 2^25 <= m (the start's bound on 2^(32 + p) / m).
+template <int NB>
+__device__ __forceinline__ uint32_t w1l_pow2(uint64_t E, uint32_t m, uint32_t mp)
+{
+    W1LState st{0, m, mp};
+    walk_bits_start<NB>(E - 32, st, W1LStart{});
+    return st.residue();
+}
 
 // r6 = 2^E mod m in [0, m) for E >= 42, 2^25 <= m < 2^31. The start value
 // takes the leading up-to-four bits of E - 32 at once.
@@ -720,8 +749,9 @@ __device__ __forceinline__ void walk_bits_start_pair(uint64_t EpA, uint64_t EpB,
 // agree above bit S, those bits come from one word P and both ladders share the
 // shift counts, and so they do in the last six bits (EpA - EpB = 320 = 5 * 2^6).
 // Other groups, and exponents outside [2^(S+4) + 630, 2^(S+32)), walk their own bits.
-// S: 12 / 13 / 14 / 15 measured 127.0 / 125.9 / 125.1 / 125.2 ms on 512 positions below 1e8.
-constexpr int kGroupBits = 14;
+// S = 12 / 13 / 14 / 15 / 16 measured 113.9 / 110.4 / 108.9 / 108.2 / 107.6 ms on 512 positions
+// below 1e8.
+constexpr int kGroupBits = 16;
 template <int NB, typename State, typename Start>
 __device__ __forceinline__ void walk_bits_group(uint64_t EpA, uint64_t EpB, uint64_t ep_max, State &A, State &B,
                                                 Start start)

@@ -25,7 +25,9 @@ constexpr uint32_t kDen1[7] = {1, 3, 1, 3, 5, 7, 9};
 
 // Residue-width limits of the term kernels (m odd, m >= 3).
 constexpr uint64_t kW1Max = 1ull << 28;   // width 1 (one 32-bit word) for m < 2^28
-constexpr uint64_t kW1MMin = 1ull << 25;  // width-1 tiles from here on run the middle kind's steps
+constexpr uint64_t kW1L3Min = 1ull << 17; // lazy width-1 steps, started from three exponent bits, ...
+constexpr uint64_t kW1L4Min = 1ull << 25; // ... from four, ...
+constexpr uint64_t kW1LMax = 1ull << 29;  // ... up to here, in width-1 and middle tiles
 constexpr uint64_t kW1MMax = 1ull << 31;  // middle width 1 for 2^28 <= m < 2^31
 constexpr uint64_t kW1SMax = 1ull << 32;  // strict width 1 for 2^31 <= m < 2^32
 constexpr uint64_t kW2FLow = 15ull << 34; // float-quotient steps without an offset for 2^32 <= m < 15 * 2^34

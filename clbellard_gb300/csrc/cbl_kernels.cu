@@ -15,7 +15,7 @@
 
 namespace cbl {
 
-constexpr int kBlock192 = 256;
+constexpr int kBlock192 = 128;
 
 // numer of series f as a shift (KernelFuncs.as:9): 32,1,256,64,4,4,1
 __device__ __forceinline__ int numer_log2(int f)
@@ -50,7 +50,8 @@ __device__ __forceinline__ void shr_digits(uint32_t q[N], int s)
 
 // One term's N quotient digits: k < d gives frac(2^(10(d-k))/m), k >= d the
 // tail value 2^(-10(k-d))/m (digits of 1/m shifted right by 10(k-d)).
-// KIND: 1 = width 1 (m < 2^28), 5 = middle width 1 (2^25 <= m < 2^31),
+// KIND: 1 = width 1 (m < 2^28), 9 and 10 = lazy width 1 with a start of three (2^17 <= m
+// < 2^29) and four bits (2^25 <= m < 2^29), 5 = middle width 1 (2^25 <= m < 2^31),
 // 3 = strict width 1 (2^28 <= m < 2^32), 7 and 8 = float-quotient width 2 (2^32 <= m
 // < 15 * 2^34 and < 94 * 2^32), 4 = short width 2 (2^32 <= m < 2^44),
 // 2 = width 2 (2^28 <= m < 2^60), 6 = wide width 2 (2^60 <= m < 2^62).
@@ -61,6 +62,9 @@ __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, 
     const uint64_t E = TAIL ? 32ull * N : 10ull * (d - k) + 32ull * N;
     if (KIND == 1) {
         const uint32_t r = w1_pow2(E, (uint32_t)m, mp);
+        w1_digits<N>(r, (uint32_t)m, mp, q);
+    } else if (KIND == 9 || KIND == 10) {
+        const uint32_t r = w1l_pow2<KIND == 9 ? 3 : 4>(E, (uint32_t)m, mp);
         w1_digits<N>(r, (uint32_t)m, mp, q);
     } else if (KIND == 5) {
         const uint32_t r = w1m_pow2(E, (uint32_t)m, mp);
@@ -95,7 +99,8 @@ template <int KIND, int N>
 __device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t ma, uint64_t mb, uint32_t qa[N],
                                           uint32_t qb[N])
 {
-    const uint32_t mpa = neg_inv32((uint32_t)ma), mpb = neg_inv32((uint32_t)mb);
+    const uint32_t mpab = neg_inv32((uint32_t)ma * (uint32_t)mb);      // one inverse for both
+    const uint32_t mpa = mpab * (uint32_t)mb, mpb = mpab * (uint32_t)ma;
     const uint64_t Eb = Ea - 320ull;
     if (KIND == 7 || KIND == 8) {
         uint64_t ra, rb;
@@ -122,6 +127,11 @@ __device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t 
         yb = min(yb, yb - (uint32_t)mb);
         w1_digits<N>(ya, (uint32_t)ma, mpa, qa);
         w1_digits<N>(yb, (uint32_t)mb, mpb, qb);
+    } else if (KIND == 9 || KIND == 10) {
+        W1LState A{0, (uint32_t)ma, mpa}, B{0, (uint32_t)mb, mpb};
+        walk_bits_group<KIND == 9 ? 3 : 4>(Ea - 32, Eb - 32, e_max - 32, A, B, W1LStart{});
+        w1_digits<N>(A.residue(), (uint32_t)ma, mpa, qa);
+        w1_digits<N>(B.residue(), (uint32_t)mb, mpb, qb);
     } else if (KIND == 5) {
         W1MState A{0, (uint32_t)ma, mpa}, B{0, (uint32_t)mb, mpb};
         walk_bits_group<4>(Ea - 32, Eb - 32, e_max - 32, A, B, W1MStart{});
@@ -140,7 +150,7 @@ __device__ __forceinline__ void run_tile(const Seg &s, uint64_t kb, uint64_t ke,
                                          uint32_t &cnt)
 {
     uint64_t k = kb + lane;
-    if (!TAIL && (KIND == 1 || KIND == 3 || KIND == 4 || KIND == 5 || KIND == 7 || KIND == 8)) {
+    if (!TAIL && KIND != 2 && KIND != 6) {
         constexpr bool wide = KIND == 4 || KIND == 7 || KIND == 8;
         uint64_t ea = 10ull * (s.d - k) + 32ull * N, ma = (uint64_t)s.den0 * k + s.den1;
         uint64_t e_max = ea + 10u * lane;
@@ -294,8 +304,13 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
     } else if (LEVEL >= 2 && width == 2) run_tile<2, TAIL>(s, kb, ke, lane, acc, cnt);
     else if (LEVEL >= 2 && width == 6) run_tile<6, TAIL>(s, kb, ke, lane, acc, cnt);
     else if (width == 3) run_tile<3, TAIL>(s, kb, ke, lane, acc, cnt);
-    else if (width == 5 || (uint64_t)s.den0 * kb + s.den1 >= kW1MMin) run_tile<5, TAIL>(s, kb, ke, lane, acc, cnt);
-    else run_tile<1, TAIL>(s, kb, ke, lane, acc, cnt);
+    else {
+        const uint64_t m_first = (uint64_t)s.den0 * kb + s.den1, m_last = (uint64_t)s.den0 * (ke - 1) + s.den1;
+        if (m_last >= kW1LMax) run_tile<5, TAIL>(s, kb, ke, lane, acc, cnt);
+        else if (m_first >= kW1L4Min) run_tile<10, TAIL>(s, kb, ke, lane, acc, cnt);
+        else if (m_first >= kW1L3Min) run_tile<9, TAIL>(s, kb, ke, lane, acc, cnt);
+        else run_tile<1, TAIL>(s, kb, ke, lane, acc, cnt);
+    }
 }
 
 // With budget_ns != 0 a warp takes no new tile once budget_ns have passed
@@ -306,13 +321,13 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
 // flushes them when it moves to another segment, when a lane's term count
 // reaches 2^30, and before it exits: one slot update per run of tiles
 // instead of one per tile. (split: see tile_split.)
-// Registers: the one-word kinds run best at 5 CTAs an SM with 46 registers (1e9:
-// 35.9 ms; 37.4 ms with the 40 that ptxas takes unbounded, 36.2 ms at 4 CTAs),
-// the float-quotient kind at 64 registers and 4 CTAs (1e10: 561.7 ms; 591 ms when held
-// to 48 registers for 5 CTAs, with spills), the single ladders of the general
-// two-word kinds at 5 CTAs (2^27 terms at 1e13: 5.81 ms against 5.96 ms at 4).
+// Registers and blocks: 128-thread blocks let ptxas have 56 registers at 9 blocks an SM
+// for one-word kinds (512 positions below 1e8: 108.9 ms; 110.7 ms at 46 registers and 40
+// warps in blocks of 256, 125.8 ms at 11 blocks) and 72 at 7 for the float-quotient
+// kinds (1e10: 541.4 ms; 543.6 at 8, 547 at 9, 569 at 10 with spills). Three and four
+// ladders a lane, with 80 and 96 registers, ran those at 548 and 595 ms, one at 613 ms.
 template <int LEVEL, bool FIXED>
-__global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 3 : 5) terms192_kernel(const Seg *__restrict__ segs, int nseg,
+__global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 7 : 9) terms192_kernel(const Seg *__restrict__ segs, int nseg,
                                                              uint64_t ntiles, uint32_t tile_k, TileSplit split,
                                                              unsigned long long *counter,
                                                              unsigned long long *slots, uint64_t budget_ns,
@@ -550,7 +565,9 @@ __global__ void terms_each_kernel(uint64_t d, uint32_t den0, uint32_t den1, int 
     uint32_t q[6] = {0, 0, 0, 0, 0, 0};
     if (m != 1) {
         if (k < d) {
-            if (m < kW1MMin) term_digits<1, false, 6>(d, k, m, q);
+            if (m < kW1L3Min) term_digits<1, false, 6>(d, k, m, q);
+            else if (m < kW1L4Min) term_digits<9, false, 6>(d, k, m, q);
+            else if (m < kW1LMax) term_digits<10, false, 6>(d, k, m, q);
             else if (m < kW1MMax) term_digits<5, false, 6>(d, k, m, q);
             else if (m < kW1SMax) term_digits<3, false, 6>(d, k, m, q);
             else if (m < kW2FLow) term_digits<7, false, 6>(d, k, m, q);
@@ -559,7 +576,9 @@ __global__ void terms_each_kernel(uint64_t d, uint32_t den0, uint32_t den1, int 
             else if (m < kW2Max) term_digits<2, false, 6>(d, k, m, q);
             else term_digits<6, false, 6>(d, k, m, q);
         } else {
-            if (m < kW1MMin) term_digits<1, true, 6>(d, k, m, q);
+            if (m < kW1L3Min) term_digits<1, true, 6>(d, k, m, q);
+            else if (m < kW1L4Min) term_digits<9, true, 6>(d, k, m, q);
+            else if (m < kW1LMax) term_digits<10, true, 6>(d, k, m, q);
             else if (m < kW1MMax) term_digits<5, true, 6>(d, k, m, q);
             else if (m < kW1SMax) term_digits<3, true, 6>(d, k, m, q);
             else if (m < kW2SMax) term_digits<4, true, 6>(d, k, m, q);
@@ -608,7 +627,8 @@ __device__ __forceinline__ DD dd_frac(DD a)
     return (t != 0.0) ? two_sum(a.hi - t, a.lo) : a;
 }
 
-constexpr int kBlockDD = 256;
+constexpr int kBlockDD = 128;
+constexpr int kBlockSsum = 256;
 
 // 128-bit fraction, mod 1 and taken in [-1/2, 1/2), as a double-double.
 __device__ __forceinline__ DD dd_from_fraction(const uint32_t w[4])
@@ -663,7 +683,7 @@ __device__ __forceinline__ void block_sum128(const Acc<4> &acc, uint32_t *half, 
 // sign) stay under the rounding of one double-double addition.
 // Warps take tiles of tile_k terms (a multiple of 64) in turn.
 template <int LEVEL>
-__global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 3 : 5) dd_terms_kernel(uint4 *bigsum, uint64_t k0, uint64_t k1,
+__global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 7 : 9) dd_terms_kernel(uint4 *bigsum, uint64_t k0, uint64_t k1,
                                                                              uint64_t d, int sign, uint32_t den0,
                                                                              uint32_t den1, uint64_t tile_k, int tail)
 {
@@ -735,14 +755,14 @@ cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *blocks, uin
     return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(kBlockDD) dd_ssum_kernel(const uint4 *bigsum, int nblk, double2 *partial)
+__global__ void __launch_bounds__(kBlockSsum) dd_ssum_kernel(const uint4 *bigsum, int nblk, double2 *partial)
 {
     __shared__ uint32_t half[8];
     if (threadIdx.x < 8) half[threadIdx.x] = 0;
     __syncthreads();
     Acc<4> acc;
     acc_zero(acc);
-    for (int i = threadIdx.x; i < nblk; i += kBlockDD) {
+    for (int i = threadIdx.x; i < nblk; i += kBlockSsum) {
         const uint4 v = bigsum[i];
         const uint32_t q[4] = {v.x, v.y, v.z, v.w};
         acc_add(acc, q);
@@ -757,7 +777,7 @@ __global__ void __launch_bounds__(kBlockDD) dd_ssum_kernel(const uint4 *bigsum, 
 
 cudaError_t launch_dd_ssum(const uint4 *bigsum, int nblk, double2 *partial, cudaStream_t st)
 {
-    dd_ssum_kernel<<<1, kBlockDD, 0, st>>>(bigsum, nblk, partial);
+    dd_ssum_kernel<<<1, kBlockSsum, 0, st>>>(bigsum, nblk, partial);
     return cudaGetLastError();
 }
 

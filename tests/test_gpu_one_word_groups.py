@@ -1,6 +1,7 @@
 """The one-word residue kinds in warp groups of 64 terms: range sums bit-exact
-against the oracle around m = 2^25 (width 1 -> middle steps), 2^28, 2^31 and 2^32, at
-group and tile remainders, where a group's exponents cross a multiple of 2^14, at the
+against the oracle around m = 2^17 and 2^25 (starts of three and four exponent bits),
+2^28, 2^29 (lazy -> middle steps), 2^31 and 2^32, at
+group and tile remainders, where a group's exponents cross a multiple of 2^16, at the
 end of the main body, and under exponents of 46 bits and more."""
 import random
 
@@ -22,7 +23,7 @@ def first_k(oracle, f, m):
     return (m - oracle.DEN1[f] + oracle.DEN0[f] - 1) // oracle.DEN0[f]
 
 
-@pytest.mark.parametrize("limit", [25, 28, 31, 32])
+@pytest.mark.parametrize("limit", [17, 25, 28, 29, 31, 32])
 @pytest.mark.parametrize("f", [0, 4])
 def test_range_sums_at_the_limits(ctx192, oracle, f, limit):
     rng = random.Random(limit)
@@ -32,12 +33,12 @@ def test_range_sums_at_the_limits(ctx192, oracle, f, limit):
             check(ctx192, oracle, f, d, k - n // 2, k - n // 2 + n)
 
 
-@pytest.mark.parametrize("limit", [24, 27, 30, 31.6])
+@pytest.mark.parametrize("limit", [16.5, 24, 27, 28.9, 30, 31.6])
 def test_groups_across_a_prefix_boundary(ctx192, oracle, limit):
     for f in (1, 5):
         k = first_k(oracle, f, int(2 ** limit))
         d = k + 123456789
-        while (10 * (d - k) + 160) % (1 << 14) > 640:
+        while (10 * (d - k) + 160) % (1 << 16) > 640:
             k += 1
         for shift in range(0, 64, 9):
             check(ctx192, oracle, f, d, k - shift, k - shift + 3500)
