@@ -21,8 +21,8 @@
 //   strict width 1 (2^31 <= m < 2^32): R = 2^32, signed residues.
 //   float-quotient width 2 (2^32 <= m < 94 * 2^32): R = 2^24, residues below 8m,
 //     the top of each square taken off by a float quotient.
-//   short width 2 (94 * 2^32 <= m < 2^44): R = 2^48, residues in [0, 4m).
-//   width 2 (2^28 <= m < 2^60): R = 2^64 by two word steps, residues in [0, 4m).
+//   short width 2 (94 * 2^32 <= m < 39 * 2^40): R = 2^50, residues in [0, 4m).
+//   width 2 (39 * 2^40 <= m < 2^60): R = 2^64 by two word steps, residues in [0, 4m).
 //   wide width 2 (2^60 <= m < 2^62): the same steps with residues in [0, 2m).
 // The ladder step is y <- REDC(y^2) << b with b the next exponent bit; in the
 // lazy kinds 16m < R keeps the result below 4m with no conditional subtraction.
@@ -83,17 +83,24 @@ __device__ __forceinline__ uint32_t w1_start(uint32_t m)
     return (uint32_t)(r1 + (1 - q2) * (int32_t)m);
 }
 
-// Width 2 (2^28 <= m < 2^62): a value in (0, 2m) congruent to 2^65.
-__device__ __forceinline__ uint64_t w2_start(uint64_t m)
+// Width 2: a value in (0, 2m) congruent to 2^(R + p), 1 <= p <= 15, for R = 50 (2^32 <= m
+// < 2^46) or R = 64 (2^44 <= m < 2^62). The first quotient leaves |r1| <= 2^(R+p-22) + m,
+// so r1 / m is below 2^13 and its rounded estimate off by a few thousandths.
+// (R = 50 checked in float32 emulation over 4e5 moduli, every p, with reciprocals off by up
+// to 2 ulps.)
+template <int R>
+__device__ __forceinline__ uint64_t w2_start(uint64_t m, uint32_t p)
 {
     const uint32_t m0 = (uint32_t)m, m1 = (uint32_t)(m >> 32);
     const float fm = __fmaf_rn(__uint2float_rn(m1), 4294967296.0f, __uint2float_rn(m0));
     const float inv = rcp_approx(fm);
-    const uint64_t q1 = float_to_u64_trunc(36893488147419103232.0f * inv);   // 2^65 / m >= 2^5
-    const int64_t r1 = (int64_t)(0ull - q1 * m);                               // |r1| <= 2^44 + m < 2^61
+    const float scale = __int_as_float((int)((127u + R + p) << 23));            // 2^(R+p)
+    const uint64_t q1 = float_to_u64_trunc(scale * inv);
+    const uint64_t top = R + p < 64 ? 1ull << ((R + p) & 63) : 0ull;           // mod 2^64
+    const int64_t r1 = (int64_t)(top - q1 * m);
     const float fr1 = __fmaf_rn(__int2float_rn((int32_t)(r1 >> 32)), 4294967296.0f,
                                 __uint2float_rn((uint32_t)r1));
-    const int32_t q2 = __float2int_rn(fr1 * inv);                             // |r1/m| <= 2^16 + 1
+    const int32_t q2 = __float2int_rn(fr1 * inv);
     return (uint64_t)(r1 + (int64_t)(1 - q2) * (int64_t)m);
 }
 
@@ -402,30 +409,51 @@ struct W2State {
     __device__ __forceinline__ void step(uint32_t b) { w2_sqr(y0, y1, m0, m1, mp, b); }
 };
 
-// r6 = 2^E mod m in [0, m) for E >= 65 (2^28 <= m < 2^60).
-__device__ __forceinline__ uint64_t w2_pow2(uint64_t E, uint64_t m, uint32_t mp)
+__device__ __forceinline__ uint64_t two_words(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
+
+// Start of a two-word ladder from the leading bits of its exponent.
+template <int R>
+struct W2Start {
+    template <typename State>
+    __device__ __forceinline__ void operator()(State &st, uint32_t p) const
+    {
+        const uint64_t y = w2_start<R>(two_words(st.m0, st.m1), p);
+        st.y0 = (uint32_t)y;
+        st.y1 = (uint32_t)(y >> 32);
+    }
+};
+
+// Residue in [0, m) of a lazy state in [0, 4m).
+template <typename State>
+__device__ __forceinline__ uint64_t lazy_residue(const State &st)
 {
-    const uint64_t y = w2_start(m);
-    W2State st{(uint32_t)y, (uint32_t)(y >> 32), (uint32_t)m, (uint32_t)(m >> 32), mp};
-    walk_bits(E - 64, st);
-    uint64_t r = ((uint64_t)st.y1 << 32) | st.y0;
+    const uint64_t m = two_words(st.m0, st.m1);
+    uint64_t r = two_words(st.y0, st.y1);
     r = min(r, r - 2 * m);
-    r = min(r, r - m);
-    return r;
+    return min(r, r - m);
 }
 
-// --------------------------------------------------- width 2, m < 2^44 --
-// 2^32 <= m < 2^44 (m1 < 2^12), y in [0,4m) (y1 < 2^14), R = 2^48: one 32-bit
-// REDC word step and one 16-bit step. R > 16m^2/(3m) keeps the lazy residues
-// in [0, 4m): REDC(y^2) < 16m^2/2^48 + m < 2m. y^2 = y0^2 + y0 (2 y1) 2^32 +
-// y1^2 2^64 with y0 (2 y1) < 2^47 and y1^2 < 2^28, so word step 1 is
-//   s = (y0^2 + u0 m0) / 2^32 + y1^2 2^32 + y0 (2 y1) + u0 m1 < 2^61,
+// r6 = 2^E mod m in [0, m) for E >= 65 (2^44 <= m < 2^60), the leading up-to-four
+// bits of E - 64 at once.
+__device__ __forceinline__ uint64_t w2_pow2(uint64_t E, uint64_t m, uint32_t mp)
+{
+    W2State st{0, 0, (uint32_t)m, (uint32_t)(m >> 32), mp};
+    walk_bits_start<4>(E - 64, st, W2Start<64>{});
+    return lazy_residue(st);
+}
+
+// -------------------------------------------- width 2, m < 39 * 2^40 --
+// 2^32 <= m < 39 * 2^40 (m1 < 2^13.3), y in [0,4m) (y1 < 2^15.3), R = 2^50: one 32-bit
+// REDC word step and one 18-bit step. y^2 = y0^2 + y0 (2 y1) 2^32 + y1^2 2^64 with
+// y1^2 < 2^31, so word step 1 is
+//   s = (y0^2 + u0 m0) / 2^32 + y1^2 2^32 + y0 (2 y1) + u0 m1 < 2^62.6,
 // one carry chain whose carry out of the first multiply-add lands on y1^2
-// (its high words stay below 2^29 and 2^30: no carry leaves the chain).
-// The 16-bit step takes u1 = s0 mp mod 2^16, so u1 m1 < 2^28 is a single low
-// multiply (a 32-bit step needs two words there): X = s + u1 m0 + u1 m1 2^32
-// < 2^62 with its low 16 bits zero, and X / 2^16 < 2m. The doubling joins
-// that shift: y = X >> (16 - b). 14 multiply halves per step instead of 15.
+// (no carry leaves the chain). The 18-bit step takes u1 = s0 mp mod 2^18, so
+// u1 m1 < 2^32 is a single low multiply (a 32-bit step needs two words there):
+// X = s + u1 m0 + u1 m1 2^32 < 16 m^2 / 2^32 + 2^18 m < 2^64 for m < 39 * 2^40, its low 18
+// bits zero, and X / 2^18 < 16 m^2 / 2^50 + m < 1.7m. The doubling joins that
+// shift: y = X >> (18 - b). 14 multiply halves per step instead of 16. (With a 16-bit
+// step the same code reached 2^44; moduli from there on took the general step.)
 __device__ __forceinline__ void w2s_sqr(uint32_t &y0, uint32_t &y1, uint32_t m0, uint32_t m1, uint32_t mp,
                                         uint32_t b)
 {
@@ -445,14 +473,14 @@ __device__ __forceinline__ void w2s_sqr(uint32_t &y0, uint32_t &y1, uint32_t m0,
         "madc.hi.u32 %1, %2, %9, t1;\n\t}"
         : "=r"(s0), "=r"(s1)
         : "r"(u0), "r"(m0), "r"(a0), "r"(a1), "r"(ysq), "r"(y0), "r"(y2), "r"(m1));
-    const uint32_t u1 = (s0 * mp) & 0xffffu;
+    const uint32_t u1 = (s0 * mp) & 0x3ffffu;
     uint32_t x0, x1;
-    asm("mad.lo.cc.u32 %0, %2, %3, %4;\n\t"     // u1 m0 + s: low 16 bits 0
+    asm("mad.lo.cc.u32 %0, %2, %3, %4;\n\t"     // u1 m0 + s: low 18 bits 0
         "madc.hi.u32 %1, %2, %3, %5;\n\t"
         "mad.lo.u32 %1, %2, %6, %1;"              // + u1 m1 2^32
         : "=&r"(x0), "=&r"(x1)
         : "r"(u1), "r"(m0), "r"(s0), "r"(s1), "r"(m1));
-    const uint32_t sh = 16u - b;
+    const uint32_t sh = 18u - b;
     y0 = __funnelshift_r(x0, x1, sh);
     y1 = x1 >> sh;
 }
@@ -462,63 +490,13 @@ struct W2SState {
     __device__ __forceinline__ void step(uint32_t b) { w2s_sqr(y0, y1, m0, m1, mp, b); }
 };
 
-// A value in (0, 2m) congruent to 2^(48 + p), 1 <= p <= 15, for 2^32 <= m < 2^44:
-// q1 = trunc(2^(48+p) / m) from a float reciprocal (q1 < 2^31) leaves
-// |r1| <= 2^(27+p) + m; q2 = rint(r1 / m) (|r1 / m| < 2^11) is then off by at
-// most a few thousandths, so r1 - q2 m lies in (-m/2, m/2) up to that slack and
-// r1 + (1 - q2) m in (0, 2m). (Checked in float32 emulation over 4e5 moduli,
-// every p, with reciprocals off by up to 2 ulps.)
-__device__ __forceinline__ uint64_t w2s_start(uint64_t m, uint32_t p)
-{
-    const uint32_t m0 = (uint32_t)m, m1 = (uint32_t)(m >> 32);
-    const float fm = __fmaf_rn(__uint2float_rn(m1), 4294967296.0f, __uint2float_rn(m0));
-    const float inv = rcp_approx(fm);
-    const float scale = __int_as_float((int)((127u + 48u + p) << 23));      // 2^(48+p)
-    const uint64_t q1 = float_to_u64_trunc(scale * inv);
-    const int64_t r1 = (int64_t)((1ull << (48 + p)) - q1 * m);
-    const float fr1 = __fmaf_rn(__int2float_rn((int32_t)(r1 >> 32)), 4294967296.0f,
-                                __uint2float_rn((uint32_t)r1));
-    const int32_t q2 = __float2int_rn(fr1 * inv);
-    return (uint64_t)(r1 + (int64_t)(1 - q2) * (int64_t)m);
-}
-
-// r6 = 2^E mod m in [0, m) for E >= 65, 2^32 <= m < 2^44. The ladder runs in
-// Montgomery form with R = 2^48 on the bits of E - 48; the start value takes
-// their leading up-to-four bits at once.
+// r6 = 2^E mod m in [0, m) for E >= 65, 2^32 <= m < 39 * 2^40: the ladder runs in
+// Montgomery form with R = 2^50 on the bits of E - 50, the leading up-to-four at once.
 __device__ __forceinline__ uint64_t w2s_pow2(uint64_t E, uint64_t m, uint32_t mp)
 {
-    const uint64_t Ep = E - 48;
-    const uint32_t hi = (uint32_t)(Ep >> 32), lo = (uint32_t)Ep;
     W2SState st{0, 0, (uint32_t)m, (uint32_t)(m >> 32), mp};
-    if (hi != 0) {
-        const int nb = 32 - __clz(hi);
-        const int t = nb < 4 ? nb : 4;
-        const uint64_t y = w2s_start(m, hi >> (nb - t));
-        st.y0 = (uint32_t)y;
-        st.y1 = (uint32_t)(y >> 32);
-        uint32_t h = (nb - t) > 0 ? hi << (32 - (nb - t)) : 0u;   // remaining bits of hi, left-aligned
-        for (int i = t; i < nb; ++i) {
-            st.step(h >> 31);
-            h <<= 1;
-        }
-#pragma unroll
-        for (int i = 31; i >= 0; --i) st.step((lo >> i) & 1u);
-    } else {
-        const int nb = 32 - __clz(lo);
-        const int t = nb < 4 ? nb : 4;
-        const uint64_t y = w2s_start(m, lo >> (nb - t));
-        st.y0 = (uint32_t)y;
-        st.y1 = (uint32_t)(y >> 32);
-        uint32_t l = (nb - t) > 0 ? lo << (32 - (nb - t)) : 0u;
-        for (int i = t; i < nb; ++i) {
-            st.step(l >> 31);
-            l <<= 1;
-        }
-    }
-    uint64_t r = ((uint64_t)st.y1 << 32) | st.y0;
-    r = min(r, r - 2 * m);
-    r = min(r, r - m);
-    return r;
+    walk_bits_start<4>(E - 50, st, W2Start<50>{});
+    return lazy_residue(st);
 }
 
 // ------------------------------------------------ width 2, m < 94 * 2^32 --
@@ -678,15 +656,18 @@ struct W2XState {
     }
 };
 
-// r6 = 2^E mod m in [0, m) for E >= 65, 2^28 <= m < 2^62.
+__device__ __forceinline__ W2XState w2x_state(uint64_t m, uint32_t mp)
+{
+    return W2XState{0, 0, (uint32_t)m, (uint32_t)(m >> 32), mp, 2 * m};
+}
+
+// r6 = 2^E mod m in [0, m) for E >= 65, 2^44 <= m < 2^62.
 __device__ __forceinline__ uint64_t w2x_pow2(uint64_t E, uint64_t m, uint32_t mp)
 {
-    const uint64_t y = w2_start(m);                     // (0, 2m)
-    W2XState st{(uint32_t)y, (uint32_t)(y >> 32), (uint32_t)m, (uint32_t)(m >> 32), mp, 2 * m};
-    walk_bits(E - 64, st);
-    uint64_t r = ((uint64_t)st.y1 << 32) | st.y0;
-    r = min(r, r - m);
-    return r;
+    W2XState st = w2x_state(m, mp);
+    walk_bits_start<4>(E - 64, st, W2Start<64>{});
+    const uint64_t r = two_words(st.y0, st.y1);         // below 2m
+    return min(r, r - m);
 }
 
 // N REDC steps down from r < m (two-word m): q[j] are the quotient digits and
@@ -781,15 +762,6 @@ __device__ __forceinline__ void walk_bits_group(uint64_t EpA, uint64_t EpB, uint
 
 struct W1Start1 {                                        // the single-bit start of the width-1 kind
     __device__ __forceinline__ void operator()(W1State &st, uint32_t) const { st.y = w1_start(st.m); }
-};
-
-struct W2SStart {
-    __device__ __forceinline__ void operator()(W2SState &st, uint32_t p) const
-    {
-        const uint64_t y = w2s_start(((uint64_t)st.m1 << 32) | st.m0, p);
-        st.y0 = (uint32_t)y;
-        st.y1 = (uint32_t)(y >> 32);
-    }
 };
 
 // ------------------------------------------------------------ fixed point --

@@ -34,6 +34,7 @@ constexpr uint64_t kW2FLow = 15ull << 34; // float-quotient steps without an off
 constexpr uint64_t kW2FMax = 94ull << 32; // float-quotient steps for 2^32 <= m < 94 * 2^32, inside short width 2
 constexpr uint64_t kW2FExp = 1ull << 48;  // ... in tiles whose exponents are below 2^48 (the short kind's steps above)
 constexpr uint64_t kW2SMax = 1ull << 44;  // short width 2 for 2^32 <= m < 2^44
+constexpr uint64_t kW2SWide = 39ull << 40; // the short kind's steps also serve width-2 tiles up to here
 constexpr uint64_t kW2Max = 1ull << 60;   // width 2 (two words, residues < 4m) for m < 2^60
 constexpr uint64_t kW2XMax = 1ull << 62;  // wide width 2 (residues < 2m) for 2^60 <= m < 2^62
 

@@ -52,9 +52,9 @@ __device__ __forceinline__ void shr_digits(uint32_t q[N], int s)
 // tail value 2^(-10(k-d))/m (digits of 1/m shifted right by 10(k-d)).
 // KIND: 1 = width 1 (m < 2^28), 9 and 10 = lazy width 1 with a start of three (2^17 <= m
 // < 2^29) and four bits (2^25 <= m < 2^29), 5 = middle width 1 (2^25 <= m < 2^31),
-// 3 = strict width 1 (2^28 <= m < 2^32), 7 and 8 = float-quotient width 2 (2^32 <= m
-// < 15 * 2^34 and < 94 * 2^32), 4 = short width 2 (2^32 <= m < 2^44),
-// 2 = width 2 (2^28 <= m < 2^60), 6 = wide width 2 (2^60 <= m < 2^62).
+// 3 = strict width 1 (2^31 <= m < 2^32), 7 and 8 = float-quotient width 2 (2^32 <= m
+// < 15 * 2^34 and < 94 * 2^32), 4 = short width 2 (2^32 <= m < 39 * 2^40),
+// 2 = width 2 (2^44 <= m < 2^60), 6 = wide width 2 (2^60 <= m < 2^62).
 template <int KIND, bool TAIL, int N>
 __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, uint32_t q[N])
 {
@@ -88,13 +88,11 @@ __device__ __forceinline__ void term_digits(uint64_t d, uint64_t k, uint64_t m, 
     if (TAIL) shr_digits<N>(q, (int)(10 * (k - d)));
 }
 
-// Two terms (exponents Ea and Ea - 320) of a lane per iteration, their ladders interleaved
-// (kinds 1, 3, 4, 5, 7, 8; the width-2 kinds above 2^44 run one term at a time).
-// e_max is the largest exponent of the warp's 64.
-// Same-box timings against one term per iteration, identical bits: 1e9
-// 40.65 -> 38.55 ms, 1e10 841.0 -> 838.9 ms, batch 10.61 -> 10.08 s. Pairing
-// only some kinds traded these against each other (the kernel's code layout
-// and registers change with every instantiation), so all four are paired.
+// Two terms (exponents Ea and Ea - 320) of a lane per iteration, their ladders in
+// turn. e_max is the largest exponent of the warp's 64. One ladder a lane measured
+// 40.7 against 46.9e9 terms/s (float-quotient kinds), 21.6 against 23.1e9 (width 2 at
+// 1e14), 12.1 against 13.0e9 (wide width 2 at 9e17); three and four lose again
+// (terms192_kernel).
 template <int KIND, int N>
 __device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t ma, uint64_t mb, uint32_t qa[N],
                                           uint32_t qb[N])
@@ -109,14 +107,20 @@ __device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t 
         w2_redc_down<N>(rb, mb, mpb, qb);
     } else if (KIND == 4) {
         W2SState A{0, 0, (uint32_t)ma, (uint32_t)(ma >> 32), mpa}, B{0, 0, (uint32_t)mb, (uint32_t)(mb >> 32), mpb};
-        walk_bits_start_pair<4>(Ea - 48, Eb - 48, A, B, W2SStart{});   // R = 2^48
-        uint64_t ra = ((uint64_t)A.y1 << 32) | A.y0, rb = ((uint64_t)B.y1 << 32) | B.y0;
-        ra = min(ra, ra - 2 * ma);
-        ra = min(ra, ra - ma);
-        rb = min(rb, rb - 2 * mb);
-        rb = min(rb, rb - mb);
-        w2_redc_down<N>(ra, ma, mpa, qa);
-        w2_redc_down<N>(rb, mb, mpb, qb);
+        walk_bits_group<4>(Ea - 50, Eb - 50, e_max - 50, A, B, W2Start<50>{});     // R = 2^50
+        w2_redc_down<N>(lazy_residue(A), ma, mpa, qa);
+        w2_redc_down<N>(lazy_residue(B), mb, mpb, qb);
+    } else if (KIND == 2) {
+        W2State A{0, 0, (uint32_t)ma, (uint32_t)(ma >> 32), mpa}, B{0, 0, (uint32_t)mb, (uint32_t)(mb >> 32), mpb};
+        walk_bits_group<4>(Ea - 64, Eb - 64, e_max - 64, A, B, W2Start<64>{});
+        w2_redc_down<N>(lazy_residue(A), ma, mpa, qa);
+        w2_redc_down<N>(lazy_residue(B), mb, mpb, qb);
+    } else if (KIND == 6) {
+        W2XState A = w2x_state(ma, mpa), B = w2x_state(mb, mpb);
+        walk_bits_group<4>(Ea - 64, Eb - 64, e_max - 64, A, B, W2Start<64>{});
+        const uint64_t ra = two_words(A.y0, A.y1), rb = two_words(B.y0, B.y1);     // below 2m
+        w2_redc_down<N>(min(ra, ra - ma), ma, mpa, qa);
+        w2_redc_down<N>(min(rb, rb - mb), mb, mpb, qb);
     } else if (KIND == 1) {
         W1State A{0, (uint32_t)ma, mpa}, B{0, (uint32_t)mb, mpb};
         walk_bits_group<1>(Ea - 32, Eb - 32, e_max - 32, A, B, W1Start1{});
@@ -150,8 +154,8 @@ __device__ __forceinline__ void run_tile(const Seg &s, uint64_t kb, uint64_t ke,
                                          uint32_t &cnt)
 {
     uint64_t k = kb + lane;
-    if (!TAIL && KIND != 2 && KIND != 6) {
-        constexpr bool wide = KIND == 4 || KIND == 7 || KIND == 8;
+    if (!TAIL) {
+        constexpr bool wide = KIND == 2 || KIND == 4 || KIND == 6 || KIND == 7 || KIND == 8;
         uint64_t ea = 10ull * (s.d - k) + 32ull * N, ma = (uint64_t)s.den0 * k + s.den1;
         uint64_t e_max = ea + 10u * lane;
         const uint64_t m32 = 32ull * s.den0;
@@ -301,7 +305,9 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
         if (fq && m_last < kW2FLow) run_tile<7, TAIL>(s, kb, ke, lane, acc, cnt);
         else if (fq && m_last < kW2FMax) run_tile<8, TAIL>(s, kb, ke, lane, acc, cnt);
         else run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
-    } else if (LEVEL >= 2 && width == 2) run_tile<2, TAIL>(s, kb, ke, lane, acc, cnt);
+    } else if (LEVEL >= 2 && width == 2 && (uint64_t)s.den0 * (ke - 1) + s.den1 < kW2SWide)
+        run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (LEVEL >= 2 && width == 2) run_tile<2, TAIL>(s, kb, ke, lane, acc, cnt);
     else if (LEVEL >= 2 && width == 6) run_tile<6, TAIL>(s, kb, ke, lane, acc, cnt);
     else if (width == 3) run_tile<3, TAIL>(s, kb, ke, lane, acc, cnt);
     else {
@@ -572,7 +578,7 @@ __global__ void terms_each_kernel(uint64_t d, uint32_t den0, uint32_t den1, int 
             else if (m < kW1SMax) term_digits<3, false, 6>(d, k, m, q);
             else if (m < kW2FLow) term_digits<7, false, 6>(d, k, m, q);
             else if (m < kW2FMax) term_digits<8, false, 6>(d, k, m, q);
-            else if (m < kW2SMax) term_digits<4, false, 6>(d, k, m, q);
+            else if (m < kW2SWide) term_digits<4, false, 6>(d, k, m, q);
             else if (m < kW2Max) term_digits<2, false, 6>(d, k, m, q);
             else term_digits<6, false, 6>(d, k, m, q);
         } else {
@@ -581,7 +587,7 @@ __global__ void terms_each_kernel(uint64_t d, uint32_t den0, uint32_t den1, int 
             else if (m < kW1LMax) term_digits<10, true, 6>(d, k, m, q);
             else if (m < kW1MMax) term_digits<5, true, 6>(d, k, m, q);
             else if (m < kW1SMax) term_digits<3, true, 6>(d, k, m, q);
-            else if (m < kW2SMax) term_digits<4, true, 6>(d, k, m, q);
+            else if (m < kW2SWide) term_digits<4, true, 6>(d, k, m, q);
             else if (m < kW2Max) term_digits<2, true, 6>(d, k, m, q);
             else term_digits<6, true, 6>(d, k, m, q);
         }
