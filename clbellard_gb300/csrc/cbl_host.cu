@@ -990,18 +990,22 @@ int cbl_run_job(cbl_ctx *c, uint64_t needD, int s, uint64_t b, uint64_t batchsiz
 }
 
 // ---- balanced work-mode planning
-// Relative cost of one ladder step per residue kind, from each kind's measured
-// term time on its own k-range (GB300; 0.6e8-4.6e8 terms per range, divided by
-// bitlen(10(d-k)) + 8 and scaled to W1 = 7): W1 7, W1M 5.9, W1S 8.2, W2S 14.5,
-// W2 16.8, W2X 24.3.
-static double step_cost(uint64_t m)
+// Relative cost of one ladder step per residue kind, from measured term rates on
+// k-ranges of one kind (GB300; rate times bitlen(10(d-k)) + 8): one-word kinds 3.0,
+// 2.7 from 2^25 and 3.9 from 2^31 on, float-quotient 5.0 and 5.4, short width 2 7.3,
+// width 2 8.0, wide width 2 11.5.
+struct StepCost {
+    uint64_t below;
+    double cost;
+};
+static const StepCost kStepCost[8] = {{kW1L4Min, 3.0}, {kW1MMax, 2.7}, {kW1SMax, 3.9}, {kW2FLow, 5.0},
+                                      {kW2FMax, 5.4},  {kW2SWide, 7.3}, {kW2Max, 8.0}, {UINT64_MAX, 11.5}};
+
+static const StepCost &step_cost(uint64_t m)
 {
-    if (m < kW1Max) return 7.0;
-    if (m < kW1MMax) return 5.9;
-    if (m < kW1SMax) return 8.2;
-    if (m < kW2SMax) return 14.5;
-    if (m < kW2Max) return 16.8;
-    return 24.3;
+    int i = 0;
+    while (m >= kStepCost[i].below) ++i;
+    return kStepCost[i];
 }
 
 // Estimated cost of terms k in [k0, k1) of series f at position d (k < d):
@@ -1021,16 +1025,14 @@ static double range_cost(uint64_t d, int f, uint64_t k0, uint64_t k1)
         uint64_t knext = d - (lim - 1) / 10;                 // first k with 10(d-k) < 2^(bl-1)
         if (knext <= k) knext = k + 1;
         const uint64_t m = den0 * k + den1;
-        const uint64_t bounds[5] = {kW1Max, kW1MMax, kW1SMax, kW2SMax, kW2Max};
-        for (uint64_t b : bounds)
-            if (m < b) {
-                const uint64_t kb = (b - den1 + den0 - 1) / den0;
-                if (kb < knext) knext = kb;
-                break;
-            }
+        const StepCost &c = step_cost(m);
+        if (c.below != UINT64_MAX) {
+            const uint64_t kb = (c.below - den1 + den0 - 1) / den0;
+            if (kb < knext) knext = kb;
+        }
         if (knext > k1) knext = k1;
         if (knext <= k) knext = k + 1;
-        total += (double)(knext - k) * (bl + 8) * step_cost(m);
+        total += (double)(knext - k) * (bl + 8) * c.cost;
         k = knext;
     }
     return total;
