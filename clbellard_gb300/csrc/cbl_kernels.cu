@@ -17,6 +17,28 @@ namespace cbl {
 
 constexpr int kBlock192 = 128;
 
+// The one-block kernels behind a term kernel (Ssum, Sum7) are launched as programmatic
+// dependents: they may be scheduled while their predecessor still runs and wait for its
+// end, memory included, in await_predecessor(). allow_dependent() lets that happen from a
+// block's start on. Seven series at 1e7 in mode 0, 14 such launches: 392 -> 362 us.
+__device__ __forceinline__ void await_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_dependent() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+template <typename... Params, typename... Args>
+static cudaError_t launch_dependent(void (*kernel)(Params...), int block, cudaStream_t st, Args... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // numer of series f as a shift (KernelFuncs.as:9): 32,1,256,64,4,4,1
 __device__ __forceinline__ int numer_log2(int f)
 {
@@ -340,6 +362,7 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 7 : 9) terms192_kernel
                                                              int carry)
 {
     const int lane = threadIdx.x & 31;
+    allow_dependent();
     const uint64_t t_start = budget_ns ? global_ns() : 0;
     uint64_t nitems = ntiles, item = 0;
     if (FIXED) {                                    // this block's share, dealt to its warps in turn
@@ -533,6 +556,8 @@ cudaError_t launch_combine(const unsigned long long *slots, int npos, const int 
 
 __global__ void ssum192_kernel(const unsigned long long *slots, uint64_t *partial)
 {
+    allow_dependent();
+    await_predecessor();
     uint64_t w[3];
     normalise6(slots, w);
     partial[0] = w[2]; partial[1] = w[1]; partial[2] = w[0];
@@ -540,12 +565,12 @@ __global__ void ssum192_kernel(const unsigned long long *slots, uint64_t *partia
 
 cudaError_t launch_ssum192(const unsigned long long *slots, uint64_t *partial, cudaStream_t st)
 {
-    ssum192_kernel<<<1, 1, 0, st>>>(slots, partial);
-    return cudaGetLastError();
+    return launch_dependent(ssum192_kernel, 1, st, slots, partial);
 }
 
 __global__ void sum7_192_kernel(uint64_t *partial, uint64_t *ans, int sh)
 {
+    await_predecessor();
     uint64_t w[3] = {partial[2], partial[1], partial[0]};
     shl192(w, sh);
     partial[0] = w[2]; partial[1] = w[1]; partial[2] = w[0];
@@ -556,8 +581,7 @@ __global__ void sum7_192_kernel(uint64_t *partial, uint64_t *ans, int sh)
 
 cudaError_t launch_sum7_192(uint64_t *partial, uint64_t *ans, int numer_log2, cudaStream_t st)
 {
-    sum7_192_kernel<<<1, 1, 0, st>>>(partial, ans, numer_log2);
-    return cudaGetLastError();
+    return launch_dependent(sum7_192_kernel, 1, st, partial, ans, numer_log2);
 }
 
 // ---------------------------------------------------------- per-term kernel --
@@ -696,6 +720,7 @@ __global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 7 : 9) dd_terms_kernel(
     __shared__ uint32_t half[8];
     const int lane = threadIdx.x & 31;
     const uint64_t step = (uint64_t)gridDim.x * (kBlockDD / 32) * tile_k;
+    allow_dependent();
     if (threadIdx.x < 8) half[threadIdx.x] = 0;
     __syncthreads();
     Acc<4> acc;
@@ -764,8 +789,10 @@ cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *blocks, uin
 __global__ void __launch_bounds__(kBlockSsum) dd_ssum_kernel(const uint4 *bigsum, int nblk, double2 *partial)
 {
     __shared__ uint32_t half[8];
+    allow_dependent();
     if (threadIdx.x < 8) half[threadIdx.x] = 0;
     __syncthreads();
+    await_predecessor();
     Acc<4> acc;
     acc_zero(acc);
     for (int i = threadIdx.x; i < nblk; i += kBlockSsum) {
@@ -783,8 +810,7 @@ __global__ void __launch_bounds__(kBlockSsum) dd_ssum_kernel(const uint4 *bigsum
 
 cudaError_t launch_dd_ssum(const uint4 *bigsum, int nblk, double2 *partial, cudaStream_t st)
 {
-    dd_ssum_kernel<<<1, kBlockSsum, 0, st>>>(bigsum, nblk, partial);
-    return cudaGetLastError();
+    return launch_dependent(dd_ssum_kernel, kBlockSsum, st, bigsum, nblk, partial);
 }
 
 __device__ __forceinline__ DD dd_unit(DD a)   // into [0, 1)
@@ -799,6 +825,7 @@ __device__ __forceinline__ DD dd_unit(DD a)   // into [0, 1)
 // add into the answer.
 __global__ void dd_sum7_kernel(double2 *partial, double2 *ans, int numer)
 {
+    await_predecessor();
     DD a = dd_unit(DD{partial->x, partial->y});
     a.hi *= (double)numer;
     a.lo *= (double)numer;
@@ -810,8 +837,7 @@ __global__ void dd_sum7_kernel(double2 *partial, double2 *ans, int numer)
 
 cudaError_t launch_dd_sum7(double2 *partial, double2 *ans, int numer, cudaStream_t st)
 {
-    dd_sum7_kernel<<<1, 1, 0, st>>>(partial, ans, numer);
-    return cudaGetLastError();
+    return launch_dependent(dd_sum7_kernel, 1, st, partial, ans, numer);
 }
 
 }  // namespace cbl
