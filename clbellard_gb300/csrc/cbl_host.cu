@@ -40,6 +40,8 @@ struct cbl_ctx {
     int64_t launches = 0;
     int tile_k = kDefaultTile;
     int ctas_per_sm = 0;
+    TermGrid term_ctas[kTermLevels];          // resident CTAs per SM, 0 = not asked yet
+    int dd_ctas[kTermLevels] = {};
     // 192-bit buffers
     // tile table: the segments, then (prepared passes) one shift per position
     unsigned char *d_table = nullptr;
@@ -246,10 +248,13 @@ uint64_t order_and_number(std::vector<Seg> &v, uint32_t tile_k)
     return t;
 }
 
-int grid_192(const cbl_ctx *c, int level)
+// Resident grids of a level's term kernels (asked of the runtime once a context).
+TermGrid grid_192(cbl_ctx *c, int level)
 {
-    int per = c->ctas_per_sm > 0 ? c->ctas_per_sm : terms192_max_ctas_per_sm(level);
-    return std::max(1, c->sm_count * per);
+    TermGrid &per = c->term_ctas[level];
+    if (per.tiles == 0) per = terms192_ctas_per_sm(level);
+    return TermGrid{std::max(1, c->sm_count * (c->ctas_per_sm > 0 ? c->ctas_per_sm : per.tiles)),
+                    std::max(1, c->sm_count * (c->ctas_per_sm > 0 ? c->ctas_per_sm : per.shares))};
 }
 
 // Term-kernel level of a set of segments.
@@ -291,7 +296,8 @@ int dd_range(cbl_ctx *c, uint64_t k0, uint64_t k1, uint64_t d, int sign, uint32_
         const uint64_t b = std::max(a, std::min(k1, a + chunk));
         const bool last = b >= k1;
         const int level = b > a ? term_level((uint64_t)den0 * a + den1, (uint64_t)den0 * (b - 1) + den1) : 0;
-        const int grid = std::min(kDDBlocks, c->sm_count * dd_terms_max_ctas_per_sm(level));
+        if (c->dd_ctas[level] == 0) c->dd_ctas[level] = dd_terms_max_ctas_per_sm(level);
+        const int grid = std::min(kDDBlocks, c->sm_count * c->dd_ctas[level]);
         int blocks = 0;
         CK(launch_dd_terms(level, c->d_bigsum, grid, &blocks, a, b, d, sign, den0, den1, tail && last, c->st));
         c->dd_blocks = std::max(c->dd_blocks, blocks);
@@ -1302,7 +1308,7 @@ int cbl_prepared_info(const cbl_ctx *c, uint64_t *terms, uint64_t *tiles, int *s
     if (terms) *terms = c->prep_terms;
     if (tiles) *tiles = c->prep_ntiles;
     if (segments) *segments = c->prep_nseg;
-    if (grid) *grid = grid_192(c, c->prep_level);
+    if (grid) *grid = grid_192(const_cast<cbl_ctx *>(c), c->prep_level).tiles;
     return CBL_OK;
     CBL_GUARD_END
 }
@@ -1370,7 +1376,7 @@ int cbl_autotune(cbl_ctx *c, const uint64_t *pos, int n, int force, int *best_ti
             if (rc) return rc;
             d_max = std::max(d_max, d);
         }
-        const int occ = terms192_max_ctas_per_sm(term_level(0, 10 * (d_max + kTail192) + 9));
+        const int occ = terms192_ctas_per_sm(term_level(0, 10 * (d_max + kTail192) + 9)).tiles;
         const int tiles[] = {512, 1024, 2048, 4096, 8192};
         ms_best = 1e300;
         for (int t : tiles) {

@@ -58,21 +58,28 @@ constexpr uint32_t kFlagSign = 1u;
 inline uint32_t seg_flags(int sign, int width) { return (uint32_t)(sign & 1) | ((uint32_t)width << 4); }
 
 // Instantiation of the term kernel for a table whose moduli lie in [min_m, max_m]:
-// 0 one-word kinds only (m < 2^32), 1 also the float-quotient and short two-word
-// kinds (m < 2^44), 2 any kind but without the float-quotient steps (moduli below
-// 94 * 2^32 take the short kind's there). Short two-word terms run 2 % faster at
-// level 2 (48 registers, 5 CTAs an SM) than beside the float-quotient steps at level 1,
-// so a table without moduli for those takes level 2.
-constexpr int kTermLevels = 3;
+// 0 the width-1 and lazy kinds only (m < 2^29), 1 all one-word kinds (m < 2^32), 2 also
+// the float-quotient and short two-word kinds (m < 2^44), 3 any kind but without the
+// float-quotient steps (moduli below 94 * 2^32 take the short kind's there). A kernel's
+// registers and code follow its widest kind: one-word terms ran 5 % slower beside the
+// float-quotient steps, and short two-word terms are 2 % faster at level 3 than
+// beside the float-quotient steps, so a table without moduli for those takes level 3.
+constexpr int kTermLevels = 4;
 __host__ __device__ inline int term_level(uint64_t min_m, uint64_t max_m)
 {
-    return max_m < kW1SMax ? 0 : max_m < kW2SMax && min_m < kW2FMax ? 1 : 2;
+    return max_m < kW1LMax ? 0 : max_m < kW1SMax ? 1 : max_m < kW2SMax && min_m < kW2FMax ? 2 : 3;
 }
 
 // How a pass without a time budget deals its tiles out: from the tile counter, or
 // (fixed) as 2^log2_parts parts of part_k terms each, one contiguous share a block.
 struct TileSplit {
     uint32_t log2_parts, fixed, part_k;
+};
+
+// Resident blocks (of one SM, or of a grid) of the term kernel's two forms.
+struct TermGrid {
+    int tiles = 0;         // tiles from the counter
+    int shares = 0;        // fixed shares
 };
 
 // Launch wrappers (cbl_kernels.cu).
@@ -85,8 +92,8 @@ struct TileSplit {
 // A slot receives at most one flush per tile, so slot_needs_carry() decides it
 // from the tile counts.
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
-                            unsigned long long *counter, unsigned long long *slots, int grid, cudaStream_t st,
-                            uint64_t budget_ns, bool carry, bool reset_counter);
+                            unsigned long long *counter, unsigned long long *slots, const TermGrid &grids,
+                            cudaStream_t st, uint64_t budget_ns, bool carry, bool reset_counter);
 constexpr uint64_t kCarryTiles = 1ull << 31;
 inline bool slot_needs_carry(uint64_t max_tiles_per_slot) { return max_tiles_per_slot >= kCarryTiles; }
 // slots (nslot x 6 digit sums) of position i, series f = slots[(7 i + f) * 6 ..]:
@@ -122,6 +129,6 @@ cudaError_t launch_probe_imad(uint32_t *sink, int grid, int block, int iters, ui
 int probe_imad_grid(int sm_count);   // one full wave of probe CTAs
 
 int device_sm_count(int device);
-int terms192_max_ctas_per_sm(int level);
+TermGrid terms192_ctas_per_sm(int level);
 
 }  // namespace cbl

@@ -166,8 +166,8 @@ __device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t 
     } else {
         W1SState A{0, (uint32_t)ma, 0u - mpa}, B{0, (uint32_t)mb, 0u - mpb};
         walk_bits_group<4>(Ea - 32, Eb - 32, e_max - 32, A, B, W1SStart{});
-        w1_digits<N>(A.residue(), (uint32_t)ma, mpa, qa);
-        w1_digits<N>(B.residue(), (uint32_t)mb, mpb, qb);
+        w1_digits<N>(A.y, (uint32_t)ma, mpa, qa);
+        w1_digits<N>(B.y, (uint32_t)mb, mpb, qb);
     }
 }
 
@@ -319,26 +319,21 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
                                               uint32_t &cnt)
 {
     const int width = (int)((s.flags >> 4) & 15u);
+    const uint64_t m_first = (uint64_t)s.den0 * kb + s.den1, m_last = (uint64_t)s.den0 * (ke - 1) + s.den1;
     if (LEVEL == 2 && width == 4) {
-        run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
-    } else if (LEVEL == 1 && width == 4) {
-        const uint64_t m_last = (uint64_t)s.den0 * (ke - 1) + s.den1;
         const bool fq = TAIL || 10 * (s.d - kb) + 32 * N < kW2FExp;
         if (fq && m_last < kW2FLow) run_tile<7, TAIL>(s, kb, ke, lane, acc, cnt);
         else if (fq && m_last < kW2FMax) run_tile<8, TAIL>(s, kb, ke, lane, acc, cnt);
         else run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
-    } else if (LEVEL >= 2 && width == 2 && (uint64_t)s.den0 * (ke - 1) + s.den1 < kW2SWide)
+    } else if (LEVEL == 3 && (width == 4 || (width == 2 && m_last < kW2SWide))) {
         run_tile<4, TAIL>(s, kb, ke, lane, acc, cnt);
-    else if (LEVEL >= 2 && width == 2) run_tile<2, TAIL>(s, kb, ke, lane, acc, cnt);
-    else if (LEVEL >= 2 && width == 6) run_tile<6, TAIL>(s, kb, ke, lane, acc, cnt);
-    else if (width == 3) run_tile<3, TAIL>(s, kb, ke, lane, acc, cnt);
-    else {
-        const uint64_t m_first = (uint64_t)s.den0 * kb + s.den1, m_last = (uint64_t)s.den0 * (ke - 1) + s.den1;
-        if (m_last >= kW1LMax) run_tile<5, TAIL>(s, kb, ke, lane, acc, cnt);
-        else if (m_first >= kW1L4Min) run_tile<10, TAIL>(s, kb, ke, lane, acc, cnt);
-        else if (m_first >= kW1L3Min) run_tile<9, TAIL>(s, kb, ke, lane, acc, cnt);
-        else run_tile<1, TAIL>(s, kb, ke, lane, acc, cnt);
-    }
+    } else if (LEVEL == 3 && width == 2) run_tile<2, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (LEVEL == 3 && width == 6) run_tile<6, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (LEVEL >= 1 && width == 3) run_tile<3, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (LEVEL >= 1 && m_last >= kW1LMax) run_tile<5, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (m_first >= kW1L4Min) run_tile<10, TAIL>(s, kb, ke, lane, acc, cnt);
+    else if (m_first >= kW1L3Min) run_tile<9, TAIL>(s, kb, ke, lane, acc, cnt);
+    else run_tile<1, TAIL>(s, kb, ke, lane, acc, cnt);
 }
 
 // With budget_ns != 0 a warp takes no new tile once budget_ns have passed
@@ -355,7 +350,7 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
 // kinds (1e10: 541.4 ms; 543.6 at 8, 547 at 9, 569 at 10 with spills). Three and four
 // ladders a lane, with 80 and 96 registers, ran those at 548 and 595 ms, one at 613 ms.
 template <int LEVEL, bool FIXED>
-__global__ void __launch_bounds__(kBlock192, LEVEL == 1 ? 7 : 9) terms192_kernel(const Seg *__restrict__ segs, int nseg,
+__global__ void __launch_bounds__(kBlock192, LEVEL == 2 ? 7 : 9) terms192_kernel(const Seg *__restrict__ segs, int nseg,
                                                              uint64_t ntiles, uint32_t tile_k, TileSplit split,
                                                              unsigned long long *counter,
                                                              unsigned long long *slots, uint64_t budget_ns,
@@ -417,7 +412,9 @@ typedef void (*Terms192Fn)(const Seg *, int, uint64_t, uint32_t, TileSplit, unsi
 template <bool FIXED>
 static Terms192Fn terms192_fn(int level)
 {
-    return level == 0 ? terms192_kernel<0, FIXED> : level == 1 ? terms192_kernel<1, FIXED> : terms192_kernel<2, FIXED>;
+    static const Terms192Fn fn[kTermLevels] = {terms192_kernel<0, FIXED>, terms192_kernel<1, FIXED>,
+                                               terms192_kernel<2, FIXED>, terms192_kernel<3, FIXED>};
+    return fn[level];
 }
 
 // A pass with fewer tiles than resident warps leaves most of the GPU idle and its
@@ -442,12 +439,12 @@ TileSplit tile_split(uint64_t ntiles, uint32_t tile_k, int grid)
 }
 
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
-                            unsigned long long *counter, unsigned long long *slots, int grid, cudaStream_t st,
-                            uint64_t budget_ns, bool carry, bool reset_counter)
+                            unsigned long long *counter, unsigned long long *slots, const TermGrid &grids,
+                            cudaStream_t st, uint64_t budget_ns, bool carry, bool reset_counter)
 {
     // a budgeted pass stops and resumes at whole tiles
-    const TileSplit sp = budget_ns ? TileSplit{0, 0, tile_k} : tile_split(ntiles, tile_k, grid);
-    if (sp.fixed) grid = (int)std::min<uint64_t>(grid, ntiles << sp.log2_parts);
+    const TileSplit sp = budget_ns ? TileSplit{0, 0, tile_k} : tile_split(ntiles, tile_k, grids.tiles);
+    const int grid = sp.fixed ? (int)std::min<uint64_t>(grids.shares, ntiles << sp.log2_parts) : grids.tiles;
     if (reset_counter && !sp.fixed) {
         const cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
         if (e != cudaSuccess) return e;
@@ -457,11 +454,18 @@ cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntile
     return cudaGetLastError();
 }
 
-int terms192_max_ctas_per_sm(int level)
+template <typename Kernel>
+static int max_ctas_per_sm(Kernel fn, int block)
 {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, terms192_fn<false>(level), kBlock192, 0) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, 0) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
+}
+
+TermGrid terms192_ctas_per_sm(int level)
+{
+    return TermGrid{max_ctas_per_sm(terms192_fn<false>(level), kBlock192),
+                    max_ctas_per_sm(terms192_fn<true>(level), kBlock192)};
 }
 
 int device_sm_count(int device)
@@ -713,7 +717,7 @@ __device__ __forceinline__ void block_sum128(const Acc<4> &acc, uint32_t *half, 
 // sign) stay under the rounding of one double-double addition.
 // Warps take tiles of tile_k terms (a multiple of 64) in turn.
 template <int LEVEL>
-__global__ void __launch_bounds__(kBlockDD, LEVEL == 1 ? 7 : 9) dd_terms_kernel(uint4 *bigsum, uint64_t k0, uint64_t k1,
+__global__ void __launch_bounds__(kBlockDD, LEVEL == 2 ? 7 : 9) dd_terms_kernel(uint4 *bigsum, uint64_t k0, uint64_t k1,
                                                                              uint64_t d, int sign, uint32_t den0,
                                                                              uint32_t den1, uint64_t tile_k, int tail)
 {
@@ -765,15 +769,12 @@ typedef void (*DDTermsFn)(uint4 *, uint64_t, uint64_t, uint64_t, int, uint32_t, 
 
 static DDTermsFn dd_terms_fn(int level)
 {
-    return level == 0 ? dd_terms_kernel<0> : level == 1 ? dd_terms_kernel<1> : dd_terms_kernel<2>;
+    static const DDTermsFn fn[kTermLevels] = {dd_terms_kernel<0>, dd_terms_kernel<1>, dd_terms_kernel<2>,
+                                              dd_terms_kernel<3>};
+    return fn[level];
 }
 
-int dd_terms_max_ctas_per_sm(int level)
-{
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dd_terms_fn(level), kBlockDD, 0) != cudaSuccess) return 1;
-    return n > 0 ? n : 1;
-}
+int dd_terms_max_ctas_per_sm(int level) { return max_ctas_per_sm(dd_terms_fn(level), kBlockDD); }
 
 cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *blocks, uint64_t k0, uint64_t k1, uint64_t d,
                             int sign, uint32_t den0, uint32_t den1, bool tail, cudaStream_t st)

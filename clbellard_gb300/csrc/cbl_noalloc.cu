@@ -214,7 +214,7 @@ namespace {
 struct DeviceSetup {
     bool ready = false;
     unsigned char *scratch = nullptr;   // device address of g_noalloc_scratch on this device
-    int grid[kTermLevels] = {0, 0, 0};
+    TermGrid grid[kTermLevels];
 };
 
 constexpr int kMaxDevices = 64;
@@ -237,7 +237,10 @@ int setup_device(int dev, DeviceSetup **out)
         cudaFuncAttributes attr;
         if (cudaFuncGetAttributes(&attr, noalloc_table_kernel) != cudaSuccess) return CBL_E_CUDA;
         s.scratch = static_cast<unsigned char *>(p);
-        for (int l = 0; l < kTermLevels; ++l) s.grid[l] = sms * terms192_max_ctas_per_sm(l);
+        for (int l = 0; l < kTermLevels; ++l) {
+            const TermGrid per = terms192_ctas_per_sm(l);
+            s.grid[l] = TermGrid{sms * per.tiles, sms * per.shares};
+        }
         s.ready = true;
     }
     *out = &s;
