@@ -366,6 +366,7 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 2 ? 7 : 9) terms192_kernel
         nitems = nitems * (blockIdx.x + 1) / gridDim.x;
     }
     int cur = -1;                                   // segment of the sums held in acc
+    int seg = 0;                                    // segment of the last item
     Acc192 acc;
     acc_zero(acc);
     uint32_t cnt = 0;
@@ -380,10 +381,24 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 2 ? 7 : 9) terms192_kernel
         }
         if (item >= nitems) break;
         const uint64_t t = FIXED ? item >> split.log2_parts : item;
+        // items come in order: in a share mostly this segment's or the next one's, or a
+        // part past its tile's end (64 positions below 1e5: 104 -> 96 us; the counter's
+        // few, larger items gain nothing)
         int lo = 0, hi = nseg - 1;
+        if (FIXED) {
+            lo = seg;
+            if (lo + 1 < nseg && segs[lo + 1].tile0 <= t) ++lo;
+            if (lo + 1 >= nseg || segs[lo + 1].tile0 > t) hi = lo;
+        }
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
             if (segs[mid].tile0 <= t) lo = mid; else hi = mid - 1;
+        }
+        if (FIXED) {                                // parts past the end of their tile
+            seg = lo;
+            const uint64_t off = (t - segs[lo].tile0) * tile_k +
+                                 ((uint32_t)item & ((1u << split.log2_parts) - 1u)) * split.part_k;
+            if (segs[lo].k0 + off >= segs[lo].k1) continue;
         }
         if (lo != cur || __any_sync(0xffffffffu, cnt >= (1u << 30))) {
             if (cur >= 0) flush_segment(segs[cur], lane, acc, cnt, slots, carry);
@@ -392,11 +407,10 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 2 ? 7 : 9) terms192_kernel
             cur = lo;
         }
         const Seg s = segs[lo];
-        const uint64_t k0 = s.k0 + (t - s.tile0) * tile_k;
-        uint64_t kb = k0, ke = min(s.k1, k0 + tile_k);
+        uint64_t kb = s.k0 + (t - s.tile0) * tile_k, ke = min(s.k1, kb + tile_k);
         if (FIXED) {
             kb += ((uint32_t)item & ((1u << split.log2_parts) - 1u)) * split.part_k;
-            ke = min(ke, kb + split.part_k);
+            ke = min(ke, kb + split.part_k);        // a last part may start past the tile's end
             if (kb >= ke) continue;
         }
         if (kb >= s.d) run_tile_kind<LEVEL, true>(s, kb, ke, lane, acc, cnt);
