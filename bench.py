@@ -38,26 +38,26 @@ UNIT = "terms/s"
 # ------------------------------------------------------------ work model --
 def algorithmic_mults(d: int) -> int:
     """Algorithmic 32-bit multiply halves of one position (tails excluded):
-    per term W = 4S + 12 for m < 2^32 and 18S + 33 for m >= 2^32, with
-    S = bitlen(10(d-k)) - 1 squarings (the fixed work definition used for the
-    roofline)."""
+    per term W = 5 (B - 4) + 18 for m < 2^32 and 8 (B - 5) + 30 for m >= 2^32, with
+    B = bitlen(10(d-k)): the ladder steps after the start value (four or five
+    bits) times the halves of the one-word and float-quotient steps, and six
+    quotient digits."""
     from clbellard_gb300 import formula
     total = 0
     for f in range(7):
         _, _, den0, den1 = formula(f)
         k32 = max(0, ((1 << 32) - den1 + den0 - 1) // den0)   # first k with m >= 2^32
-        # e = d - k in [1, d]; S = bitlen(10e) - 1; split e by bitlen of 10e
+        # e = d - k in [1, d], split by B = bitlen(10e)
         for b in range(1, 70):
             lo_e = max(1, -(-(1 << (b - 1)) // 10))          # smallest e with 10e >= 2^(b-1)
             hi_e = min(d, ((1 << b) - 1) // 10)              # largest e with 10e < 2^b
             if hi_e < lo_e:
                 continue
-            S = b - 1
             # k = d - e, so e in [lo_e, hi_e] <-> k in [d - hi_e, d - lo_e]
             ka, kb = d - hi_e, d - lo_e
             n32 = max(0, min(kb, k32 - 1) - ka + 1)           # k < k32: m < 2^32
             n64 = (kb - ka + 1) - n32
-            total += n32 * (4 * S + 12) + n64 * (18 * S + 33)
+            total += n32 * (5 * max(0, b - 4) + 18) + n64 * (8 * max(0, b - 5) + 30)
     return total
 
 
@@ -360,7 +360,7 @@ def ours_arm(args):
         "roofline": {"bound": "int", "achieved": achieved, "peak": peak_ops / 1e9, "unit": "Gmul/s",
                      "frac": achieved / (peak_ops / 1e9), "traffic": traffic,
                      "kernel": "terms192_kernel", "kernel_ms": kms,
-                     "work": "32-bit multiply halves: 4S+12 per term (m<2^32), 18S+33 (m>=2^32)",
+                     "work": "32-bit multiply halves: 5(B-4)+18 per term (m<2^32), 8(B-5)+30 (m>=2^32), B=bitlen(10(d-k))",
                      "peak_source": "measured mad.lo.u32 issue rate (dependent chains, one half each) on this "
                                     "GPU (no integer peak in MEASURED_PEAKS.json)"},
         "gpu_launches": launches,
