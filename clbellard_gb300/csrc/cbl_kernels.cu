@@ -8,7 +8,8 @@
 //                    reductions (Bellard.cl:601-675).
 //   combine_kernel   Ssum_192 + Sum7_192 for every position (Bellard.cl:1300-1398).
 //   dd_*             the 106-bit double-double mode (Bellard.cl:729-763, 914-982,
-//                    1118-1144, 1274-1353), the only FP64 on the GPU.
+//                    1118-1144, 1274-1353): 128-bit fractions summed as integers,
+//                    double-doubles from Ssum on (the only FP64 on the GPU).
 #include "cbl_arith.cuh"
 #include "cbl_internal.h"
 #include <algorithm>

@@ -73,8 +73,8 @@ int cbl_Sglobal32mtg(cbl_ctx *ctx, uint64_t offset, uint64_t d, uint64_t k_max,
                      int64_t numesign, uint64_t den0, uint64_t den1);
 /* Sglobal64mtg / Sglobal64mtg_192 / Sglobal64mtg_192_Refresh (Bellard.cl:914-1092,
  * Bellard_div2by1.cl:313-359): same contract for any modulus below 2^62. In
- * mode 0, moduli from 2^53 up take the OVERDOUBLE route (Bellard.cl:937-945):
- * r and m as exact double-doubles and a double-double division. */
+ * mode 0 one path covers them all: the fractions' first 128 bits, as integers
+ * (the reference switches to its OVERDOUBLE build from 2^53 on, Bellard.cl:937-945). */
 int cbl_Sglobal64mtg(cbl_ctx *ctx, uint64_t offset, uint64_t d, uint64_t k_max,
                      int64_t numesign, uint64_t den0, uint64_t den1);
 /* Sglobal_after / Sglobal_after_192 (Bellard.cl:1118-1253): the tail terms
