@@ -77,7 +77,7 @@ struct cbl_ctx {
     std::vector<int> prep_shift;
     // double-double buffers
     uint4 *d_bigsum = nullptr;                       // 128-bit fractions, one per block of the term kernel
-    int dd_blocks = 1;                               // leading bigSum entries in use since cbl_Set0mem
+    int dd_blocks = 0;                               // leading bigSum entries that hold sums
     double2 *d_ddpartial = nullptr;
     double2 *d_ddans = nullptr;
     // scratch host
@@ -298,9 +298,7 @@ int dd_range(cbl_ctx *c, uint64_t k0, uint64_t k1, uint64_t d, int sign, uint32_
         const int level = b > a ? term_level((uint64_t)den0 * a + den1, (uint64_t)den0 * (b - 1) + den1) : 0;
         if (c->dd_ctas[level] == 0) c->dd_ctas[level] = dd_terms_max_ctas_per_sm(level);
         const int grid = std::min(kDDBlocks, c->sm_count * c->dd_ctas[level]);
-        int blocks = 0;
-        CK(launch_dd_terms(level, c->d_bigsum, grid, &blocks, a, b, d, sign, den0, den1, tail && last, c->st));
-        c->dd_blocks = std::max(c->dd_blocks, blocks);
+        CK(launch_dd_terms(level, c->d_bigsum, grid, &c->dd_blocks, a, b, d, sign, den0, den1, tail && last, c->st));
         c->launches++;
         if (last) break;
     }
@@ -477,7 +475,6 @@ int cbl_create(int device, int precision, cbl_ctx **out)
         cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6 * c->slot_cap, c->st);
         cudaMemsetAsync(c->d_partial, 0, sizeof(uint64_t) * 3, c->st);
         cudaMemsetAsync(c->d_ans, 0, sizeof(uint64_t) * 3, c->st);
-        cudaMemsetAsync(c->d_bigsum, 0, sizeof(uint4) * kDDBlocks, c->st);
         cudaMemsetAsync(c->d_ddpartial, 0, sizeof(double2), c->st);
         cudaMemsetAsync(c->d_ddans, 0, sizeof(double2), c->st);
         if (cudaStreamSynchronize(c->st) != cudaSuccess) rc = CBL_E_CUDA;
@@ -590,8 +587,7 @@ int cbl_Set0mem(cbl_ctx *c)
         CK(cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6, c->st));
         c->slot0_tiles = 0;
     } else {
-        CK(cudaMemsetAsync(c->d_bigsum, 0, sizeof(uint4) * kDDBlocks, c->st));
-        c->dd_blocks = 1;
+        c->dd_blocks = 0;                                 // no entry holds a sum
     }
     return CBL_OK;
     CBL_GUARD_END

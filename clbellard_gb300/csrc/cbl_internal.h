@@ -115,9 +115,10 @@ cudaError_t launch_terms_each(uint64_t d, uint32_t den0, uint32_t den1, int sign
                               int n, uint64_t *out3n, cudaStream_t st);
 
 // Double-double (mode 0) kernels. bigSum is kDDBlocks 128-bit fractions mod 1
-// (little-endian words). launch_dd_terms runs at most `grid` blocks (one wave), block i
-// adding into bigsum[i]; *blocks = the number launched; tail adds the terms k = d .. d+9.
-cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *blocks, uint64_t k0, uint64_t k1, uint64_t d,
+// (little-endian words), of which the first *used hold sums. launch_dd_terms runs at most
+// `grid` blocks (one wave), block i adding into bigsum[i], or setting it from *used on, and
+// raises *used; tail adds the terms k = d .. d+9.
+cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *used, uint64_t k0, uint64_t k1, uint64_t d,
                             int sign, uint32_t den0, uint32_t den1, bool tail, cudaStream_t st);
 int dd_terms_max_ctas_per_sm(int level);
 cudaError_t launch_dd_ssum(const uint4 *bigsum, int nblk, double2 *partial, cudaStream_t st);

@@ -49,3 +49,15 @@ def test_sums_accumulate_over_calls(ctxdd, oracle):
     hi, lo = ctxdd.read_partial()
     t = (Fraction(hi) + Fraction(lo) - want) % 1
     assert min(t, 1 - t) < TOL
+
+
+def test_sums_start_from_zero(ctxdd, oracle):
+    """Set0mem empties bigSum, whatever an earlier range left in more of its entries."""
+    d, f = 3999999999, 2
+    ctxdd.Set0mem()
+    ctxdd.BatchCalc(1000, 3000000, f, d)
+    ctxdd.Set0mem()
+    ctxdd.Ssum()
+    assert ctxdd.read_partial() == (0.0, 0.0)
+    check(ctxdd, oracle, f, d, 500, 620)
+    check(ctxdd, oracle, f, d, 500, 20500)
