@@ -57,6 +57,13 @@ static_assert(sizeof(Seg) == 48, "Seg layout");
 constexpr uint32_t kFlagSign = 1u;
 inline uint32_t seg_flags(int sign, int width) { return (uint32_t)(sign & 1) | ((uint32_t)width << 4); }
 
+// Programmatic dependent launches: a kernel launched as the dependent of the stream's last
+// kernel may be scheduled once every block of that one has passed allow_dependent() or
+// ended, and waits for its end, memory included, in await_predecessor() (which returns at
+// once in a plain launch).
+__device__ __forceinline__ void await_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_dependent() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 // Instantiation of the term kernel for a table whose moduli lie in [min_m, max_m]:
 // 0 the width-1 and lazy kinds only (m < 2^29), 1 all one-word kinds (m < 2^32), 2 also
 // the float-quotient and short two-word kinds (m < 2^44), 3 any kind but without the
@@ -91,17 +98,21 @@ struct TermGrid {
 // then carry each wrap into the digit sum two places up (exact mod 2^192).
 // A slot receives at most one flush per tile, so slot_needs_carry() decides it
 // from the tile counts.
+// dependent: the stream's last operation is the kernel that wrote segs; the launch is its
+// programmatic dependent (cbl_kernels.cu).
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
                             unsigned long long *counter, unsigned long long *slots, const TermGrid &grids,
-                            cudaStream_t st, uint64_t budget_ns, bool carry, bool reset_counter);
+                            cudaStream_t st, uint64_t budget_ns, bool carry, bool reset_counter,
+                            bool dependent = false);
 constexpr uint64_t kCarryTiles = 1ull << 31;
 inline bool slot_needs_carry(uint64_t max_tiles_per_slot) { return max_tiles_per_slot >= kCarryTiles; }
 // slots (nslot x 6 digit sums) of position i, series f = slots[(7 i + f) * 6 ..]:
 // out3[3i..3i+2] (word 0 most significant) = sum_f (S_f << (numer_log2[f] + shift[i])).
 // The same words also go to copy3 (n positions, may be pinned host memory) and, for
-// position 0, to first3, where those are not null.
+// position 0, to first3, where those are not null. dependent: as in launch_terms192.
 cudaError_t launch_combine(const unsigned long long *slots, int npos, const int *shift,
-                           uint64_t *out3, uint64_t *copy3, uint64_t *first3, cudaStream_t st);
+                           uint64_t *out3, uint64_t *copy3, uint64_t *first3, cudaStream_t st,
+                           bool dependent = false);
 // slots[0 .. 6*nslot) <- preset[j % 6] (device array of 6), instead of zero.
 cudaError_t launch_slot_fill(unsigned long long *slots, int nslot, const unsigned long long *preset,
                              cudaStream_t st);

@@ -18,16 +18,12 @@ namespace cbl {
 
 constexpr int kBlock192 = 128;
 
-// The one-block kernels behind a term kernel (Ssum, Sum7) and the mode-0 term kernel
-// are launched as programmatic dependents: they may be scheduled while their predecessor
-// still runs and wait for its end, memory included, in await_predecessor() before they
-// touch anything that it wrote or reads. allow_dependent() lets the next one be scheduled
-// from a block's start on. Seven series at 1e7 in mode 0: 392 us with plain launches, 362 us
-// with dependent Ssum and Sum7, 264 us with the term kernel too, whose terms of one series
+// Programmatic dependents (cbl_internal.h) are the one-block kernels behind a term kernel
+// (Ssum, Sum7), the mode-0 term kernel, and the term and combine kernels of an
+// allocation-free call; each waits before it touches anything that its predecessor
+// wrote or reads. Seven series at 1e7 in mode 0: 392 us with plain launches, 362 us with
+// dependent Ssum and Sum7, 264 us with the term kernel too, whose terms of one series
 // run beside Ssum and Sum7 of the one before.
-__device__ __forceinline__ void await_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void allow_dependent() { asm volatile("griddepcontrol.launch_dependents;"); }
-
 template <typename... Params, typename... Args>
 static cudaError_t launch_dependent(void (*kernel)(Params...), int grid, int block, cudaStream_t st, Args... args)
 {
@@ -362,6 +358,7 @@ __global__ void __launch_bounds__(kBlock192, LEVEL == 2 ? 7 : 9) terms192_kernel
 {
     const int lane = threadIdx.x & 31;
     allow_dependent();
+    await_predecessor();                            // the tile table's kernel, where one precedes
     const uint64_t t_start = budget_ns ? global_ns() : 0;
     uint64_t nitems = ntiles, item = 0;
     if (FIXED) {                                    // this block's share, dealt to its warps in turn
@@ -458,7 +455,7 @@ TileSplit tile_split(uint64_t ntiles, uint32_t tile_k, int grid)
 
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
                             unsigned long long *counter, unsigned long long *slots, const TermGrid &grids,
-                            cudaStream_t st, uint64_t budget_ns, bool carry, bool reset_counter)
+                            cudaStream_t st, uint64_t budget_ns, bool carry, bool reset_counter, bool dependent)
 {
     // a budgeted pass stops and resumes at whole tiles
     const TileSplit sp = budget_ns ? TileSplit{0, 0, tile_k} : tile_split(ntiles, tile_k, grids.tiles);
@@ -468,6 +465,9 @@ cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntile
         if (e != cudaSuccess) return e;
     }
     const Terms192Fn fn = sp.fixed ? terms192_fn<true>(level) : terms192_fn<false>(level);
+    if (dependent)
+        return launch_dependent(fn, grid, kBlock192, st, segs, nseg, ntiles, tile_k, sp, counter, slots, budget_ns,
+                                carry ? 1 : 0);
     fn<<<grid, kBlock192, 0, st>>>(segs, nseg, ntiles, tile_k, sp, counter, slots, budget_ns, carry ? 1 : 0);
     return cudaGetLastError();
 }
@@ -549,6 +549,7 @@ cudaError_t launch_slot_fill(unsigned long long *slots, int nslot, const unsigne
 __global__ void combine_kernel(const unsigned long long *slots, int npos, const int *shift, uint64_t *out3,
                                uint64_t *copy3, uint64_t *first3)
 {
+    await_predecessor();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npos) return;
     uint64_t ans[3] = {0, 0, 0};
@@ -569,9 +570,11 @@ __global__ void combine_kernel(const unsigned long long *slots, int npos, const 
 }
 
 cudaError_t launch_combine(const unsigned long long *slots, int npos, const int *shift, uint64_t *out3,
-                           uint64_t *copy3, uint64_t *first3, cudaStream_t st)
+                           uint64_t *copy3, uint64_t *first3, cudaStream_t st, bool dependent)
 {
     const int b = 128;
+    if (dependent)
+        return launch_dependent(combine_kernel, (npos + b - 1) / b, b, st, slots, npos, shift, out3, copy3, first3);
     combine_kernel<<<(npos + b - 1) / b, b, 0, st>>>(slots, npos, shift, out3, copy3, first3);
     return cudaGetLastError();
 }

@@ -8,7 +8,8 @@
 //
 // The positions travel to the GPU as a kernel parameter, and a one-block
 // kernel builds the tile table in the array, so a call issues no host-to-device
-// copy: it enqueues a memset and three kernels on the caller's stream and
+// copy: it enqueues three kernels on the caller's stream (the second and third as
+// programmatic dependents, so they are in place when their predecessor ends) and
 // returns without waiting for them.
 #include "../../include/clbellard.h"
 #include "cbl_internal.h"
@@ -42,11 +43,6 @@ __host__ __device__ __forceinline__ uint32_t series_den0(int f) { return f < 2 ?
 __host__ __device__ __forceinline__ uint32_t series_den1(int f) { return (0x9753131u >> (4 * f)) & 15u; }
 __host__ __device__ __forceinline__ int series_sign(int f) { return (0x3Bu >> f) & 1u; }
 
-struct Piece {
-    uint64_t k0, k1;
-    uint32_t kind;     // residue kind 1..6 (cbl_internal.h)
-};
-
 // First k with den0 k + den1 >= limit; with den0 and den1 known the division folds away.
 constexpr uint64_t first_k(uint64_t limit, uint64_t den0, uint64_t den1) { return (limit - den1 + den0 - 1) / den0; }
 
@@ -67,45 +63,32 @@ constexpr KindCuts make_kind_cuts()
 [[maybe_unused]] constexpr KindCuts kCuts = make_kind_cuts();
 __constant__ KindCuts d_cuts = make_kind_cuts();
 
-// The pieces of series f at position d, in increasing k. k = 0 of a series
-// with den1 = 1 has m = 1 and contributes exactly 0, so it is left out.
-__host__ __device__ inline int series_pieces(uint64_t d, int f, Piece out[kMaxPieces])
+// A piece's terms k in [k0, k1); empty where k0 >= k1.
+struct Piece {
+    uint64_t k0, k1;
+};
+
+// The part of series f at position d in residue kind q (0 .. 5, in order of m), main body
+// or tail. k = 0 of a series with den1 = 1 has m = 1 and contributes exactly 0, so it is
+// left out.
+__host__ __device__ __forceinline__ Piece series_piece(uint64_t d, int f, int q, bool tail)
 {
 #ifdef __CUDA_ARCH__
     const uint64_t *cut = d_cuts.k[f];
 #else
     const uint64_t *cut = kCuts.k[f];
 #endif
-    constexpr uint32_t kind[6] = {1, 5, 3, 4, 2, 6};
-    uint64_t k = series_den1(f) == 1 ? 1 : 0;
-    const uint64_t k1 = d + kTail192;
-    int n = 0;
-    for (int i = 0; i < 6; ++i) {                                    // main body and tail of each kind's range
-        const uint64_t end = i < 5 && cut[i] < k1 ? cut[i] : k1;
-        const uint64_t body = end < d ? end : d;
-        if (k < body) {
-            out[n++] = Piece{k, body, kind[i]};
-            k = body;
-        }
-        if (k < end) {
-            out[n++] = Piece{k, end, kind[i]};
-            k = end;
-        }
-    }
-    return n;
-}
-
-// Bucket of a piece: main body before tail, then the costlier residue kind
-// first (wide width 2, width 2, short width 2, strict, middle, width 1).
-__host__ __device__ __forceinline__ int piece_bucket(const Piece &p, uint64_t d)
-{
-    const int order = p.kind == 6 ? 0 : p.kind == 2 ? 1 : p.kind == 4 ? 2 : p.kind == 3 ? 3 : p.kind == 5 ? 4 : 5;
-    return (p.k0 >= d ? 6 : 0) + order;
+    Piece p;
+    p.k0 = q > 0 ? cut[q - 1] : series_den1(f) == 1 ? 1 : 0;
+    p.k1 = tail ? d + kTail192 : d;
+    if (tail && p.k0 < d) p.k0 = d;
+    if (q < 5 && cut[q] < p.k1) p.k1 = cut[q];
+    return p;
 }
 
 __host__ __device__ __forceinline__ uint64_t piece_tiles(const Piece &p)
 {
-    return (p.k1 - p.k0 + kTileTerms - 1) / kTileTerms;
+    return p.k0 < p.k1 ? (p.k1 - p.k0 + kTileTerms - 1) / kTileTerms : 0;
 }
 
 struct PositionArgs {
@@ -119,93 +102,126 @@ struct PositionArgs {
 // process exits; all calls on a device share it.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
-// One block, thread i for position i (of kMaxPos). The table is ordered
-// costliest tiles first: by bucket, then by d (larger first, ties by position
-// index), then by series; a series has at most one piece per bucket. Thread i
-// counts its pieces and tiles per bucket under its rank in that d order, the block
-// scans the counts (bucket-major, then rank) into offsets, 12 cells a thread, then
-// every thread writes its segments. One thread doing the scan, and 64-bit divisions
-// for the cuts, made this 34 us of a 1.46 ms call.
-__global__ void __launch_bounds__(kMaxPos) noalloc_table_kernel(PositionArgs a, Seg *segs)
+// A piece's place among its position's series, in the eight lanes that hold them: the
+// segments and tiles of the series before it, and of all of them (in lane 7's next).
+struct Place {
+    uint32_t seg, next_seg;
+    uint64_t tile, next_tile;
+};
+
+__device__ __forceinline__ Place place_among_series(uint64_t tiles, int f)
 {
+    uint32_t s = tiles != 0;
+    uint64_t t = tiles;
+#pragma unroll
+    for (int w = 1; w < 8; w *= 2) {
+        const uint32_t us = __shfl_up_sync(0xffffffffu, s, w, 8);
+        const uint64_t ut = __shfl_up_sync(0xffffffffu, t, w, 8);
+        if (f >= w) {
+            s += us;
+            t += ut;
+        }
+    }
+    return Place{s - (tiles != 0), s, t - tiles, t};
+}
+
+// One block, eight lanes a position (of kMaxPos), lane f for series f. The table is
+// ordered costliest tiles first: by bucket (main body before tail, then the costlier
+// residue kind), then by d (larger first, ties by position index), then by series; a
+// series has at most one piece per bucket. The lanes of a position count its pieces and
+// tiles per bucket under its rank in that d order, two warps scan the counts
+// (bucket-major, then rank) into offsets, 12 cells a thread, then every lane writes
+// its segments. The zeros for the kernels behind it go first. What bounds it is latency:
+// loads, fetches of code that no warp has run yet and barriers in sequence, which is why a
+// series is a lane and no loop is unrolled. With one thread a position, a memset of its own
+// and plain launches behind it a call of one position at 1e4 took 26.4 us (calls in a
+// row) and 64 positions at 1e4 53 us; now 19.1 and 44 us.
+__global__ void __launch_bounds__(8 * kMaxPos) noalloc_table_kernel(const __grid_constant__ PositionArgs a, Seg *segs,
+                                                                    uint4 *zero)
+{
+    __shared__ uint64_t sd[kMaxPos];
     __shared__ uint32_t seg_off[kBuckets * kMaxPos];
     __shared__ uint64_t tile_off[kBuckets * kMaxPos];
     __shared__ uint32_t warp_segs;
     __shared__ uint64_t warp_tiles;
     static_assert(kMaxPos == 64, "two warps scan");
-    const int i = threadIdx.x;
+    allow_dependent();
+    const int tid = threadIdx.x, i = tid >> 3, f = tid & 7;
+#pragma unroll 1
+    for (int z = tid; z < (int)(kOffSegs / sizeof(uint4)); z += 8 * kMaxPos) zero[z] = make_uint4(0, 0, 0, 0);
+    if (tid < kMaxPos) sd[tid] = a.d[tid];
+    __syncthreads();
+    const bool used = i < a.n;
+    const uint64_t d = used ? sd[i] : 0;
+    int rank = 0;                                           // unused positions keep their own cells, empty
+#pragma unroll 1
+    for (int j = f; j < a.n; j += 8) rank += sd[j] > d || (sd[j] == d && j < i);
+#pragma unroll
+    for (int w = 1; w < 8; w *= 2) rank += __shfl_xor_sync(0xffffffffu, rank, w);
+    if (!used) rank = i;
+#pragma unroll 1
     for (int b = 0; b < kBuckets; ++b) {
-        seg_off[b * kMaxPos + i] = 0;
-        tile_off[b * kMaxPos + i] = 0;
+        const uint64_t tiles = used && f < 7 ? piece_tiles(series_piece(d, f, 5 - b % 6, b >= 6)) : 0;
+        const Place at = place_among_series(tiles, f);
+        if (f == 7) {
+            seg_off[b * kMaxPos + rank] = at.next_seg;
+            tile_off[b * kMaxPos + rank] = at.next_tile;
+        }
     }
     __syncthreads();
-    int rank = 0;
-    uint64_t d = 0;
-    Piece p[kMaxPieces];
-    if (i < a.n) {
-        d = a.d[i];
-        for (int j = 0; j < a.n; ++j)
-            if (a.d[j] > d || (a.d[j] == d && j < i)) ++rank;
-        for (int f = 0; f < 7; ++f) {
-            const int np = series_pieces(d, f, p);
-            for (int q = 0; q < np; ++q) {
-                const int c = piece_bucket(p[q], d) * kMaxPos + rank;
-                seg_off[c] += 1;
-                tile_off[c] += piece_tiles(p[q]);
+    if (tid < 64) {                                         // exclusive scan over cells 12 tid .. 12 tid + 11
+        uint32_t s = 0;
+        uint64_t t = 0;
+#pragma unroll 1
+        for (int c = kBuckets * tid; c < kBuckets * (tid + 1); ++c) {
+            s += seg_off[c];
+            t += tile_off[c];
+        }
+        const uint32_t own_s = s;
+        const uint64_t own_t = t;
+        for (int w = 1; w < 32; w *= 2) {
+            const uint32_t us = __shfl_up_sync(0xffffffffu, s, w);
+            const uint64_t ut = __shfl_up_sync(0xffffffffu, t, w);
+            if ((tid & 31) >= w) {
+                s += us;
+                t += ut;
             }
         }
-    }
-    __syncthreads();
-    uint32_t s = 0;                                         // exclusive scan over cells 12 i .. 12 i + 11
-    uint64_t t = 0;
-    for (int c = kBuckets * i; c < kBuckets * (i + 1); ++c) {
-        s += seg_off[c];
-        t += tile_off[c];
-    }
-    const uint32_t own_s = s;
-    const uint64_t own_t = t;
-    for (int w = 1; w < 32; w *= 2) {
-        const uint32_t us = __shfl_up_sync(0xffffffffu, s, w);
-        const uint64_t ut = __shfl_up_sync(0xffffffffu, t, w);
-        if ((i & 31) >= w) {
-            s += us;
-            t += ut;
+        if (tid == 31) {
+            warp_segs = s;
+            warp_tiles = t;
+        }
+        asm volatile("bar.sync 1, 64;" ::: "memory");       // the two scanning warps
+        s += (tid >= 32 ? warp_segs : 0) - own_s;
+        t += (tid >= 32 ? warp_tiles : 0) - own_t;
+#pragma unroll 1
+        for (int c = kBuckets * tid; c < kBuckets * (tid + 1); ++c) {
+            const uint32_t cs = seg_off[c];
+            const uint64_t ct = tile_off[c];
+            seg_off[c] = s;
+            tile_off[c] = t;
+            s += cs;
+            t += ct;
         }
     }
-    if (i == 31) {
-        warp_segs = s;
-        warp_tiles = t;
-    }
     __syncthreads();
-    s += (i >= 32 ? warp_segs : 0) - own_s;
-    t += (i >= 32 ? warp_tiles : 0) - own_t;
-    for (int c = kBuckets * i; c < kBuckets * (i + 1); ++c) {
-        const uint32_t cs = seg_off[c];
-        const uint64_t ct = tile_off[c];
-        seg_off[c] = s;
-        tile_off[c] = t;
-        s += cs;
-        t += ct;
-    }
-    __syncthreads();
-    if (i >= a.n) return;
-    for (int f = 0; f < 7; ++f) {
-        const int np = series_pieces(d, f, p);
-        for (int q = 0; q < np; ++q) {
-            const int c = piece_bucket(p[q], d) * kMaxPos + rank;
-            Seg s;
-            s.d = d;
-            s.k0 = p[q].k0;
-            s.k1 = p[q].k1;
-            s.tile0 = tile_off[c];
-            s.den0 = series_den0(f);
-            s.den1 = series_den1(f);
-            s.slot = (uint32_t)(i * 7 + f);
-            s.flags = (uint32_t)series_sign(f) | (p[q].kind << 4);
-            segs[seg_off[c]] = s;
-            seg_off[c] += 1;                                // this (bucket, rank) cell is this thread's alone
-            tile_off[c] += piece_tiles(p[q]);
-        }
+#pragma unroll 1
+    for (int b = 0; b < kBuckets; ++b) {
+        const int q = 5 - b % 6;
+        const Piece p = series_piece(d, f < 7 ? f : 0, q, b >= 6);
+        const uint64_t tiles = used && f < 7 ? piece_tiles(p) : 0;
+        const Place at = place_among_series(tiles, f);
+        if (tiles == 0) continue;
+        Seg s;
+        s.d = d;
+        s.k0 = p.k0;
+        s.k1 = p.k1;
+        s.tile0 = tile_off[b * kMaxPos + rank] + at.tile;
+        s.den0 = series_den0(f);
+        s.den1 = series_den1(f);
+        s.slot = (uint32_t)(i * 7 + f);
+        s.flags = (uint32_t)series_sign(f) | (((0x624351u >> (4 * q)) & 15u) << 4);     // kinds 1, 5, 3, 4, 2, 6
+        segs[seg_off[b * kMaxPos + rank] + at.seg] = s;
     }
 }
 
@@ -269,12 +285,14 @@ extern "C" int cbl_batch_noalloc(const uint64_t *pos, int n, uint64_t *d_out3n, 
         args.d[i] = d;
         const uint64_t m_last = 10 * (d + kTail192 - 1) + 9;
         max_m = max_m > m_last ? max_m : m_last;
-        Piece p[kMaxPieces];
         for (int f = 0; f < 7; ++f) {
-            const int np = series_pieces(d, f, p);
-            nseg += np;
             uint64_t series_tiles = 0;
-            for (int q = 0; q < np; ++q) series_tiles += piece_tiles(p[q]);
+            for (int q = 0; q < 6 && (q == 0 || kCuts.k[f][q - 1] < d + kTail192); ++q)
+                for (int tail = 0; tail < 2; ++tail) {
+                    const uint64_t tiles = piece_tiles(series_piece(d, f, q, tail != 0));
+                    nseg += tiles != 0;
+                    series_tiles += tiles;
+                }
             ntiles += series_tiles;
             max_series_tiles = max_series_tiles > series_tiles ? max_series_tiles : series_tiles;
         }
@@ -291,16 +309,15 @@ extern "C" int cbl_batch_noalloc(const uint64_t *pos, int n, uint64_t *d_out3n, 
     auto *slots = reinterpret_cast<unsigned long long *>(base + kOffSlots);
     auto *shift = reinterpret_cast<int *>(base + kOffShift);
     auto *dsegs = reinterpret_cast<Seg *>(base + kOffSegs);
-    // the array keeps the previous call's contents: zero the counter, the digit
-    // sums and the shifts; the table kernel overwrites the first nseg segments
-    if (cudaMemsetAsync(base, 0, kOffSegs, st) != cudaSuccess) return CBL_E_CUDA;
-    noalloc_table_kernel<<<1, kMaxPos, 0, st>>>(args, dsegs);
+    // the array keeps the previous call's contents: the table kernel zeroes the counter, the
+    // digit sums and the shifts and overwrites the first nseg segments
+    noalloc_table_kernel<<<1, 8 * kMaxPos, 0, st>>>(args, dsegs, reinterpret_cast<uint4 *>(base));
     if (cudaGetLastError() != cudaSuccess) return CBL_E_CUDA;
     const int level = term_level(0, max_m);
     if (launch_terms192(level, dsegs, nseg, ntiles, (uint32_t)kTileTerms, counter, slots, ds->grid[level], st, 0,
-                        slot_needs_carry(max_series_tiles), false) != cudaSuccess)
+                        slot_needs_carry(max_series_tiles), false, true) != cudaSuccess)
         return CBL_E_CUDA;
-    if (launch_combine(slots, n, shift, d_out3n, nullptr, nullptr, st) != cudaSuccess) return CBL_E_CUDA;
+    if (launch_combine(slots, n, shift, d_out3n, nullptr, nullptr, st, true) != cudaSuccess) return CBL_E_CUDA;
     return CBL_OK;
     CBL_GUARD_END
 }

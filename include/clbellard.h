@@ -223,8 +223,8 @@ const char *cbl_strerror(int code);
  * significant word first), bit-identical to cbl_batch, once `stream` (a
  * cudaStream_t, 0 for the legacy default stream) reaches that point. The
  * positions go to the GPU as a kernel argument and the tile table is built on
- * the device, so the call makes no host-to-device copy: it enqueues a memset
- * and three kernels and returns without waiting for them.
+ * the device, so the call makes no host-to-device copy: it enqueues three
+ * kernels and returns without waiting for them.
  * The kernels' scratch is one static device array of CBL_NOALLOC_SCRATCH_BYTES
  * (about 169 KiB) that every GPU loading this library holds until the process
  * exits. The first call on each device looks up that array's device address
