@@ -349,8 +349,10 @@ __device__ __forceinline__ void run_tile_kind(const Seg &s, uint64_t kb, uint64_
 // warps in blocks of 256, 125.8 ms at 11 blocks) and 72 at 7 for the float-quotient
 // kinds (1e10: 541.4 ms; 543.6 at 8, 547 at 9, 569 at 10 with spills). Three and four
 // ladders a lane, with 80 and 96 registers, ran those at 548 and 595 ms, one at 613 ms.
+// segs is not __restrict__: as a dependent the kernel starts while its predecessor still
+// writes the table, so loads of it must stay coherent and behind await_predecessor().
 template <int LEVEL, bool FIXED>
-__global__ void __launch_bounds__(kBlock192, LEVEL == 2 ? 7 : 9) terms192_kernel(const Seg *__restrict__ segs, int nseg,
+__global__ void __launch_bounds__(kBlock192, LEVEL == 2 ? 7 : 9) terms192_kernel(const Seg *segs, int nseg,
                                                              uint64_t ntiles, uint32_t tile_k, TileSplit split,
                                                              unsigned long long *counter,
                                                              unsigned long long *slots, uint64_t budget_ns,
