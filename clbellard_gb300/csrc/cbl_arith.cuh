@@ -752,24 +752,37 @@ __device__ __forceinline__ void walk_bits_start_pair(uint64_t EpA, uint64_t EpB,
 // agree above bit S, those bits come from one word P and both ladders share the
 // shift counts, and so they do in the last six bits (EpA - EpB = 320 = 5 * 2^6).
 // Other groups, and exponents outside [2^(S+4) + 630, 2^(S+32)), walk their own bits.
+// LONG (the two-word kinds of large positions): exponents from 2^(S+32) on too, whose bits
+// above S are walked in two words (2^26 terms at 1e14, m from 2e12 on: 2905 us; 3025 us when
+// such groups walked their own bits).
 // S = 12 / 13 / 14 / 15 / 16 measured 113.9 / 110.4 / 108.9 / 108.2 / 107.6 ms on 512 positions
 // below 1e8.
 constexpr int kGroupBits = 16;
-template <int NB, typename State, typename Start>
+template <int NB, bool LONG = false, typename State, typename Start>
 __device__ __forceinline__ void walk_bits_group(uint64_t EpA, uint64_t EpB, uint64_t ep_max, State &A, State &B,
                                                 Start start)
 {
     constexpr int S = kGroupBits;
     const uint32_t P = (uint32_t)(ep_max >> S);
-    if (ep_max >= (1ull << (S + 4)) + 630 && ep_max >> (S + 32) == 0 && (uint32_t)((ep_max - 630) >> S) == P) {
-        int j = 32 - NB - __clz(P);
-        start(A, P >> j);
-        start(B, P >> j);
+    if (ep_max >= (1ull << (S + 4)) + 630 && (LONG || ep_max >> (S + 32) == 0) &&
+        (LONG ? (ep_max - 630) >> S == ep_max >> S : (uint32_t)((ep_max - 630) >> S) == P)) {
+        const uint32_t over = LONG ? (uint32_t)(ep_max >> (S + 32)) : 0u;
+        int more = 32 - __clz(over);                         // common bits below the first word's
+        uint32_t W = LONG ? __funnelshift_r(P, over, more) : P;
+        int j = 32 - NB - __clz(W);
+        start(A, W >> j);
+        start(B, W >> j);
+        for (;;) {
 #pragma unroll 4
-        for (--j; j >= 0; --j) {
-            const uint32_t b = (P >> j) & 1u;
-            A.step(b);
-            B.step(b);
+            for (--j; j >= 0; --j) {
+                const uint32_t b = (W >> j) & 1u;
+                A.step(b);
+                B.step(b);
+            }
+            if (!LONG || more == 0) break;
+            W = P;
+            j = more;
+            more = 0;
         }
         const uint32_t la = (uint32_t)EpA, lb = (uint32_t)EpB;
 #pragma unroll
