@@ -752,9 +752,10 @@ __device__ __forceinline__ void walk_bits_start_pair(uint64_t EpA, uint64_t EpB,
 // agree above bit S, those bits come from one word P and both ladders share the
 // shift counts, and so they do in the last six bits (EpA - EpB = 320 = 5 * 2^6).
 // Other groups, and exponents outside [2^(S+4) + 630, 2^(S+32)), walk their own bits.
-// LONG (the two-word kinds of large positions): exponents from 2^(S+32) on too, whose bits
-// above S are walked in two words (2^26 terms at 1e14, m from 2e12 on: 2905 us; 3025 us when
-// such groups walked their own bits).
+// LONG (the short two-word kind): exponents from 2^(S+32) on too, whose bits above S are
+// walked in two words (2^28 terms at 1e14, m from 2e12 on: 11.51 ms; 11.78 ms when such
+// groups walked their own bits). The general kinds do without: with it there too the
+// short kind ran 0.5 % slower at 1e13 (10.82 against 10.76 ms), one kernel holding all.
 // S = 12 / 13 / 14 / 15 / 16 measured 113.9 / 110.4 / 108.9 / 108.2 / 107.6 ms on 512 positions
 // below 1e8.
 constexpr int kGroupBits = 16;

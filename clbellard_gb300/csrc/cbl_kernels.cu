@@ -134,12 +134,12 @@ __device__ __forceinline__ void term_pair(uint64_t Ea, uint64_t e_max, uint64_t 
         w2_redc_down<N>(lazy_residue(B), mb, mpb, qb);
     } else if (KIND == 2) {
         W2State A{0, 0, (uint32_t)ma, (uint32_t)(ma >> 32), mpa}, B{0, 0, (uint32_t)mb, (uint32_t)(mb >> 32), mpb};
-        walk_bits_group<4, true>(Ea - 64, Eb - 64, e_max - 64, A, B, W2Start<64>{});
+        walk_bits_group<4>(Ea - 64, Eb - 64, e_max - 64, A, B, W2Start<64>{});
         w2_redc_down<N>(lazy_residue(A), ma, mpa, qa);
         w2_redc_down<N>(lazy_residue(B), mb, mpb, qb);
     } else if (KIND == 6) {
         W2XState A = w2x_state(ma, mpa), B = w2x_state(mb, mpb);
-        walk_bits_group<4, true>(Ea - 64, Eb - 64, e_max - 64, A, B, W2Start<64>{});
+        walk_bits_group<4>(Ea - 64, Eb - 64, e_max - 64, A, B, W2Start<64>{});
         const uint64_t ra = two_words(A.y0, A.y1), rb = two_words(B.y0, B.y1);     // below 2m
         w2_redc_down<N>(min(ra, ra - ma), ma, mpa, qa);
         w2_redc_down<N>(min(rb, rb - mb), mb, mpb, qb);
