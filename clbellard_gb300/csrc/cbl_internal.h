@@ -77,11 +77,35 @@ __host__ __device__ inline int term_level(uint64_t min_m, uint64_t max_m)
     return max_m < kW1LMax ? 0 : max_m < kW1SMax ? 1 : max_m < kW2SMax && min_m < kW2FMax ? 2 : 3;
 }
 
+constexpr int kBlock192 = 128;            // threads of the term kernel's blocks
+
 // How a pass without a time budget deals its tiles out: from the tile counter, or
 // (fixed) as 2^log2_parts parts of part_k terms each, one contiguous share a block.
 struct TileSplit {
     uint32_t log2_parts, fixed, part_k;
 };
+
+// A pass with fewer tiles than resident warps leaves most of the GPU idle and its
+// lanes a long serial run (position 1e6: 1367 tiles for 6080 warps, 64 terms a
+// lane). Its tiles are cut into parts of down to 64 terms, about four a warp, and
+// every block takes one contiguous share: no counter to wait for, and one slot
+// update a block instead of one a part (those queue at three cache lines: 141 us
+// at 1e6). Measured, term kernel: 1e4 24.5 -> 8 us, 1e5 39 -> 10.4 us, 1e6 52 -> 39 us,
+// 2^20 terms at 1e11 187 -> 64 us. From one tile a warp on, contiguous shares lose to
+// the counter (1e7 268 -> 274 us, 1e8 2.61 -> 2.82 ms): costs differ along the table.
+inline TileSplit tile_split(uint64_t ntiles, uint32_t tile_k, int grid)
+{
+    const uint64_t warps = (uint64_t)grid * (kBlock192 / 32);
+    TileSplit sp{0, 0, tile_k};
+    if (ntiles >= warps) return sp;
+    sp.fixed = 1;
+    while (sp.part_k > 64 && (ntiles << sp.log2_parts) < 4 * warps) {
+        ++sp.log2_parts;
+        const uint64_t unit = 64ull << sp.log2_parts;              // rounded up: the parts cover the tile
+        sp.part_k = (uint32_t)((tile_k + unit - 1) / unit) * 64;
+    }
+    return sp;
+}
 
 // Resident blocks (of one SM, or of a grid) of the term kernel's two forms.
 struct TermGrid {

@@ -16,8 +16,6 @@
 
 namespace cbl {
 
-constexpr int kBlock192 = 128;
-
 // Programmatic dependents (cbl_internal.h) are the one-block kernels behind a term kernel
 // (Ssum, Sum7), the mode-0 term kernel, and the term and combine kernels of an
 // allocation-free call; each waits before it touches anything that its predecessor
@@ -432,27 +430,6 @@ static Terms192Fn terms192_fn(int level)
     static const Terms192Fn fn[kTermLevels] = {terms192_kernel<0, FIXED>, terms192_kernel<1, FIXED>,
                                                terms192_kernel<2, FIXED>, terms192_kernel<3, FIXED>};
     return fn[level];
-}
-
-// A pass with fewer tiles than resident warps leaves most of the GPU idle and its
-// lanes a long serial run (position 1e6: 1367 tiles for 6080 warps, 64 terms a
-// lane). Its tiles are cut into parts of down to 64 terms, about four a warp, and
-// every block takes one contiguous share: no counter to wait for, and one slot
-// update a block instead of one a part (those queue at three cache lines: 141 us
-// at 1e6). Measured, term kernel: 1e4 24.5 -> 8 us, 1e5 39 -> 10.4 us, 1e6 52 -> 39 us,
-// 2^20 terms at 1e11 187 -> 64 us. From one tile a warp on, contiguous shares lose to
-// the counter (1e7 268 -> 274 us, 1e8 2.61 -> 2.82 ms): costs differ along the table.
-TileSplit tile_split(uint64_t ntiles, uint32_t tile_k, int grid)
-{
-    const uint64_t warps = (uint64_t)grid * (kBlock192 / 32);
-    TileSplit sp{0, 0, tile_k};
-    if (ntiles >= warps) return sp;
-    sp.fixed = 1;
-    while (sp.part_k > 64 && (ntiles << sp.log2_parts) < 4 * warps) {
-        ++sp.log2_parts;
-        sp.part_k = ((tile_k >> sp.log2_parts) + 63) / 64 * 64;
-    }
-    return sp;
 }
 
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
