@@ -67,7 +67,7 @@ struct cbl_ctx {
     uint64_t prep_ntiles = 0;
     uint64_t prep_terms = 0;
     bool prep_carry = false;                         // a prepared slot may take >= 2^31 flushes
-    uint64_t slot0_tiles = 0;                        // tiles added into slot 0 since it was zeroed
+    uint64_t slot0_flushes = 0;                      // most flushes that slot 0 took since it was zeroed
     cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;   // around the term kernel of the last prepared run
     bool ev_valid = false;
     cudaGraphExec_t graph = nullptr;                 // captured prepared pass
@@ -275,12 +275,14 @@ int run_segments(cbl_ctx *c, std::vector<Seg> &v)
     const uint64_t ntiles = order_and_number(v, (uint32_t)c->tile_k);
     const int rc = upload_table(c, v, nullptr, 0);
     if (rc) return rc;
-    // slot 0 collects every launch since cbl_Set0mem: carry once it may have
-    // taken 2^31 flushes (at most one per tile)
-    c->slot0_tiles = std::min<uint64_t>(c->slot0_tiles + ntiles, kCarryTiles);
     const int level = segs_level(v);
-    CK(launch_terms192(level, c->d_segs, (int)v.size(), ntiles, (uint32_t)c->tile_k, c->d_counter, c->d_slots,
-                       grid_192(c, level), c->st, 0, slot_needs_carry(c->slot0_tiles), true));
+    const TermGrid grid = grid_192(c, level);
+    // slot 0 collects every launch since cbl_Set0mem: carry once it may have
+    // taken 2^31 flushes
+    c->slot0_flushes = std::min<uint64_t>(c->slot0_flushes + flush_bound(ntiles, (uint32_t)c->tile_k, grid.tiles),
+                                          kCarryFlushes);
+    CK(launch_terms192(level, c->d_segs, (int)v.size(), ntiles, (uint32_t)c->tile_k, c->d_counter, c->d_slots, grid,
+                       c->st, 0, slot_needs_carry(c->slot0_flushes), true));
     c->launches++;
     return CBL_OK;
 }
@@ -585,7 +587,7 @@ int cbl_Set0mem(cbl_ctx *c)
     cudaSetDevice(c->device);
     if (is192(c)) {
         CK(cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6, c->st));
-        c->slot0_tiles = 0;
+        c->slot0_flushes = 0;
     } else {
         c->dd_blocks = 0;                                 // no entry holds a sum
     }
@@ -803,7 +805,7 @@ static int upload_prepared(cbl_ctx *c)
         t += (sg.k1 - sg.k0 + c->tile_k - 1) / c->tile_k;
         max_slot_tiles = std::max(max_slot_tiles, t);
     }
-    c->prep_carry = slot_needs_carry(max_slot_tiles);
+    c->prep_carry = slot_needs_carry(max_slot_tiles);   // in parts a pass has fewer tiles than warps: no carry
     const int rc = upload_table(c, v, c->prep_shift.data(), n);
     if (rc) return rc;
     drop_graph(c);
@@ -846,7 +848,7 @@ static bool prepared_carry(const cbl_ctx *c) { return c->prep_carry || c->d_pres
 // (until cbl_Set0mem).
 static cudaError_t clear_slots(cbl_ctx *c, int nslot)
 {
-    c->slot0_tiles = kCarryTiles;
+    c->slot0_flushes = kCarryFlushes;
     if (c->d_preset) return launch_slot_fill(c->d_slots, nslot, c->d_preset, c->st);
     return cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6 * nslot, c->st);
 }

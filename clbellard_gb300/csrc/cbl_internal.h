@@ -107,6 +107,14 @@ inline TileSplit tile_split(uint64_t ntiles, uint32_t tile_k, int grid)
     return sp;
 }
 
+// Most flushes into one slot that a pass can make: a warp or block flushes only sums of
+// tiles of its own or, in the fixed form, of parts of its own (one 2048-term tile is up to
+// 32 parts in as many blocks, each with its flush).
+inline uint64_t flush_bound(uint64_t ntiles, uint32_t tile_k, int grid)
+{
+    return ntiles << tile_split(ntiles, tile_k, grid).log2_parts;
+}
+
 // Resident blocks (of one SM, or of a grid) of the term kernel's two forms.
 struct TermGrid {
     int tiles = 0;         // tiles from the counter
@@ -120,16 +128,15 @@ struct TermGrid {
 // carry: the slots' digit sums may wrap past 2^64 (a slot can receive 2^31 or
 // more flushes since it was zeroed, or it started from a preset); the flushes
 // then carry each wrap into the digit sum two places up (exact mod 2^192).
-// A slot receives at most one flush per tile, so slot_needs_carry() decides it
-// from the tile counts.
+// slot_needs_carry() decides it from flush_bound().
 // dependent: the stream's last operation is the kernel that wrote segs; the launch is its
 // programmatic dependent (cbl_kernels.cu).
 cudaError_t launch_terms192(int level, const Seg *segs, int nseg, uint64_t ntiles, uint32_t tile_k,
                             unsigned long long *counter, unsigned long long *slots, const TermGrid &grids,
                             cudaStream_t st, uint64_t budget_ns, bool carry, bool reset_counter,
                             bool dependent = false);
-constexpr uint64_t kCarryTiles = 1ull << 31;
-inline bool slot_needs_carry(uint64_t max_tiles_per_slot) { return max_tiles_per_slot >= kCarryTiles; }
+constexpr uint64_t kCarryFlushes = 1ull << 31;
+inline bool slot_needs_carry(uint64_t max_flushes) { return max_flushes >= kCarryFlushes; }
 // slots (nslot x 6 digit sums) of position i, series f = slots[(7 i + f) * 6 ..]:
 // out3[3i..3i+2] (word 0 most significant) = sum_f (S_f << (numer_log2[f] + shift[i])).
 // The same words also go to copy3 (n positions, may be pinned host memory) and, for

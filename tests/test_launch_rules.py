@@ -1,5 +1,5 @@
 """The host's launch rules (csrc/cbl_internal.h), compiled for the CPU: how a pass is
-dealt out to blocks."""
+dealt out to blocks, and how many flushes a digit-sum slot can take from it."""
 import ctypes
 import os
 import subprocess
@@ -17,6 +17,8 @@ extern "C" void split(uint64_t ntiles, uint32_t tile_k, int grid, uint32_t out[3
     out[1] = s.fixed;
     out[2] = s.part_k;
 }
+extern "C" uint64_t flushes(uint64_t ntiles, uint32_t tile_k, int grid) { return cbl::flush_bound(ntiles, tile_k, grid); }
+extern "C" int carry(uint64_t n) { return cbl::slot_needs_carry(n); }
 """
 
 
@@ -29,6 +31,9 @@ def rules(tmp_path_factory):
                     str(d / "rules.cpp"), "-o", str(d / "rules.so")], check=True)
     lib = ctypes.CDLL(str(d / "rules.so"))
     lib.split.argtypes = [ctypes.c_uint64, ctypes.c_uint32, ctypes.c_int, ctypes.POINTER(ctypes.c_uint32)]
+    lib.flushes.argtypes = [ctypes.c_uint64, ctypes.c_uint32, ctypes.c_int]
+    lib.flushes.restype = ctypes.c_uint64
+    lib.carry.argtypes = [ctypes.c_uint64]
     return lib
 
 
@@ -53,3 +58,51 @@ def test_parts_cover_their_tile(rules, grid):
             assert part_k << log2_parts >= tile_k, (tile_k, ntiles)
             assert log2_parts == 0 or part_k % 64 == 0, (tile_k, ntiles)
         assert split(rules, 4 * grid, tile_k, grid) == (0, 0, tile_k)
+
+
+def flushes_in_shares(segments, tile_k, split, blocks):
+    """Flushes of a pass in fixed shares into the one slot of its segments (term counts),
+    dealt out as the term kernel does it: a block's items go to its four warps in turn, a
+    warp flushes at a change of segment, and the warps still in warp 0's segment at the
+    end flush once together."""
+    log2_parts, _, part_k = split
+    items = []                                              # the segment of each part, None past its end
+    for s, n in enumerate(segments):
+        for t in range(-(-n // tile_k)):
+            items += [s if t * tile_k + p * part_k < min(n, (t + 1) * tile_k) and p * part_k < tile_k else None
+                      for p in range(1 << log2_parts)]
+    total = 0
+    for b in range(blocks):
+        share = items[len(items) * b // blocks:len(items) * (b + 1) // blocks]
+        last = []
+        for w in range(4):
+            run = [s for s in share[w::4] if s is not None]
+            total += sum(x != y for x, y in zip(run, run[1:]))
+            last.append(run[-1] if run else None)
+        total += sum(s is not None and s != last[0] for s in last) + (last[0] is not None)
+    return total
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+@pytest.mark.parametrize("segments", [[65536], [1], [2048 * 3, 20], [100000, 300, 5, 20], [409600]])
+def test_flush_bound_covers_fixed_shares(rules, grid, segments):
+    for tile_k in (64, 2048, 4128, 65536):
+        ntiles = sum(-(-n // tile_k) for n in segments)
+        sp = split(rules, ntiles, tile_k, grid)
+        bound = rules.flushes(ntiles, tile_k, grid)
+        if sp[1]:
+            blocks = min(grid, ntiles << sp[0])
+            assert flushes_in_shares(segments, tile_k, sp, blocks) <= bound
+        else:
+            assert bound == ntiles
+
+
+def test_carry_before_a_digit_sum_can_wrap(rules):
+    """Launches of 65,536 terms into one slot, 32 tiles each, make hundreds of flushes a
+    launch: the carry is on well before 2^32 of them."""
+    sp = split(rules, 32, 2048, 1368)
+    made = flushes_in_shares([65536], 2048, sp, min(1368, 32 << sp[0]))
+    assert made > 10 * 32
+    launches = (1 << 32) // made                            # as many as could not wrap
+    assert rules.carry(launches * rules.flushes(32, 2048, 1368))
+    assert not rules.carry((1 << 31) - 1)
