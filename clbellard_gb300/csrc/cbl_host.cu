@@ -31,6 +31,16 @@ typedef unsigned __int128 u128;
 
 }  // namespace
 
+// A tile table on the device (the segments, then one shift per position) and its pinned staging.
+struct TileTable {
+    unsigned char *dev = nullptr;
+    unsigned char *host = nullptr;
+    size_t cap = 0;
+    bool busy = false;                        // the staging may still feed a copy in flight
+    Seg *segs = nullptr;                      // = dev
+    int *shift = nullptr;                     // inside dev
+};
+
 struct cbl_ctx {
     int device = 0;
     int precision = 1;
@@ -42,17 +52,15 @@ struct cbl_ctx {
     int ctas_per_sm = 0;
     TermGrid term_ctas[kTermLevels];          // resident CTAs per SM, 0 = not asked yet
     int dd_ctas[kTermLevels] = {};
-    // 192-bit buffers
-    // tile table: the segments, then (prepared passes) one shift per position
-    unsigned char *d_table = nullptr;
-    unsigned char *h_table = nullptr;         // its pinned staging
-    size_t table_cap = 0;
-    bool staging_busy = false;                // h_table may still feed a copy in flight
-    Seg *d_segs = nullptr;                    // = d_table
-    int *d_shift = nullptr;                   // inside d_table
+    // 192-bit buffers: tile table, tile counter and slots of the prepared passes, and a table,
+    // counter and slot (bigSum) of their own for the kernel-by-kernel calls, which may come
+    // between a prepare and its passes
+    TileTable prep_table, job_table;
     unsigned long long *d_counter = nullptr;
-    unsigned long long *d_slots = nullptr;   // nslot x 6 digit sums; slot 0 is bigSum
+    unsigned long long *d_slots = nullptr;   // nslot x 6 digit sums
     int slot_cap = 0;
+    unsigned long long *d_job_counter = nullptr;      // inside d_counter's allocation, a cache line each
+    unsigned long long *d_bigslot = nullptr;
     uint64_t *d_partial = nullptr;           // 3 words, most significant first
     uint64_t *d_ans = nullptr;               // 3 words
     uint64_t *d_out3 = nullptr;
@@ -67,7 +75,7 @@ struct cbl_ctx {
     uint64_t prep_ntiles = 0;
     uint64_t prep_terms = 0;
     bool prep_carry = false;                         // a prepared slot may take >= 2^31 flushes
-    uint64_t slot0_flushes = 0;                      // most flushes that slot 0 took since it was zeroed
+    uint64_t bigslot_flushes = 0;                    // most flushes that bigSum took since it was zeroed
     cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;   // around the term kernel of the last prepared run
     bool ev_valid = false;
     cudaGraphExec_t graph = nullptr;                 // captured prepared pass
@@ -109,38 +117,42 @@ void drop_graph(cbl_ctx *c)
 int sync(cbl_ctx *c)
 {
     CK(cudaStreamSynchronize(c->st));
-    c->staging_busy = false;
+    c->prep_table.busy = c->job_table.busy = false;
     return CBL_OK;
 }
 
-int ensure_table(cbl_ctx *c, size_t bytes)
+void free_table(TileTable &t)
 {
-    if (bytes <= c->table_cap) return CBL_OK;
-    const size_t cap = std::max(bytes, 2 * c->table_cap);
-    cudaFree(c->d_table);
-    cudaFreeHost(c->h_table);
-    c->d_table = c->h_table = nullptr;
-    c->table_cap = 0;
-    if (cudaMalloc(&c->d_table, cap) != cudaSuccess) return CBL_E_NOMEM;
-    if (cudaMallocHost(&c->h_table, cap) != cudaSuccess) return CBL_E_NOMEM;
-    c->table_cap = cap;
+    cudaFree(t.dev);
+    cudaFreeHost(t.host);
+    t = TileTable{};
+}
+
+int ensure_table(TileTable &t, size_t bytes)
+{
+    if (bytes <= t.cap) return CBL_OK;
+    const size_t cap = std::max(bytes, 2 * t.cap);
+    free_table(t);
+    if (cudaMalloc(&t.dev, cap) != cudaSuccess) return CBL_E_NOMEM;
+    if (cudaMallocHost(&t.host, cap) != cudaSuccess) return CBL_E_NOMEM;
+    t.cap = cap;
     return CBL_OK;
 }
 
 // Upload a tile table (segments, then n shifts) through the pinned staging buffer,
 // waiting for the stream only where an earlier copy may still read that buffer.
-int upload_table(cbl_ctx *c, const std::vector<Seg> &v, const int *shift, int n)
+int upload_table(cbl_ctx *c, TileTable &t, const std::vector<Seg> &v, const int *shift, int n)
 {
     const size_t seg_bytes = sizeof(Seg) * v.size(), bytes = seg_bytes + sizeof(int) * (size_t)n;
-    int rc = c->staging_busy ? sync(c) : CBL_OK;
-    if (!rc) rc = ensure_table(c, bytes);
+    int rc = t.busy ? sync(c) : CBL_OK;
+    if (!rc) rc = ensure_table(t, bytes);
     if (rc) return rc;
-    std::memcpy(c->h_table, v.data(), seg_bytes);
-    if (n > 0) std::memcpy(c->h_table + seg_bytes, shift, sizeof(int) * (size_t)n);
-    c->staging_busy = true;
-    CK(cudaMemcpyAsync(c->d_table, c->h_table, bytes, cudaMemcpyHostToDevice, c->st));
-    c->d_segs = reinterpret_cast<Seg *>(c->d_table);
-    c->d_shift = reinterpret_cast<int *>(c->d_table + seg_bytes);
+    std::memcpy(t.host, v.data(), seg_bytes);
+    if (n > 0) std::memcpy(t.host + seg_bytes, shift, sizeof(int) * (size_t)n);
+    t.busy = true;
+    CK(cudaMemcpyAsync(t.dev, t.host, bytes, cudaMemcpyHostToDevice, c->st));
+    t.segs = reinterpret_cast<Seg *>(t.dev);
+    t.shift = reinterpret_cast<int *>(t.dev + seg_bytes);
     return CBL_OK;
 }
 
@@ -268,21 +280,21 @@ int segs_level(const std::vector<Seg> &v)
     return term_level(lo, hi);
 }
 
-// Upload segments and run the persistent term kernel (accumulates into slots).
+// Upload segments and run the persistent term kernel (accumulates into bigSum).
 int run_segments(cbl_ctx *c, std::vector<Seg> &v)
 {
     if (v.empty()) return CBL_OK;
     const uint64_t ntiles = order_and_number(v, (uint32_t)c->tile_k);
-    const int rc = upload_table(c, v, nullptr, 0);
+    const int rc = upload_table(c, c->job_table, v, nullptr, 0);
     if (rc) return rc;
     const int level = segs_level(v);
     const TermGrid grid = grid_192(c, level);
-    // slot 0 collects every launch since cbl_Set0mem: carry once it may have
+    // bigSum collects every launch since cbl_Set0mem: carry once it may have
     // taken 2^31 flushes
-    c->slot0_flushes = std::min<uint64_t>(c->slot0_flushes + flush_bound(ntiles, (uint32_t)c->tile_k, grid.tiles),
-                                          kCarryFlushes);
-    CK(launch_terms192(level, c->d_segs, (int)v.size(), ntiles, (uint32_t)c->tile_k, c->d_counter, c->d_slots, grid,
-                       c->st, 0, slot_needs_carry(c->slot0_flushes), true));
+    c->bigslot_flushes = std::min<uint64_t>(c->bigslot_flushes + flush_bound(ntiles, (uint32_t)c->tile_k, grid.tiles),
+                                            kCarryFlushes);
+    CK(launch_terms192(level, c->job_table.segs, (int)v.size(), ntiles, (uint32_t)c->tile_k, c->d_job_counter,
+                       c->d_bigslot, grid, c->st, 0, slot_needs_carry(c->bigslot_flushes), true));
     c->launches++;
     return CBL_OK;
 }
@@ -461,7 +473,11 @@ int cbl_create(int device, int precision, cbl_ctx **out)
         std::snprintf(c->devname, sizeof c->devname, "%s", prop.name);
     int rc = CBL_OK;
     if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess) rc = CBL_E_CUDA;
-    if (!rc && cudaMalloc(&c->d_counter, sizeof(unsigned long long)) != cudaSuccess) rc = CBL_E_NOMEM;
+    if (!rc && cudaMalloc(&c->d_counter, sizeof(unsigned long long) * 48) != cudaSuccess) rc = CBL_E_NOMEM;
+    if (!rc) {
+        c->d_job_counter = c->d_counter + 16;
+        c->d_bigslot = c->d_counter + 32;
+    }
     if (!rc && cudaMalloc(&c->d_partial, sizeof(uint64_t) * 3) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ans, sizeof(uint64_t) * 3) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_bigsum, sizeof(uint4) * kDDBlocks) != cudaSuccess) rc = CBL_E_NOMEM;
@@ -471,10 +487,12 @@ int cbl_create(int device, int precision, cbl_ctx **out)
     if (!rc && cudaEventCreate(&c->ev_k0) != cudaSuccess) rc = CBL_E_CUDA;
     if (!rc && cudaEventCreate(&c->ev_k1) != cudaSuccess) rc = CBL_E_CUDA;
     if (!rc) rc = ensure_slots(c, 8);
-    if (!rc) rc = ensure_table(c, 64 * sizeof(Seg));
+    if (!rc) rc = ensure_table(c->prep_table, 64 * sizeof(Seg));
+    if (!rc) rc = ensure_table(c->job_table, 16 * sizeof(Seg));
     if (!rc) rc = ensure_pos(c, 1);
     if (!rc) {
         cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6 * c->slot_cap, c->st);
+        cudaMemsetAsync(c->d_bigslot, 0, sizeof(unsigned long long) * 6, c->st);
         cudaMemsetAsync(c->d_partial, 0, sizeof(uint64_t) * 3, c->st);
         cudaMemsetAsync(c->d_ans, 0, sizeof(uint64_t) * 3, c->st);
         cudaMemsetAsync(c->d_ddpartial, 0, sizeof(double2), c->st);
@@ -496,8 +514,8 @@ int cbl_destroy(cbl_ctx *c)
     if (!c) return CBL_E_ARG;
     cudaSetDevice(c->device);
     if (c->st) cudaStreamSynchronize(c->st);
-    cudaFree(c->d_table);
-    cudaFreeHost(c->h_table);
+    free_table(c->prep_table);
+    free_table(c->job_table);
     cudaFree(c->d_counter);
     cudaFree(c->d_slots);
     cudaFree(c->d_partial);
@@ -586,8 +604,8 @@ int cbl_Set0mem(cbl_ctx *c)
     if (!c) return CBL_E_ARG;
     cudaSetDevice(c->device);
     if (is192(c)) {
-        CK(cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6, c->st));
-        c->slot0_flushes = 0;
+        CK(cudaMemsetAsync(c->d_bigslot, 0, sizeof(unsigned long long) * 6, c->st));
+        c->bigslot_flushes = 0;
     } else {
         c->dd_blocks = 0;                                 // no entry holds a sum
     }
@@ -659,7 +677,7 @@ int cbl_Ssum(cbl_ctx *c)
     CBL_GUARD_BEGIN
     if (!c) return CBL_E_ARG;
     cudaSetDevice(c->device);
-    if (is192(c)) CK(launch_ssum192(c->d_slots, c->d_partial, c->st));
+    if (is192(c)) CK(launch_ssum192(c->d_bigslot, c->d_partial, c->st));
     else CK(launch_dd_ssum(c->d_bigsum, c->dd_blocks, c->d_ddpartial, c->st));
     c->launches++;
     return CBL_OK;
@@ -749,7 +767,7 @@ int cbl_query(cbl_ctx *c)
     if (!c) return CBL_E_ARG;
     const cudaError_t e = cudaStreamQuery(c->st);
     if (e == cudaSuccess) {
-        c->staging_busy = false;
+        c->prep_table.busy = c->job_table.busy = false;
         return 0;
     }
     if (e == cudaErrorNotReady) {
@@ -806,7 +824,7 @@ static int upload_prepared(cbl_ctx *c)
         max_slot_tiles = std::max(max_slot_tiles, t);
     }
     c->prep_carry = slot_needs_carry(max_slot_tiles);   // in parts a pass has fewer tiles than warps: no carry
-    const int rc = upload_table(c, v, c->prep_shift.data(), n);
+    const int rc = upload_table(c, c->prep_table, v, c->prep_shift.data(), n);
     if (rc) return rc;
     drop_graph(c);
     c->prep_nseg = (int)v.size();
@@ -843,12 +861,9 @@ static int prepare_positions(cbl_ctx *c, const uint64_t *d, const int *shift, in
 // flushes or starts from a preset.
 static bool prepared_carry(const cbl_ctx *c) { return c->prep_carry || c->d_preset != nullptr; }
 
-// Zero the first nslot slots, or set them to the test preset. Slot 0 is then
-// no longer a known count of flushes from zero for the kernel-by-kernel calls
-// (until cbl_Set0mem).
+// Zero the first nslot slots, or set them to the test preset.
 static cudaError_t clear_slots(cbl_ctx *c, int nslot)
 {
-    c->slot0_flushes = kCarryFlushes;
     if (c->d_preset) return launch_slot_fill(c->d_slots, nslot, c->d_preset, c->st);
     return cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6 * nslot, c->st);
 }
@@ -864,10 +879,10 @@ static int enqueue_prepared(cbl_ctx *c, bool capturing, uint64_t *host3, uint64_
     const int n = c->prep_npos;
     CK(clear_slots(c, 7 * n));
     CK(cudaEventRecordWithFlags(c->ev_k0, c->st, evf));
-    CK(launch_terms192(c->prep_level, c->d_segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k, c->d_counter,
-                       c->d_slots, grid_192(c, c->prep_level), c->st, 0, prepared_carry(c), true));
+    CK(launch_terms192(c->prep_level, c->prep_table.segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k,
+                       c->d_counter, c->d_slots, grid_192(c, c->prep_level), c->st, 0, prepared_carry(c), true));
     CK(cudaEventRecordWithFlags(c->ev_k1, c->st, evf));
-    CK(launch_combine(c->d_slots, n, c->d_shift, c->d_out3, host3, ans, c->st));
+    CK(launch_combine(c->d_slots, n, c->prep_table.shift, c->d_out3, host3, ans, c->st));
     return CBL_OK;
 }
 
@@ -1416,15 +1431,15 @@ int cbl_run_prepared_budget(cbl_ctx *c, double budget_ms, uint64_t *tiles_done, 
         c->partial = 1;
     }
     const uint64_t budget_ns = (uint64_t)(budget_ms * 1e6) + 1;
-    CK(launch_terms192(c->prep_level, c->d_segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k, c->d_counter,
-                       c->d_slots, grid_192(c, c->prep_level), c->st, budget_ns, prepared_carry(c), false));
+    CK(launch_terms192(c->prep_level, c->prep_table.segs, c->prep_nseg, c->prep_ntiles, (uint32_t)c->tile_k,
+                       c->d_counter, c->d_slots, grid_192(c, c->prep_level), c->st, budget_ns, prepared_carry(c), false));
     c->launches++;
     CK(cudaMemcpyAsync(c->h_small, c->d_counter, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->st));
     int rc = sync(c);
     if (rc) return rc;
     const uint64_t done = std::min<uint64_t>(c->h_small[0], c->prep_ntiles);
     if (done >= c->prep_ntiles) {
-        CK(launch_combine(c->d_slots, n, c->d_shift, c->d_out3, nullptr, nullptr, c->st));
+        CK(launch_combine(c->d_slots, n, c->prep_table.shift, c->d_out3, nullptr, nullptr, c->st));
         c->launches++;
         c->partial = 0;
     }

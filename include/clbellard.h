@@ -150,7 +150,10 @@ int cbl_workdir_sum(const char *workdir, char out[49], int counts[7]);
 /* out3n[3*i .. 3*i+2] = 192-bit result for reference position pos[i] (modes 1-2). */
 int cbl_batch(cbl_ctx *ctx, const uint64_t *pos, int n, uint64_t *out3n);
 
-/* ---- prepared runs (the timed device pass of a benchmark) */
+/* ---- prepared runs (the timed device pass of a benchmark)
+ * A prepared table, its passes and their progress stand apart from bigSum: kernel-by-kernel
+ * calls and jobs (cbl_Sglobal*, cbl_BatchCalc, cbl_run_job) may come in between. cbl_compute,
+ * cbl_compute_hexpos and cbl_batch prepare their own positions. */
 /* Build and upload the tile table for reference positions pos[0..n). */
 int cbl_prepare(cbl_ctx *ctx, const uint64_t *pos, int n);
 /* Enqueue one full pass over the prepared positions (no host sync). */
