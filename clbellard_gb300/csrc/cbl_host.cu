@@ -49,7 +49,7 @@ struct cbl_ctx {
     char devname[256] = {0};
     int64_t launches = 0;
     int tile_k = kDefaultTile;
-    int ctas_per_sm = 0;
+    int ctas_per_sm = 0;                      // of 256 threads (tuned_blocks), 0 = as many as are resident
     TermGrid term_ctas[kTermLevels];          // resident CTAs per SM, 0 = not asked yet
     int dd_ctas[kTermLevels] = {};
     // 192-bit buffers: tile table, tile counter and slots of the prepared passes, and a table,
@@ -265,8 +265,8 @@ TermGrid grid_192(cbl_ctx *c, int level)
 {
     TermGrid &per = c->term_ctas[level];
     if (per.tiles == 0) per = terms192_ctas_per_sm(level);
-    return TermGrid{std::max(1, c->sm_count * (c->ctas_per_sm > 0 ? c->ctas_per_sm : per.tiles)),
-                    std::max(1, c->sm_count * (c->ctas_per_sm > 0 ? c->ctas_per_sm : per.shares))};
+    return TermGrid{std::max(1, c->sm_count * tuned_blocks(c->ctas_per_sm, per.tiles)),
+                    std::max(1, c->sm_count * tuned_blocks(c->ctas_per_sm, per.shares))};
 }
 
 // Term-kernel level of a set of segments.
@@ -1321,7 +1321,7 @@ int cbl_prepared_info(const cbl_ctx *c, uint64_t *terms, uint64_t *tiles, int *s
     if (terms) *terms = c->prep_terms;
     if (tiles) *tiles = c->prep_ntiles;
     if (segments) *segments = c->prep_nseg;
-    if (grid) *grid = grid_192(const_cast<cbl_ctx *>(c), c->prep_level).tiles;
+    if (grid) *grid = blocks_to_ctas(grid_192(const_cast<cbl_ctx *>(c), c->prep_level).tiles);
     return CBL_OK;
     CBL_GUARD_END
 }
@@ -1389,7 +1389,7 @@ int cbl_autotune(cbl_ctx *c, const uint64_t *pos, int n, int force, int *best_ti
             if (rc) return rc;
             d_max = std::max(d_max, d);
         }
-        const int occ = terms192_ctas_per_sm(term_level(0, 10 * (d_max + kTail192) + 9)).tiles;
+        const int occ = blocks_to_ctas(terms192_ctas_per_sm(term_level(0, 10 * (d_max + kTail192) + 9)).tiles);
         const int tiles[] = {512, 1024, 2048, 4096, 8192};
         ms_best = 1e300;
         for (int t : tiles) {

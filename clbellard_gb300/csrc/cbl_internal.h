@@ -107,6 +107,18 @@ inline TileSplit tile_split(uint64_t ntiles, uint32_t tile_k, int grid)
     return sp;
 }
 
+// cbl_set_tuning, the autotuner with its cache file, and cbl_prepared_info count CTAs of
+// 256 threads, whatever blocks the kernels run in: resident warps, and so the meaning of a
+// stored or written setting, do not change with the kernels' block size. Blocks an SM for
+// a setting (0 = as many as are resident, which is also the most: one wave at every level).
+constexpr int kCtaThreads = 256;
+inline int tuned_blocks(int ctas, int resident)
+{
+    return ctas > 0 && ctas < resident && ctas * (kCtaThreads / kBlock192) < resident
+               ? ctas * (kCtaThreads / kBlock192) : resident;
+}
+inline int blocks_to_ctas(int blocks) { return (blocks + kCtaThreads / kBlock192 - 1) / (kCtaThreads / kBlock192); }
+
 // Most flushes into one slot that a pass can make: a warp or block flushes only sums of
 // tiles of its own or, in the fixed form, of parts of its own (one 2048-term tile is up to
 // 32 parts in as many blocks, each with its flush).

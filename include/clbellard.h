@@ -180,7 +180,8 @@ int cbl_set_graph(cbl_ctx *ctx, int enable);
 /* Device time of the term kernel in the last cbl_run_prepared (CUDA events on
  * the context's stream around that launch); waits for it to finish. */
 int cbl_kernel_ms(cbl_ctx *ctx, float *ms);
-/* Terms (7*d summed, tail excluded), warp tiles, segments and persistent grid of the prepared run. */
+/* Terms (7*d summed, tail excluded), warp tiles, segments and persistent grid (in CTAs of
+ * 256 threads) of the prepared run. */
 int cbl_prepared_info(const cbl_ctx *ctx, uint64_t *terms, uint64_t *tiles, int *segments, int *grid);
 
 /* ---- diagnostics */
@@ -209,7 +210,9 @@ int cbl_autotune(cbl_ctx *ctx, const uint64_t *pos, int n, int force, int *best_
  * within a few tiles, which exercises the carry that keeps results exact however
  * many tiles land in one slot (positions beyond 2^32 tiles per series). */
 int cbl_set_slot_preset(cbl_ctx *ctx, const uint64_t preset[6]);
-/* Tuning: terms per warp tile (multiple of 32) and persistent CTAs per SM (0 = auto). */
+/* Tuning: terms per warp tile (multiple of 32) and persistent CTAs per SM (0 = auto, as many
+ * as are resident, which is also the most). A CTA counts 256 threads here and in the
+ * autotuner, whatever block size the kernels use. */
 int cbl_set_tuning(cbl_ctx *ctx, int tile_terms, int ctas_per_sm);
 const char *cbl_strerror(int code);
 

@@ -18,6 +18,8 @@ extern "C" void split(uint64_t ntiles, uint32_t tile_k, int grid, uint32_t out[3
     out[2] = s.part_k;
 }
 extern "C" uint64_t flushes(uint64_t ntiles, uint32_t tile_k, int grid) { return cbl::flush_bound(ntiles, tile_k, grid); }
+extern "C" int blocks(int ctas, int resident) { return cbl::tuned_blocks(ctas, resident); }
+extern "C" int block_threads() { return cbl::kBlock192; }
 extern "C" int carry(uint64_t n) { return cbl::slot_needs_carry(n); }
 """
 
@@ -106,3 +108,12 @@ def test_carry_before_a_digit_sum_can_wrap(rules):
     launches = (1 << 32) // made                            # as many as could not wrap
     assert rules.carry(launches * rules.flushes(32, 2048, 1368))
     assert not rules.carry((1 << 31) - 1)
+
+
+@pytest.mark.parametrize("resident", [1, 7, 9, 16])
+def test_tuning_counts_256_threads_a_cta(rules, resident):
+    """A setting of n CTAs is n x 256 threads an SM, up to what is resident."""
+    threads = rules.block_threads()
+    for ctas in (1, 2, 3, 4, 5, 8, 1000, (1 << 31) - 1):
+        assert rules.blocks(ctas, resident) * threads == min(ctas * 256, resident * threads), ctas
+    assert rules.blocks(0, resident) == resident
