@@ -1327,7 +1327,12 @@ int cbl_prepared_info(const cbl_ctx *c, uint64_t *terms, uint64_t *tiles, int *s
 }
 
 // ---- autotuning: tile size x persistent CTAs per SM, timed on the caller's
-// positions, cached per (device name, SM count, positions) in a text file.
+// positions, cached per (device name, SM count, kernels, positions) in a text file.
+// kernels: the term kernels' generation, raised when their tuning may have moved, then
+// the block size and the resident blocks of the level at hand: an entry that other
+// kernels were timed for is not found and is measured again.
+constexpr int kTuneGeneration = 2;
+
 static std::string tune_cache_path()
 {
     if (const char *p = std::getenv("CBL_TUNE_CACHE")) return p;
@@ -1371,9 +1376,18 @@ int cbl_autotune(cbl_ctx *c, const uint64_t *pos, int n, int force, int *best_ti
     if (!c || !pos || n <= 0) return CBL_E_ARG;
     if (!is192(c)) return CBL_E_PRECISION;
     cudaSetDevice(c->device);
+    uint64_t d_max = 0;
+    for (int i = 0; i < n; ++i) {
+        uint64_t d = 0;
+        const int rc = cbl_pos_to_d(pos[i], &d, nullptr);
+        if (rc) return rc;
+        d_max = std::max(d_max, d);
+    }
+    const int level = term_level(0, 10 * (d_max + kTail192) + 9);
+    const int blocks = terms192_ctas_per_sm(level).tiles;
     char key[400];
-    std::snprintf(key, sizeof key, "%s|sm%d|n%d|h%016llx", c->devname, c->sm_count, n,
-                  (unsigned long long)fnv1a(pos, sizeof(uint64_t) * n));
+    std::snprintf(key, sizeof key, "%s|sm%d|g%d.%dx%d|n%d|h%016llx", c->devname, c->sm_count, kTuneGeneration, kBlock192,
+                  blocks, n, (unsigned long long)fnv1a(pos, sizeof(uint64_t) * n));
     for (char *q = key; *q; ++q)
         if (*q == ' ') *q = '_';
     int tile = 0, ctas = 0;
@@ -1382,14 +1396,7 @@ int cbl_autotune(cbl_ctx *c, const uint64_t *pos, int n, int force, int *best_ti
         int rc = cbl_set_tuning(c, tile, ctas);
         if (rc) return rc;
     } else {
-        uint64_t d_max = 0;
-        for (int i = 0; i < n; ++i) {
-            uint64_t d = 0;
-            const int rc = cbl_pos_to_d(pos[i], &d, nullptr);
-            if (rc) return rc;
-            d_max = std::max(d_max, d);
-        }
-        const int occ = blocks_to_ctas(terms192_ctas_per_sm(term_level(0, 10 * (d_max + kTail192) + 9)).tiles);
+        const int occ = blocks_to_ctas(blocks);
         const int tiles[] = {512, 1024, 2048, 4096, 8192};
         ms_best = 1e300;
         for (int t : tiles) {

@@ -198,7 +198,8 @@ int64_t cbl_launch_count(const cbl_ctx *ctx);
  * (512..8192 terms) and persistent CTAs per SM (the occupancy limit and two
  * below it), keeps the fastest (cbl_set_tuning) and appends it to a cache
  * file ($CBL_TUNE_CACHE, default ~/.cache/clbellard_tune.txt) keyed by device,
- * SM count and positions; a cached entry is reused unless force != 0
+ * SM count, kernels (entries of other builds' kernels are not taken) and
+ * positions; a cached entry is reused unless force != 0
  * (*best_ms is then -1). Leaves the context prepared for pos. */
 int cbl_autotune(cbl_ctx *ctx, const uint64_t *pos, int n, int force, int *best_tile, int *best_ctas,
                  double *best_ms);
