@@ -84,7 +84,7 @@ struct cbl_ctx {
     std::vector<Seg> prep_segs;                      // host copy of the prepared segments
     std::vector<int> prep_shift;
     // double-double buffers
-    uint4 *d_bigsum = nullptr;                       // 128-bit fractions, one per block of the term kernel
+    uint2 *d_bigsum = nullptr;                       // 192-bit fractions, one per block of the term kernel
     int dd_blocks = 0;                               // leading bigSum entries that hold sums
     double2 *d_ddpartial = nullptr;
     double2 *d_ddans = nullptr;
@@ -304,15 +304,21 @@ int dd_range(cbl_ctx *c, uint64_t k0, uint64_t k1, uint64_t d, int sign, uint32_
 {
     if (k1 > k0 && (u128)den0 * (k1 - 1) + den1 >= (u128)kW2XMax) return CBL_E_POSITION;
     if (k0 == 0 && den1 == 1) k0 = 1;                    // m = 1 contributes exactly 0
-    // chunks of 2^30 terms keep each launch to a bounded time; the last takes the tail
+    // the terms next to d, which may be small, go with the tail: [end0, end1)
+    const uint64_t end0 = k0 < k1 ? std::max(k0, d - std::min<uint64_t>(d, kEndDD)) : d;
+    const uint64_t end1 = tail ? d + kTailDD : k1;
+    const int end_n = end1 > end0 ? (int)(end1 - end0) : 0;
+    k1 = std::min(k1, end0);
+    // chunks of 2^30 terms keep each launch to a bounded time; the last takes the end
     const uint64_t chunk = 1ull << 30;
-    for (uint64_t a = k0; a < k1 || tail; a += chunk) {
+    for (uint64_t a = k0; a < k1 || end_n > 0; a += chunk) {
         const uint64_t b = std::max(a, std::min(k1, a + chunk));
         const bool last = b >= k1;
         const int level = b > a ? term_level((uint64_t)den0 * a + den1, (uint64_t)den0 * (b - 1) + den1) : 0;
         if (c->dd_ctas[level] == 0) c->dd_ctas[level] = dd_terms_max_ctas_per_sm(level);
         const int grid = std::min(kDDBlocks, c->sm_count * c->dd_ctas[level]);
-        CK(launch_dd_terms(level, c->d_bigsum, grid, &c->dd_blocks, a, b, d, sign, den0, den1, tail && last, c->st));
+        CK(launch_dd_terms(level, c->d_bigsum, grid, &c->dd_blocks, a, b, d, sign, den0, den1, end0,
+                           last ? end_n : 0, c->st));
         c->launches++;
         if (last) break;
     }
@@ -480,7 +486,7 @@ int cbl_create(int device, int precision, cbl_ctx **out)
     }
     if (!rc && cudaMalloc(&c->d_partial, sizeof(uint64_t) * 3) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ans, sizeof(uint64_t) * 3) != cudaSuccess) rc = CBL_E_NOMEM;
-    if (!rc && cudaMalloc(&c->d_bigsum, sizeof(uint4) * kDDBlocks) != cudaSuccess) rc = CBL_E_NOMEM;
+    if (!rc && cudaMalloc(&c->d_bigsum, 3 * sizeof(uint2) * kDDBlocks) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ddpartial, sizeof(double2)) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ddans, sizeof(double2)) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMallocHost(&c->h_small, sizeof(uint64_t) * 8) != cudaSuccess) rc = CBL_E_NOMEM;

@@ -40,6 +40,8 @@ constexpr uint64_t kW2XMax = 1ull << 62;  // wide width 2 (residues < 2m) for 2^
 
 constexpr int kTail192 = 20;   // tail terms k = d..d+19 (Bellard.cl:1164-1239)
 constexpr int kTailDD = 10;    // tail terms k = d..d+9  (Bellard.cl:1125)
+constexpr int kEndDD = 6;      // terms before d with 2^(10(d-k)) < 2^62, which may be below every modulus
+static_assert(kEndDD + kTailDD <= 32, "a lane each");
 
 // One contiguous k-range of one series at one position, within one residue
 // width. Tiles of `tile_k` consecutive k are handed to warps in order of the
@@ -168,14 +170,15 @@ cudaError_t launch_sum7_192(uint64_t *partial, uint64_t *ans, int numer_log2, cu
 cudaError_t launch_terms_each(uint64_t d, uint32_t den0, uint32_t den1, int sign, const uint64_t *k,
                               int n, uint64_t *out3n, cudaStream_t st);
 
-// Double-double (mode 0) kernels. bigSum is kDDBlocks 128-bit fractions mod 1
-// (little-endian words), of which the first *used hold sums. launch_dd_terms runs at most
-// `grid` blocks (one wave), block i adding into bigsum[i], or setting it from *used on, and
-// raises *used; tail adds the terms k = d .. d+9.
-cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *used, uint64_t k0, uint64_t k1, uint64_t d,
-                            int sign, uint32_t den0, uint32_t den1, bool tail, cudaStream_t st);
+// Double-double (mode 0) kernels. bigSum is kDDBlocks 192-bit fractions mod 1
+// (little-endian words, three uint2 each), of which the first *used hold sums.
+// launch_dd_terms runs at most `grid` blocks (one wave), block i adding into entry i, or
+// setting it from *used on, and raises *used; k in [k0, k1) with k1 <= d, and the end_n
+// (at most kEndDD + kTailDD) terms from end0 >= d - kEndDD on.
+cudaError_t launch_dd_terms(int level, uint2 *bigsum, int grid, int *used, uint64_t k0, uint64_t k1, uint64_t d,
+                            int sign, uint32_t den0, uint32_t den1, uint64_t end0, int end_n, cudaStream_t st);
 int dd_terms_max_ctas_per_sm(int level);
-cudaError_t launch_dd_ssum(const uint4 *bigsum, int nblk, double2 *partial, cudaStream_t st);
+cudaError_t launch_dd_ssum(const uint2 *bigsum, int nblk, double2 *partial, cudaStream_t st);
 cudaError_t launch_dd_sum7(double2 *partial, double2 *ans, int numer, cudaStream_t st);
 
 // Throughput probe: grid x block threads each run `iters` rounds of 16

@@ -8,7 +8,7 @@
 //                    reductions (Bellard.cl:601-675).
 //   combine_kernel   Ssum_192 + Sum7_192 for every position (Bellard.cl:1300-1398).
 //   dd_*             the 106-bit double-double mode (Bellard.cl:729-763, 914-982,
-//                    1118-1144, 1274-1353): 128-bit fractions summed as integers,
+//                    1118-1144, 1274-1353): fractions summed as integers,
 //                    double-doubles from Ssum on (the only FP64 on the GPU).
 #include "cbl_arith.cuh"
 #include "cbl_internal.h"
@@ -664,12 +664,37 @@ __device__ __forceinline__ DD dd_frac(DD a)
 constexpr int kBlockDD = 128;
 constexpr int kBlockSsum = 256;
 
-// 128-bit fraction, mod 1 and taken in [-1/2, 1/2), as a double-double.
-__device__ __forceinline__ DD dd_from_fraction(const uint32_t w[4])
+// 192-bit fraction, mod 1 and taken in [-1/2, 1/2), as a double-double: the magnitude is
+// shifted up to its leading bit, so a small fraction keeps its own bits; 53 of them are the
+// high double, exactly, the next 64 the low one, rounded. Integers and one addition: a
+// chain of double-double additions over the words made Ssum 1 us longer (seven series
+// kernel by kernel: 56 us at 1e4 and 76.6 at 1e6; 46 and 66.1 us so).
+__device__ __forceinline__ DD dd_from_fraction(const uint32_t w[6])
 {
-    const DD top = two_sum((double)(int32_t)w[3] * 0x1p-32, (double)w[2] * 0x1p-64);
-    const DD low = two_sum((double)w[1] * 0x1p-96, (double)w[0] * 0x1p-128);
-    return dd_add(top, low);
+    uint64_t a = ((uint64_t)w[5] << 32) | w[4], b = ((uint64_t)w[3] << 32) | w[2], c = ((uint64_t)w[1] << 32) | w[0];
+    const bool minus = (int64_t)a < 0;
+    if (minus) {
+        c = 0ull - c;
+        b = ~b + (c == 0);
+        a = ~a + (b == 0 && c == 0);
+    }
+    int e = 0;
+#pragma unroll 1
+    while (a == 0 && e < 128) {
+        a = b;
+        b = c;
+        c = 0;
+        e += 64;
+    }
+    if (a == 0) return DD{0.0, 0.0};
+    const int s = __clzll((long long)a);
+    if (s > 0) {
+        a = (a << s) | (b >> (64 - s));
+        b = (b << s) | (c >> (64 - s));
+    }
+    e += s;
+    const double scale = __hiloint2double((int)((uint32_t)(1023 - 53 - e) << 20 | (minus ? 0x80000000u : 0u)), 0);
+    return two_sum(__ull2double_rn(a >> 11) * scale, __ull2double_rn((a << 53) | (b >> 11)) * (scale * 0x1p-64));
 }
 
 // Residue kind of a modulus (Seg::flags), and the first k of the next kind.
@@ -684,50 +709,85 @@ __device__ __forceinline__ uint32_t modulus_kind(uint64_t m, uint64_t &limit)
     return 6;
 }
 
-// Sum over a block of its lanes' 128-bit accumulators, mod 1, in w of thread 0.
-// half: 8 words of shared memory, zero before the call.
-__device__ __forceinline__ void block_sum128(const Acc<4> &acc, uint32_t *half, uint32_t w[4])
+// Add a warp's lanes' accumulators, as the top N of six digits, into half: 12 words of
+// shared memory, the sums of the digits' 16-bit halves.
+template <int N>
+__device__ __forceinline__ void add_halves(const Acc<N> &acc, uint32_t *half)
 {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < N; ++j) {
         const uint32_t lo = __reduce_add_sync(0xffffffffu, acc.w[j] & 0xffffu);
         const uint32_t hi = __reduce_add_sync(0xffffffffu, acc.w[j] >> 16);
         if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&half[2 * j], lo);
-            atomicAdd(&half[2 * j + 1], hi);
+            atomicAdd(&half[2 * (6 - N + j)], lo);
+            atomicAdd(&half[2 * (6 - N + j) + 1], hi);
         }
     }
-    __syncthreads();
+}
+
+// The halves' sums, mod 1.
+__device__ __forceinline__ void fraction_of(const uint32_t *half, uint32_t w[6])
+{
     uint64_t c = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 6; ++j) {
         c += (uint64_t)half[2 * j] + ((uint64_t)half[2 * j + 1] << 16);
         w[j] = (uint32_t)c;
         c >>= 32;
     }
 }
 
-// Terms k in [k0, k1) of one series, k1 <= d, and with tail the terms k = d .. d+9. A
-// term's fraction enters the sum as its first 128 bits: the ladder runs to
-// 2^(10(d-k) + 128) and four REDC steps give them as quotient digits, as in the
-// 192-bit mode. Lanes, blocks and bigSum add 128-bit integers mod 1, and Ssum makes one
-// double-double of the sum: FP64 (1.6 operations a clock and SM here) is left to
-// Ssum and Sum7, where the terms took two divisions and 25 operations each (2^25
-// terms at 1e10: 3.25 ms; 0.74 ms so). The truncations (below 2^-128 a term, of either
-// sign) stay under the rounding of one double-double addition.
-// Warps take tiles of tile_k terms (a multiple of 64) in turn.
-template <int LEVEL>
-__global__ void __launch_bounds__(kBlockDD, LEVEL == 2 ? 7 : 9) dd_terms_kernel(uint4 *bigsum, uint64_t k0, uint64_t k1,
-                                                                             uint64_t d, int sign, uint32_t den0,
-                                                                             uint32_t den1, uint64_t tile_k, int tail,
-                                                                             int used)
+// Signed fraction of one term next to d (d - k <= kEndDD) or of the tail (k >= d) in
+// 192 bits: 2^(10(d-k)) / m is small there, and 128 bits would keep few of its own (66 of a
+// tail at the position limit). Long division, in one warp a launch.
+__device__ __forceinline__ Acc<6> end_fraction(uint64_t d, uint64_t k, uint64_t m, int sign)
 {
-    __shared__ uint32_t half[8];
+    uint64_t r = k < d ? (1ull << 10 * (d - k)) % m : 1, top = 0, mid = 0, low = 0;
+#pragma unroll 1
+    for (int j = 0; j < 3; ++j) {
+        const unsigned __int128 n = (unsigned __int128)r << 64;
+        top = mid;
+        mid = low;
+        low = (uint64_t)(n / m);
+        r = (uint64_t)n - low * m;
+    }
+    Acc<6> x{{(uint32_t)low, (uint32_t)(low >> 32), (uint32_t)mid, (uint32_t)(mid >> 32), (uint32_t)top,
+              (uint32_t)(top >> 32)}};
+    if (k > d) shr_digits<6>(x.w, (int)(10 * (k - d)));
+    if ((k + (uint64_t)sign) & 1) acc_negate_minus(x, 0);
+    return x;
+}
+
+// Terms k in [k0, k1) of one series, k1 <= d, and the terms k = end0 .. end0 + end_n - 1
+// next to d and behind it. A term's fraction enters the sum as its first 128 bits: the
+// ladder runs to 2^(10(d-k) + 128) and four REDC steps give them as quotient digits, as in
+// the 192-bit mode. Lanes add 128-bit integers mod 1, blocks and bigSum 192-bit ones, and
+// Ssum makes one double-double of the sum: FP64 (1.6 operations a clock and SM here) is left
+// to Ssum and Sum7, where the terms took two divisions and 25 operations each (2^25
+// terms at 1e10: 3.25 ms; 0.74 ms so). The truncations (below 2^-128 a term, of either
+// sign) stay under the rounding of one double-double addition of terms of their size; the
+// terms at the end, which are small by nature, come in 192 bits (end_fraction).
+// Warps take tiles of tile_k terms (a multiple of 64) in turn; the last warp, which has a
+// tile less than others unless they come out even, takes the end.
+template <int LEVEL>
+__global__ void __launch_bounds__(kBlockDD, LEVEL == 2 ? 7 : 9) dd_terms_kernel(uint2 *bigsum, uint64_t k0, uint64_t k1,
+                                                                             uint64_t d, int sign, uint32_t den0,
+                                                                             uint32_t den1, uint64_t tile_k,
+                                                                             uint64_t end0, int end_n, int used)
+{
+    __shared__ uint32_t half[12];
     const int lane = threadIdx.x & 31;
     const uint64_t step = (uint64_t)gridDim.x * (kBlockDD / 32) * tile_k;
     allow_dependent();
-    if (threadIdx.x < 8) half[threadIdx.x] = 0;
+    if (threadIdx.x < 12) half[threadIdx.x] = 0;
     __syncthreads();
+    if (end_n > 0 && blockIdx.x == gridDim.x - 1 && threadIdx.x >= kBlockDD - 32) {
+        const uint64_t k = end0 + lane, m = (uint64_t)den0 * k + den1;
+        Acc<6> x;
+        acc_zero(x);
+        if (lane < end_n && m != 1) x = end_fraction(d, k, m, sign);
+        add_halves<6>(x, half);
+    }
     Acc<4> acc;
     acc_zero(acc);
     uint64_t odd = k0 & 1;                              // acc holds terms of lanes whose k has parity odd + lane
@@ -746,31 +806,31 @@ __global__ void __launch_bounds__(kBlockDD, LEVEL == 2 ? 7 : 9) dd_terms_kernel(
         }
     }
     if ((odd + lane + sign) & 1) acc_negate(acc);
-    if (tail && blockIdx.x == 0 && threadIdx.x < kTailDD) {
-        const uint64_t k = d + lane, m = (uint64_t)den0 * k + den1;
-        if (m != 1) {
-            const unsigned __int128 x = ~(unsigned __int128)0 / m >> 10 * lane;     // 2^128 / m: m is odd
-            const uint32_t q[4] = {(uint32_t)x, (uint32_t)(x >> 32), (uint32_t)(x >> 64), (uint32_t)(x >> 96)};
-            if ((k + (uint64_t)sign) & 1) acc_negate(acc);
-            acc_add(acc, q);
-            if ((k + (uint64_t)sign) & 1) acc_negate(acc);
-        }
-    }
-    uint32_t w[4];
-    block_sum128(acc, half, w);
+    add_halves<4>(acc, half);
+    __syncthreads();
     if (threadIdx.x == 0) {
+        uint32_t q[6];
+        fraction_of(half, q);
         await_predecessor();
-        Acc<4> v{{w[0], w[1], w[2], w[3]}};
+        Acc<6> v;
+        acc_zero(v);
+        uint2 *own = bigsum + 3 * blockIdx.x;
         if ((int)blockIdx.x < used) {                   // entries from `used` on hold nothing yet
-            const uint4 o = bigsum[blockIdx.x];
-            const uint32_t q[4] = {o.x, o.y, o.z, o.w};
-            acc_add(v, q);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const uint2 o = own[j];
+                v.w[2 * j] = o.x;
+                v.w[2 * j + 1] = o.y;
+            }
         }
-        bigsum[blockIdx.x] = make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]);
+        acc_add(v, q);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) own[j] = make_uint2(v.w[2 * j], v.w[2 * j + 1]);
     }
 }
 
-typedef void (*DDTermsFn)(uint4 *, uint64_t, uint64_t, uint64_t, int, uint32_t, uint32_t, uint64_t, int, int);
+typedef void (*DDTermsFn)(uint2 *, uint64_t, uint64_t, uint64_t, int, uint32_t, uint32_t, uint64_t, uint64_t, int,
+                          int);
 
 static DDTermsFn dd_terms_fn(int level)
 {
@@ -781,42 +841,44 @@ static DDTermsFn dd_terms_fn(int level)
 
 int dd_terms_max_ctas_per_sm(int level) { return max_ctas_per_sm(dd_terms_fn(level), kBlockDD); }
 
-cudaError_t launch_dd_terms(int level, uint4 *bigsum, int grid, int *used, uint64_t k0, uint64_t k1, uint64_t d,
-                            int sign, uint32_t den0, uint32_t den1, bool tail, cudaStream_t st)
+cudaError_t launch_dd_terms(int level, uint2 *bigsum, int grid, int *used, uint64_t k0, uint64_t k1, uint64_t d,
+                            int sign, uint32_t den0, uint32_t den1, uint64_t end0, int end_n, cudaStream_t st)
 {
     // eight tiles a resident warp: their costs fall along k, and each warp takes every eighth part
     const uint64_t warps = (uint64_t)grid * (kBlockDD / 32), n = k1 > k0 ? k1 - k0 : 0;
     const uint64_t tile_k = std::max<uint64_t>(1, (n + 8 * 64 * warps - 1) / (8 * 64 * warps)) * 64;
     const int blocks = (int)std::min<uint64_t>(grid, std::max<uint64_t>(1, (n + tile_k - 1) / tile_k));
     const cudaError_t e = launch_dependent(dd_terms_fn(level), blocks, kBlockDD, st, bigsum, k0, k0 + n, d, sign, den0,
-                                           den1, tile_k, tail ? 1 : 0, *used);
+                                           den1, tile_k, end0, end_n, *used);
     *used = std::max(*used, blocks);
     return e;
 }
 
-__global__ void __launch_bounds__(kBlockSsum) dd_ssum_kernel(const uint4 *bigsum, int nblk, double2 *partial)
+__global__ void __launch_bounds__(kBlockSsum) dd_ssum_kernel(const uint2 *bigsum, int nblk, double2 *partial)
 {
-    __shared__ uint32_t half[8];
+    __shared__ uint32_t half[12];
     allow_dependent();
-    if (threadIdx.x < 8) half[threadIdx.x] = 0;
+    if (threadIdx.x < 12) half[threadIdx.x] = 0;
     __syncthreads();
     await_predecessor();
-    Acc<4> acc;
+    Acc<6> acc;
     acc_zero(acc);
     for (int i = threadIdx.x; i < nblk; i += kBlockSsum) {
-        const uint4 v = bigsum[i];
-        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+        const uint2 a = bigsum[3 * i], b = bigsum[3 * i + 1], c = bigsum[3 * i + 2];
+        const uint32_t q[6] = {a.x, a.y, b.x, b.y, c.x, c.y};
         acc_add(acc, q);
     }
-    uint32_t w[4];
-    block_sum128(acc, half, w);
+    add_halves<6>(acc, half);
+    __syncthreads();
     if (threadIdx.x == 0) {
+        uint32_t w[6];
+        fraction_of(half, w);
         const DD v = dd_from_fraction(w);
         *partial = make_double2(v.hi, v.lo);
     }
 }
 
-cudaError_t launch_dd_ssum(const uint4 *bigsum, int nblk, double2 *partial, cudaStream_t st)
+cudaError_t launch_dd_ssum(const uint2 *bigsum, int nblk, double2 *partial, cudaStream_t st)
 {
     return launch_dependent(dd_ssum_kernel, 1, kBlockSsum, st, bigsum, nblk, partial);
 }

@@ -73,14 +73,15 @@ int cbl_Sglobal32mtg(cbl_ctx *ctx, uint64_t offset, uint64_t d, uint64_t k_max,
                      int64_t numesign, uint64_t den0, uint64_t den1);
 /* Sglobal64mtg / Sglobal64mtg_192 / Sglobal64mtg_192_Refresh (Bellard.cl:914-1092,
  * Bellard_div2by1.cl:313-359): same contract for any modulus below 2^62. In
- * mode 0 one path covers them all: the fractions' first 128 bits, as integers
+ * mode 0 one path covers them all: the fractions' first 128 bits (192 from k = d-6 on), as integers
  * (the reference switches to its OVERDOUBLE build from 2^53 on, Bellard.cl:937-945). */
 int cbl_Sglobal64mtg(cbl_ctx *ctx, uint64_t offset, uint64_t d, uint64_t k_max,
                      int64_t numesign, uint64_t den0, uint64_t den1);
 /* Sglobal_after / Sglobal_after_192 (Bellard.cl:1118-1253): the tail terms
  * k >= d (10 in mode 0, 20 in modes 1-2). */
 int cbl_Sglobal_after(cbl_ctx *ctx, uint64_t d, int64_t numesign, uint64_t den0, uint64_t den1);
-/* Ssum / Ssum_192 (Bellard.cl:1274-1315): reduce bigSum to the partial. */
+/* Ssum / Ssum_192 (Bellard.cl:1274-1315): reduce bigSum to the partial. In mode 0 the
+ * sum is taken mod 1 into [-1/2, 1/2); a small one keeps a double-double's bits of its own. */
 int cbl_Ssum(cbl_ctx *ctx);
 /* Sum7 / Sum7_192 (Bellard.cl:1324-1398): weight the partial by numer
  * (1,4,32,64,256), write the weighted partial back, add it into dev_ans. */
