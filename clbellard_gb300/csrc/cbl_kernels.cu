@@ -850,7 +850,7 @@ cudaError_t launch_dd_terms(int level, uint2 *bigsum, int grid, int *used, uint6
     const int blocks = (int)std::min<uint64_t>(grid, std::max<uint64_t>(1, (n + tile_k - 1) / tile_k));
     const cudaError_t e = launch_dependent(dd_terms_fn(level), blocks, kBlockDD, st, bigsum, k0, k0 + n, d, sign, den0,
                                            den1, tile_k, end0, end_n, *used);
-    *used = std::max(*used, blocks);
+    if (e == cudaSuccess) *used = std::max(*used, blocks);
     return e;
 }
 
