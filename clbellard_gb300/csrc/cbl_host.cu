@@ -83,6 +83,8 @@ struct cbl_ctx {
     int partial = 0;                                 // a budgeted run is in progress
     std::vector<Seg> prep_segs;                      // host copy of the prepared segments
     std::vector<int> prep_shift;
+    uint64_t prep_hash = 0;                          // identity of that table, formed by the first checkpoint call
+    bool prep_hashed = false;
     // double-double buffers
     uint2 *d_bigsum = nullptr;                       // 192-bit fractions, one per block of the term kernel
     int dd_blocks = 0;                               // leading bigSum entries that hold sums
@@ -808,11 +810,16 @@ static uint64_t fnv1a(const void *p, size_t n, uint64_t h = 1469598103934665603u
     return h;
 }
 
-// Identity of the prepared tile table, for checkpoints.
-static uint64_t seg_hash(const cbl_ctx *c)
+// Identity of the prepared tile table, for checkpoints: formed once a table, and only where a
+// checkpoint asks for it (4096 positions: 5.5 MB, longer than the rest of the call).
+static uint64_t seg_hash(cbl_ctx *c)
 {
-    return fnv1a(c->prep_shift.data(), sizeof(int) * c->prep_npos,
-                 fnv1a(c->prep_segs.data(), sizeof(Seg) * c->prep_segs.size()));
+    if (!c->prep_hashed) {
+        c->prep_hash = fnv1a(c->prep_shift.data(), sizeof(int) * c->prep_npos,
+                             fnv1a(c->prep_segs.data(), sizeof(Seg) * c->prep_segs.size()));
+        c->prep_hashed = true;
+    }
+    return c->prep_hash;
 }
 
 // Number the prepared segments' tiles for the current tile size and upload
@@ -821,6 +828,7 @@ static int upload_prepared(cbl_ctx *c)
 {
     std::vector<Seg> &v = c->prep_segs;
     const int n = c->prep_npos;
+    c->prep_hashed = false;
     const uint64_t ntiles = order_and_number(v, (uint32_t)c->tile_k);
     std::vector<uint64_t> slot_tiles((size_t)7 * n, 0);
     uint64_t max_slot_tiles = 0;
