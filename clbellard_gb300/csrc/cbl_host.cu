@@ -26,6 +26,8 @@ namespace {
 constexpr uint64_t kMaxNeedD = 999999999999999999ull;   // Bellard_192.hsp:450
 constexpr int kDDBlocks = 4096;                         // mode 0's per-block partials (bigSum)
 constexpr int kDefaultTile = 32 * 64;                   // terms per warp tile
+constexpr size_t kJobSegs = 16;                         // a kernel-by-kernel call has at most 14: two ranges, cut at
+                                                        // the tail and the five residue-kind limits
 
 typedef unsigned __int128 u128;
 
@@ -59,7 +61,9 @@ struct cbl_ctx {
     unsigned long long *d_counter = nullptr;
     unsigned long long *d_slots = nullptr;   // nslot x 6 digit sums
     int slot_cap = 0;
-    unsigned long long *d_job_counter = nullptr;      // inside d_counter's allocation, a cache line each
+    // these, and job_table's buffers, lie in the allocations of d_counter (a cache line each)
+    // and h_small: two allocations less a context, 20 us of about 60
+    unsigned long long *d_job_counter = nullptr;
     unsigned long long *d_bigslot = nullptr;
     uint64_t *d_partial = nullptr;           // 3 words, most significant first
     uint64_t *d_ans = nullptr;               // 3 words
@@ -91,7 +95,7 @@ struct cbl_ctx {
     double2 *d_ddpartial = nullptr;
     double2 *d_ddans = nullptr;
     // scratch host
-    uint64_t *h_small = nullptr;              // pinned, 8 words
+    uint64_t *h_small = nullptr;              // pinned, 8 words, then job_table's staging
     // test hook: initial digit sums of the prepared passes' slots (null = zero)
     unsigned long long *d_preset = nullptr;
 };
@@ -287,6 +291,7 @@ int run_segments(cbl_ctx *c, std::vector<Seg> &v)
 {
     if (v.empty()) return CBL_OK;
     const uint64_t ntiles = order_and_number(v, (uint32_t)c->tile_k);
+    if (v.size() > kJobSegs) return CBL_E_ARG;          // cannot be: see kJobSegs
     const int rc = upload_table(c, c->job_table, v, nullptr, 0);
     if (rc) return rc;
     const int level = segs_level(v);
@@ -481,22 +486,25 @@ int cbl_create(int device, int precision, cbl_ctx **out)
         std::snprintf(c->devname, sizeof c->devname, "%s", prop.name);
     int rc = CBL_OK;
     if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess) rc = CBL_E_CUDA;
-    if (!rc && cudaMalloc(&c->d_counter, sizeof(unsigned long long) * 48) != cudaSuccess) rc = CBL_E_NOMEM;
-    if (!rc) {
-        c->d_job_counter = c->d_counter + 16;
-        c->d_bigslot = c->d_counter + 32;
-    }
+    constexpr size_t job_bytes = kJobSegs * sizeof(Seg);
+    if (!rc && cudaMalloc(&c->d_counter, sizeof(unsigned long long) * 48 + job_bytes) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_partial, sizeof(uint64_t) * 3) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ans, sizeof(uint64_t) * 3) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_bigsum, 3 * sizeof(uint2) * kDDBlocks) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ddpartial, sizeof(double2)) != cudaSuccess) rc = CBL_E_NOMEM;
     if (!rc && cudaMalloc(&c->d_ddans, sizeof(double2)) != cudaSuccess) rc = CBL_E_NOMEM;
-    if (!rc && cudaMallocHost(&c->h_small, sizeof(uint64_t) * 8) != cudaSuccess) rc = CBL_E_NOMEM;
+    if (!rc && cudaMallocHost(&c->h_small, sizeof(uint64_t) * 8 + job_bytes) != cudaSuccess) rc = CBL_E_NOMEM;
+    if (!rc) {
+        c->d_job_counter = c->d_counter + 16;
+        c->d_bigslot = c->d_counter + 32;
+        c->job_table.dev = reinterpret_cast<unsigned char *>(c->d_counter + 48);
+        c->job_table.host = reinterpret_cast<unsigned char *>(c->h_small + 8);
+        c->job_table.cap = job_bytes;
+    }
     if (!rc && cudaEventCreate(&c->ev_k0) != cudaSuccess) rc = CBL_E_CUDA;
     if (!rc && cudaEventCreate(&c->ev_k1) != cudaSuccess) rc = CBL_E_CUDA;
     if (!rc) rc = ensure_slots(c, 8);
     if (!rc) rc = ensure_table(c->prep_table, 64 * sizeof(Seg));
-    if (!rc) rc = ensure_table(c->job_table, 16 * sizeof(Seg));
     if (!rc) rc = ensure_pos(c, 1);
     if (!rc) {
         cudaMemsetAsync(c->d_slots, 0, sizeof(unsigned long long) * 6 * c->slot_cap, c->st);
@@ -523,7 +531,6 @@ int cbl_destroy(cbl_ctx *c)
     cudaSetDevice(c->device);
     if (c->st) cudaStreamSynchronize(c->st);
     free_table(c->prep_table);
-    free_table(c->job_table);
     cudaFree(c->d_counter);
     cudaFree(c->d_slots);
     cudaFree(c->d_partial);
