@@ -818,7 +818,7 @@ static uint64_t fnv1a(const void *p, size_t n, uint64_t h = 1469598103934665603u
 }
 
 // Identity of the prepared tile table, for checkpoints: formed once a table, and only where a
-// checkpoint asks for it (4096 positions: 5.5 MB, longer than the rest of the call).
+// checkpoint asks for it (4096 uneven positions: 3 MB, longer than the rest of the call).
 static uint64_t seg_hash(cbl_ctx *c)
 {
     if (!c->prep_hashed) {

@@ -64,7 +64,10 @@ def format_worklist(wl: Worklist) -> str:
 
 
 def balanced_worklist(needD: int, njobs: int, precision: int = 1) -> Worklist:
-    """njobs jobs of about equal device time (cbl_plan_jobs), numbered per series."""
+    """njobs jobs of about equal device time (cbl_plan_jobs), numbered per series.
+    The ranges depend on njobs and on the build's cost model, and a job file names only
+    (s, b): keep the worklist (format_worklist) beside its job files, and finish a work
+    directory from the worklist it was begun with."""
     from . import plan_jobs
     wl = Worklist(needD, precision)
     count = [0] * 7

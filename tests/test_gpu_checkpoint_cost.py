@@ -22,7 +22,8 @@ def test_later_checkpoints_do_not_hash_the_table_again(cbl):
         first, blob = save()
         later = [save() for _ in range(5)]
         assert all(b == blob for _, b in later)
-        # a full identity is a byte-wise hash of about 27 MB; what is left moves 6.7 MB
+        # a full identity is a byte-wise hash of 14 segments of 48 bytes a position; what is left
+        # moves 336 bytes a position
         assert min(t for t, _ in later) < first / 2
         ctx.prepare(pos[:-1] + [pos[-1] + 1000])               # another table: another identity
         with pytest.raises(cbl.CblError):
