@@ -145,6 +145,16 @@ int ensure_table(TileTable &t, size_t bytes)
     return CBL_OK;
 }
 
+// Calls that upload a table and return without waiting are refused while the caller captures
+// the stream: a replay would copy whatever the staging holds by then. (Calls that wait are
+// refused by the wait.)
+int refuse_capture(cbl_ctx *c)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(c->st, &status));
+    return status == cudaStreamCaptureStatusNone ? CBL_OK : CBL_E_CUDA;
+}
+
 // Upload a tile table (segments, then n shifts) through the pinned staging buffer,
 // waiting for the stream only where an earlier copy may still read that buffer.
 int upload_table(cbl_ctx *c, TileTable &t, const std::vector<Seg> &v, const int *shift, int n)
@@ -292,7 +302,8 @@ int run_segments(cbl_ctx *c, std::vector<Seg> &v)
     if (v.empty()) return CBL_OK;
     const uint64_t ntiles = order_and_number(v, (uint32_t)c->tile_k);
     if (v.size() > kJobSegs) return CBL_E_ARG;          // cannot be: see kJobSegs
-    const int rc = upload_table(c, c->job_table, v, nullptr, 0);
+    int rc = refuse_capture(c);
+    if (!rc) rc = upload_table(c, c->job_table, v, nullptr, 0);
     if (rc) return rc;
     const int level = segs_level(v);
     const TermGrid grid = grid_192(c, level);
@@ -571,13 +582,15 @@ int cbl_set_tuning(cbl_ctx *c, int tile_terms, int ctas_per_sm)
     if (!c || tile_terms < 32 || tile_terms % 32 != 0 || ctas_per_sm < 0) return CBL_E_ARG;
     if (c->partial) return CBL_E_ARG;                 // a budgeted run depends on the tile numbering
     const bool renumber = tile_terms != c->tile_k && c->prep_npos > 0;
+    if (renumber) {
+        cudaSetDevice(c->device);
+        const int rc = refuse_capture(c);
+        if (rc) return rc;
+    }
     c->tile_k = tile_terms;
     c->ctas_per_sm = ctas_per_sm;
     drop_graph(c);
-    if (renumber) {
-        cudaSetDevice(c->device);
-        return upload_prepared(c);
-    }
+    if (renumber) return upload_prepared(c);
     return CBL_OK;
     CBL_GUARD_END
 }
@@ -947,10 +960,13 @@ static int run_positions(cbl_ctx *c, const uint64_t *d, const int *shift, int n,
 {
     int rc = prepare_positions(c, d, shift, n);
     if (!rc) rc = enqueue_prepared(c, false, c->h_out3, to_ans ? c->d_ans : nullptr);
-    if (rc) return rc;
-    c->ev_valid = true;
-    c->launches += 2;
-    return sync(c);
+    if (!rc) {
+        c->ev_valid = true;
+        c->launches += 2;
+        rc = sync(c);
+    }
+    if (rc) c->prep_npos = 0;                             // its table may not have reached the device
+    return rc;
 }
 
 static int compute_d(cbl_ctx *c, uint64_t d, int shift, char hex[49])
@@ -1308,7 +1324,8 @@ int cbl_prepare(cbl_ctx *c, const uint64_t *pos, int n)
         if (rc) return rc;
     }
     cudaSetDevice(c->device);
-    return prepare_positions(c, d.data(), sh.data(), n);
+    const int rc = refuse_capture(c);
+    return rc ? rc : prepare_positions(c, d.data(), sh.data(), n);
     CBL_GUARD_END
 }
 

@@ -56,7 +56,8 @@ typedef struct cbl_ctx cbl_ctx;
 int cbl_create(int device, int precision, cbl_ctx **out);
 int cbl_destroy(cbl_ctx *ctx);
 int cbl_precision(const cbl_ctx *ctx);
-/* The context's CUDA stream (a cudaStream_t), for callers that time with events. */
+/* The context's CUDA stream (a cudaStream_t), for callers that time with events. Not for
+ * capturing the library's calls: those that upload a table or wait are refused then. */
 void *cbl_stream(cbl_ctx *ctx);
 /* Device name (CL_DEVICE_NAME in the reference, Bellard_192.hsp:41,528). */
 int cbl_device_name(const cbl_ctx *ctx, char *buf, int len);
