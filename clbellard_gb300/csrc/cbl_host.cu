@@ -1432,6 +1432,7 @@ int cbl_autotune(cbl_ctx *c, const uint64_t *pos, int n, int force, int *best_ti
     double ms_best = -1.0;
     if (!force && tune_cache_lookup(key, &tile, &ctas)) {
         int rc = cbl_set_tuning(c, tile, ctas);
+        if (!rc) rc = cbl_prepare(c, pos, n);             // as a measured sweep leaves it
         if (rc) return rc;
     } else {
         const int occ = blocks_to_ctas(blocks);

@@ -28,3 +28,16 @@ def test_entries_of_other_kernels_are_measured_again(cbl, tmp_path, monkeypatch)
     with cbl.Context(0, 1) as ctx:
         assert ctx.autotune(pos) == (tile, ctas, -1.0)
         assert ctx.batch(pos) == want
+
+
+def test_a_cached_choice_leaves_the_positions_prepared(cbl, tmp_path, monkeypatch):
+    monkeypatch.setenv("CBL_TUNE_CACHE", str(tmp_path / "tune.txt"))
+    pos = [1000, 123455]
+    with cbl.Context(0, 1) as ctx:
+        ctx.autotune(pos)
+    with cbl.Context(0, 1) as ctx:
+        want = ctx.batch(pos)
+        ctx.prepare([5000])
+        assert ctx.autotune(pos)[2] == -1.0
+        ctx.run_prepared()
+        assert ctx.read_results() == want
