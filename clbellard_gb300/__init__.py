@@ -297,7 +297,6 @@ class Context:
         n = len(positions)
         pos = (ctypes.c_uint64 * max(1, n))(*positions)
         _check(load().cbl_prepare(self._h, pos, n), "prepare")
-        self._prepared = n
 
     def run_prepared(self):
         _check(load().cbl_run_prepared(self._h), "run_prepared")
@@ -326,7 +325,6 @@ class Context:
         t, c, ms = ctypes.c_int(), ctypes.c_int(), ctypes.c_double()
         _check(load().cbl_autotune(self._h, pos, n, 1 if force else 0, ctypes.byref(t), ctypes.byref(c),
                                    ctypes.byref(ms)), "autotune")
-        self._prepared = n
         return t.value, c.value, ms.value
 
     def set_slot_preset(self, preset=None):
@@ -345,7 +343,9 @@ class Context:
         return ms.value
 
     def read_results(self):
-        n = getattr(self, "_prepared", 0)
+        """Results (ints) of the positions that the context holds prepared: those of the last
+        prepare, autotune, batch or compute. A checkpoint is 40 bytes and 336 a position."""
+        n = max(0, (load().cbl_checkpoint_size(self._h) - 40) // 336)
         out = (ctypes.c_uint64 * max(3, 3 * n))()
         _check(load().cbl_read_results(self._h, out), "read_results")
         return [words_to_int(out[3 * i:3 * i + 3]) for i in range(n)]
